@@ -27,6 +27,23 @@ struct MixedF {
     float dhc;                  // delta-SPH: coef * h * c
 };
 
+// Constants of the stored-pair FP64 sums (kernels_pairs64.cu), the mass and the
+// cubic kernel's factors multiplied in.
+struct PairConst {
+    double inv_h, h;
+    double w0q, w2, w3;  // kernel value, near branch: w0q + q^2 (w2 + w3 q)
+    double w6;           // far branch: w6 (2 - q)^3
+    double s1, s1q, s2;  // kernel gradient over the separation: s1 + s1q q, (s2 / dist) (2 - q)^2
+    double w0;           // m W(0)
+    double etq_h2;
+    double av_c;         // -2 h alpha c
+    double av_beta2h;    // 2 h beta
+    double lj_rr0, lj_D;
+    double dhc2;         // -2 dhc (delta-SPH)
+    int visc, bulk;      // artificial viscosity on; its bulk coefficient is not zero
+    uint32_t cap;        // stored values per particle
+};
+
 // Everything a kernel needs from rrsph_params, precomputed on the host.
 struct DevParams {
     int dim;
@@ -40,7 +57,7 @@ struct DevParams {
     double cell;            // cell_scale_k * hsml (grid_cell_size)
     double inv_cell;
     double cut2;            // sqr(grid_cell_size()) computed as the reference does
-    double h, inv_h, mass, g, rho0;
+    double h, inv_h, mass, g, rho0, inv_rho0;
     double B;               // EOS: c^2 rho0 / 7
     double c_eos;           // eos_art_c()
     double c_av;            // params.eos_sound_vel used by the artificial viscosity
@@ -82,6 +99,7 @@ struct DevParams {
     // clears the table wholesale before the reorder writes the new one
     int keep_cells;
     MixedF mf;
+    PairConst pc;
 };
 
 // One piston of a wave-maker table (rrsph_set_wave_makers): the law of
@@ -307,9 +325,12 @@ __device__ inline double kernel_dwdr_scale(int skf, double f, double q, double d
     }
 }
 
-// eos_art_p (EOS.cpp:31-34)
+// eos_art_p (EOS.cpp:31-34). rho / rho0 as three FP64 operations: the product
+// with the rounded reciprocal, corrected by its exact residual, is the
+// correctly rounded quotient (Markstein).
 __device__ inline double eos_p(const DevParams& P, double rho) {
-    const double x = rho / P.rho0;
+    const double x0 = rho * P.inv_rho0;
+    const double x = fma(fma(-x0, P.rho0, rho), P.inv_rho0, x0);
     const double x2 = x * x;
     const double x4 = x2 * x2;
     return P.B * (x4 * x2 * x - 1.0);

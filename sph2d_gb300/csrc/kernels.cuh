@@ -71,6 +71,21 @@ struct Sorted {
     // neighbour; word NC = stencil cells with more particles than a word has
     // bits (searched again by the force pass). Null where unused.
     uint32_t* nbmask;
+    // stored-pair FP64 step (kernels_pairs64.cu; null elsewhere), cell order:
+    double* pr;        // rows of 2 (3D: 4) doubles: position (3D: + density of the forces)
+    double* pv;        // rows of 2 (4): velocity of the forces (3D: + p / rho^2)
+    double* pq;        // 2D: rows of 2: density of the forces, p / rho^2
+    double* pd;        // continuity density: rows of 2 (4): velocity v
+    double* pe;        // delta-SPH: rows of 2: density rho, 1 / rho
+    uint32_t* pnear;   // [3^dim][n], words as nbmask: the neighbours at up to one h
+    uint8_t* pbefore;  // [3^dim][n]: neighbours in the stencil cells before this one (at most 255)
+    uint8_t* pown;     // [3^dim][n], summation density: the same of those with a larger sorted index (owned pairs)
+    uint32_t* pcount;  // [n]: neighbours the masks hold
+    uint32_t* pfirst;  // [3^dim][n]: first particle of the stencil cell
+    double* pw;        // [cap][n], summation density: kernel value of neighbour number s
+    double* pf;        // [cap][n] records of its acceleration: 2 doubles (2D summation density), or 4 with the rate
+    double* ps;        // [cap][n], summation density: kernel gradient of owned pair number o
+    uint8_t* prank;    // [cap][n]: its owner's number among the neighbours of the other particle
     // mixed step with neighbour reuse: up to kVerletCap2 (2D) / kVerletCap3 (3D)
     // candidates per particle, sorted index | cell code << 27 (3D: << 25) with
     // code = (dx + 2) * 5 + (dy + 2) (3D: ((dx + 2) * 5 + (dy + 2)) * 5 + (dz + 2))
@@ -97,8 +112,11 @@ struct GatherSrc {
 template <int DIM>
 void launch_keys(const DevParams& P, const State& S, Sorted& G, StepScalars* scal, int predict, uint32_t* flags,
                  cudaStream_t st);
+// for_whom: the gathers the cell-order copies are for.
+enum : int { kReorderFp64 = 0, kReorderMixed = 1, kReorderPairs = 2 };
 template <int DIM>
-void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int mixed, cudaStream_t st);
+void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int for_whom,
+                    cudaStream_t st);
 // The pair gathers take their block size (threads, <= kMaxGatherThreads, a
 // multiple of 32) from the caller; the autotuner picks it.
 template <int DIM>
@@ -109,6 +127,19 @@ void launch_density_fp64(const DevParams& P, const State& S, const Sorted& G, St
 template <int DIM>
 void launch_forces_fp64(const DevParams& P, const State& S, const Sorted& G, uint32_t terms, StepScalars* scal,
                         uint32_t* flags, int write_mu, cudaStream_t st, int threads, int use_masks = 0);
+// The stored-pair FP64 step (kernels_pairs64.cu) on a grid reordered with kReorderPairs.
+template <int DIM>
+void launch_pair_masks(const DevParams& P, const Sorted& G, cudaStream_t st);
+template <int DIM>
+void launch_pair_terms(const DevParams& P, const Sorted& G, cudaStream_t st, int threads);
+template <int DIM>
+void launch_pair_density(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
+                         cudaStream_t st);
+template <int DIM>
+void launch_pair_forces(const DevParams& P, const Sorted& G, cudaStream_t st, int threads);
+template <int DIM>
+void launch_pair_sum(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
+                     cudaStream_t st);
 template <int DIM>
 void launch_density_mixed(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
                           cudaStream_t st, int threads);
@@ -191,6 +222,10 @@ void launch_download_direct(const DevParams& P, const State& S, double* r, doubl
 #ifndef RRSPH_DENSITY_CELL_TILES
 #define RRSPH_DENSITY_CELL_TILES 0
 #endif
+// Stored values per particle of the FP64 pair sums: about 20 neighbours in 2D
+// and 80 in 3D (120 to 160 beside the half-spaced walls); more are evaluated in place.
+constexpr uint32_t kPairCap2 = 48;
+constexpr uint32_t kPairCap3 = 160;
 constexpr int kVerletCap2 = 64;         // candidate-list entries per particle, 2D
 constexpr int kVerletCap3 = 256;        // and 3D
 inline int verlet_cap(int dim) { return dim == 3 ? kVerletCap3 : kVerletCap2; }

@@ -31,7 +31,9 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
 // the sorted arrays (the cells_start table of make_grid, GridFind.cpp:77-87).
 // R: 0 = FP64 gathers; 1 = the mixed loop with summation density; 2 = the
 // mixed loop with continuity density; 3 = mixed, outside the loop (the
-// velocities, density and pressure given by F, double copies for exports).
+// velocities, density and pressure given by F, double copies for exports);
+// 4 = the stored-pair FP64 step (packed rows; with continuity density the
+// pressure too, which waits for no sum).
 template <int DIM, int R>
 __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,6 +43,40 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
     if (k == 0 || G.key[k - 1] != key) G.cell_start[key] = k;
     if (k == P.n - 1 || G.key[k + 1] != key) G.cell_end[key] = k + 1;
     const int32_t t = S.itype[id];
+    if (R == 4) {
+        // what the neighbour masks' float test reads: an x of +inf (a non-existent
+        // particle) is beyond any cutoff, NaN (outside its cell: clamped or beyond the
+        // key's bits, the offset not accurate) asks for the double test
+        float4 o = DIM == 3 ? S.coff4[id] : make_float4(S.coff2[id].x, S.coff2[id].y, 0.0f, 0.0f);
+        const float half = 0.5f * P.mf.cell;
+        float off = fmaxf(fabsf(o.x - half), fabsf(o.y - half));
+        if (DIM == 3) off = fmaxf(off, fabsf(o.z - half));
+        if (!(off <= half * 1.001f)) o.x = __int_as_float(0x7FC00000);
+        if (t == P.type_non_existent) o.x = __int_as_float(0x7F800000);
+        G.P4[k] = o;
+        G.itype[k] = t;
+        double2* const pr = reinterpret_cast<double2*>(G.pr + (size_t)k * (DIM == 3 ? 4 : 2));
+        double2* const pv = reinterpret_cast<double2*>(G.pv + (size_t)k * (DIM == 3 ? 4 : 2));
+        pr[0] = make_double2(S.rx[id], S.ry[id]);
+        pv[0] = make_double2(F.vx[id], F.vy[id]);
+        double rho = 0.0, pr2 = 0.0;  // summation density: the density pass writes them
+        if (P.density_treatment != 0) {
+            const double rhod = S.rho[id], p = eos_p(P, rhod);
+            rho = F.rho[id];
+            pr2 = p / (rho * rho);
+            S.p[id] = p;
+            double2* const pd = reinterpret_cast<double2*>(G.pd + (size_t)k * (DIM == 3 ? 4 : 2));
+            pd[0] = make_double2(S.vx[id], S.vy[id]);
+            if (DIM == 3) pd[1] = make_double2(S.vz[id], 0.0);
+            if (P.density_treatment == 2) reinterpret_cast<double2*>(G.pe)[k] = make_double2(rhod, 1.0 / rhod);
+            if (DIM == 2) reinterpret_cast<double2*>(G.pq)[k] = make_double2(rho, pr2);
+        }
+        if (DIM == 3) {
+            pr[1] = make_double2(S.rz[id], rho);
+            pv[1] = make_double2(F.vz[id], pr2);
+        }
+        return;
+    }
     if (R == 0 || R == 3) {  // double copies: the FP64 gathers and the grid/neighbour exports
         G.rx[k] = S.rx[id];
         G.ry[k] = S.ry[id];
@@ -417,9 +453,11 @@ void launch_keys(const DevParams& P, const State& S, Sorted& G, StepScalars* sca
     k_keys<DIM><<<blocks_for(P.n, 256), 256, 0, st>>>(P, S, G, scal, predict, flags);
 }
 template <int DIM>
-void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int mixed, cudaStream_t st) {
+void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int for_whom,
+                    cudaStream_t st) {
     const unsigned b = blocks_for(P.n, 256);
-    if (!mixed) k_reorder<DIM, 0><<<b, 256, 0, st>>>(P, S, G, fsrc);
+    if (for_whom == kReorderPairs) k_reorder<DIM, 4><<<b, 256, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderFp64) k_reorder<DIM, 0><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else if (!fsrc.loop) k_reorder<DIM, 3><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else if (P.density_treatment == 0) k_reorder<DIM, 1><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else k_reorder<DIM, 2><<<b, 256, 0, st>>>(P, S, G, fsrc);

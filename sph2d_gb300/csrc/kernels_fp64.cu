@@ -1,5 +1,6 @@
-// kernels_fp64.cu — the density and force gathers in double precision (the
-// plain FP64 step). One thread per particle in cell order; the neighbours of a
+// kernels_fp64.cu — the directed density and force gathers in double precision:
+// the loop pieces, and the FP64 step for the method switches the stored-pair
+// sums (kernels_pairs64.cu) do not hold. One thread per particle in cell order; the neighbours of a
 // particle are the particles of the 3^dim cells around its cell that pass the
 // reference's cutoff test, visited in the reference's order (cells x-major,
 // ids ascending inside a cell), so the sums run in the same order as RRSPH_OMP.

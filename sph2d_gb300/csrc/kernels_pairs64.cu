@@ -1,0 +1,847 @@
+// kernels_pairs64.cu — the FP64 step's pair sums with each pair evaluated once.
+//
+// The FP64 pipe bounds this step: it takes 1.7 lanes per clock and SM where the
+// FP32 and integer pipes take 128, whatever lanes of a warp are active, and an
+// IEEE square root or division costs it 7.5 multiply-adds. So the pair terms,
+// which are symmetric (the kernel value, the coefficient of r_i - r_j in the
+// acceleration, the continuity rate), are evaluated for one of the two
+// directions only, by warps with every lane busy, and stored for both
+// particles; each particle then adds its own up in the search's order. The
+// bookkeeping this takes (masks, ranks, stores, loads) runs on the idle pipes.
+//
+//   k_pair_masks   neighbours of a particle as a bit mask per stencil cell, the
+//                  number of neighbours before each cell, their count
+//   k_pair_terms   each pair once: kernel value and gradient (summation
+//                  density); or the continuity rate and the acceleration
+//   k_pair_density rho, p of a particle from its stored kernel values
+//   k_pair_forces  each pair once: its acceleration (summation density)
+//   k_pair_sum     accelerations (and drho) from the stored ones
+//
+// Against the directed gathers (kernels_fp64.cu; both sides of a pair, IEEE
+// forms, 22 of 32 lanes): the 409k flume's density and forces 1.93 -> 0.48 ms
+// (step 1.91 -> 0.515), 385k particles in 3D 8.25 -> 2.2 ms a step, the 6k dam
+// break 189 -> 56 us. The FP64 pipe is 74-80 % busy in the pair passes.
+//
+// A pair of particles k < i is evaluated by k's warp. Neighbour number s of a
+// particle (its rank in the search's order: cells in stencil order, ids
+// ascending) has its value in slot s of the particle's column, slot * n +
+// particle; the other side's rank comes from its mask and count of the opposite
+// cell. Neighbours past the slots, and those of cells with more particles than
+// a mask has bits, are evaluated in place by both particles.
+#include "kernels.cuh"
+#include "neighbour.cuh"
+
+#include <type_traits>
+
+namespace rrsph {
+
+namespace {
+
+template <int DIM>
+struct Pm {  // masks of this dimension
+    using T = typename std::conditional<DIM == 3, unsigned long long, uint32_t>::type;
+    static constexpr uint32_t bits = DIM == 3 ? 64 : 32;
+    static constexpr int nc = DIM == 3 ? 27 : 9;
+    static __device__ __forceinline__ uint32_t popc(T m) {
+        return DIM == 3 ? (uint32_t)__popcll((unsigned long long)m) : (uint32_t)__popc((uint32_t)m);
+    }
+    static __device__ __forceinline__ uint32_t lowest(T m) {
+        return DIM == 3 ? (uint32_t)(__ffsll((long long)m) - 1) : (uint32_t)(__ffs((int)m) - 1);
+    }
+    static __device__ __forceinline__ T* masks(const Sorted& G) { return reinterpret_cast<T*>(G.nbmask); }
+    static __device__ __forceinline__ T* nears(const Sorted& G) { return reinterpret_cast<T*>(G.pnear); }
+};
+
+// Cell c of the stencil of the cell `key` (in the order of
+// get_neighbouring_cells2/3, GridUtils.h:190-250), stepping the interleaved
+// coordinates in place; false where the reference drops the cell (a coordinate
+// below 0 or above 65535, GridUtils.h:158-163, a key beyond the grid). wraps: a
+// 3D coordinate of 1024 became 0 (GridUtils.h:50-64).
+template <int DIM>
+__device__ __forceinline__ bool stencil_cell(const DevParams& P, uint32_t key, int c, uint32_t& cell, bool& wraps) {
+    constexpr uint32_t axis = DIM == 3 ? 0x09249249u : 0x55555555u;
+    uint32_t out = 0;
+    bool valid = true;
+    wraps = false;
+#pragma unroll
+    for (int a = 0; a < DIM; a++) {
+        const int d = DIM == 3 ? (a == 0 ? c / 9 : (a == 1 ? (c / 3) % 3 : c % 3)) - 1 : (a == 0 ? c / 3 : c % 3) - 1;
+        const uint32_t m = axis << a, x = key & m;
+        if (d < 0) valid = valid && x != 0;
+        if (d > 0) {
+            if (DIM == 3) wraps = wraps || x == m;
+            else valid = valid && x != m;
+        }
+        const uint32_t up = ((x | ~m) + (1u << a)) & m, down = (x - (1u << a)) & m;
+        out |= d < 0 ? down : (d > 0 ? up : x);
+    }
+    cell = out;
+    return valid && out < P.max_cells;
+}
+// Displacement of stencil cell c, in cells.
+template <int DIM>
+__device__ __forceinline__ float3 stencil_shift(int c) {
+    return DIM == 3 ? make_float3((float)(c / 9 - 1), (float)((c / 3) % 3 - 1), (float)(c % 3 - 1))
+                    : make_float3((float)(c / 3 - 1), (float)(c % 3 - 1), 0.0f);
+}
+
+struct D3 {
+    double x, y, z;
+};
+// Row k of a packed array of DIM (3D: padded to 4) doubles; .w the fourth.
+template <int DIM>
+__device__ __forceinline__ D3 row(const double* __restrict__ a, uint32_t k) {
+    const double2 q = *reinterpret_cast<const double2*>(a + (size_t)k * (DIM == 3 ? 4 : 2));
+    return {q.x, q.y, DIM == 3 ? a[(size_t)k * 4 + 2] : 0.0};
+}
+template <int DIM>
+__device__ __forceinline__ D3 row4(const double* __restrict__ a, uint32_t k, double& w) {
+    const double2* const p = reinterpret_cast<const double2*>(a + (size_t)k * 4);
+    const double2 q = p[0], u = p[1];
+    w = u.y;
+    return {q.x, q.y, u.x};
+}
+// Position, and velocity with (rho, p / rho^2) of sorted particle k: in 2D three
+// double2 rows, in 3D rho and p / rho^2 ride in the fourth words.
+template <int DIM>
+__device__ __forceinline__ void force_rows(const Sorted& G, uint32_t k, D3& r, D3& v, double& rho, double& pr2) {
+    if (DIM == 3) {
+        r = row4<3>(G.pr, k, rho);
+        v = row4<3>(G.pv, k, pr2);
+    } else {
+        r = row<2>(G.pr, k);
+        v = row<2>(G.pv, k);
+        const double2 q = reinterpret_cast<const double2*>(G.pq)[k];
+        rho = q.x;
+        pr2 = q.y;
+    }
+}
+
+__device__ __forceinline__ void warp_sum_add(unsigned long long* dst, unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, v);
+}
+
+// A double x > 0 scaled by a power of two to a float pair hi + lo (48 bits): hi
+// gets the biased exponent ex, which the caller picks.
+__device__ __forceinline__ void float_pair(double x, int ex, float& hi, float& lo) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    hi = __uint_as_float(((uint32_t)ex << 23) | ((uint32_t)(b >> 29) & 0x7FFFFFu));
+    lo = (float)((uint32_t)b & 0x1FFFFFFFu) * __uint_as_float((uint32_t)(ex - 52) << 23);
+}
+// y0 (1 + c), y0 an approximation whose low word is zero, |c| < 2^-19: the
+// mantissa is stepped as an integer in units of 2^-40 (at most 2^22 of them, what
+// the rounding constant takes).
+__device__ __forceinline__ double step_mantissa(double y0, float z, float c) {
+    const float d = fmaf(z * c, 1099511627776.0f, 12582912.0f);  // z in [1, 2) is y0's mantissa; 2^40, 1.5 * 2^23
+    const long long step = (long long)(__float_as_int(d) - 0x4B400000) << 12;
+    return __longlong_as_double(__double_as_longlong(y0) + step);
+}
+
+// 1/sqrt(x) and 1/x to 2^-40 without the FP64 pipe: the approximation instruction
+// (2^-20) and one third-order step in float pairs. The rest of the error is taken
+// out by the caller with a second-order Newton step on what it wants,
+//   d = x y:           sqrt(x) = d + (y/2)(x - d d)   (the residual is exact: half a unit)
+//   eh = 1/2 - d (y/2): 1/sqrt(x) = y + y eh
+//   e = 1 - x r:       v/x = v r + v r e
+// so that a root takes three FP64 operations, its inverse two more, and a
+// quotient three, where the IEEE forms take about eight each. The root of zero
+// or a subnormal x (coincident particles) gives infinity.
+__device__ __forceinline__ double inv_root_40(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const int hx = __double2hiint(x), hy = __double2hiint(y);
+    const float z = __uint_as_float(0x3F800000u | ((uint32_t)hy & 0xFFFFFu) << 3);
+    float mh, ml;  // x 2^(2k) with y = z 2^k: x y^2 = m z^2
+    float_pair(x, (hx >> 20) + 2 * (hy >> 20) - 3 * 1023 + 127, mh, ml);  // x > 0
+    const float p = z * z, pl = fmaf(z, z, -p);
+    float e = fmaf(-mh, p, 1.0f);
+    e = fmaf(-mh, pl, e);
+    e = fmaf(-ml, p, e);
+    const double r = step_mantissa(y, z, e * fmaf(0.375f, e, 0.5f));
+    return hx < 0x00100000 ? y : r;
+}
+__device__ __forceinline__ double inverse_40(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const int hx = __double2hiint(x), hy = __double2hiint(y);
+    const float z = __uint_as_float(0x3F800000u | ((uint32_t)hy & 0xFFFFFu) << 3);
+    float mh, ml;
+    float_pair(x, ((hx >> 20) & 0x7FF) + ((hy >> 20) & 0x7FF) - 2 * 1023 + 127, mh, ml);  // the sign is y's
+    float e = fmaf(-mh, z, 1.0f);
+    e = fmaf(-ml, z, e);
+    return step_mantissa(y, z, fmaf(e, e, e));
+}
+// Half of a normal double, by its exponent.
+__device__ __forceinline__ double half_of(double x) {
+    return __hiloint2double(__double2hiint(x) - 0x00100000, __double2loint(x));
+}
+
+// The cubic spline at squared distance d2 (SmoothingKernel.h:20-56): m W, and
+// m s with dW/dr = (r_i - r_j) s. NEAR: the branch q <= 1, where the two meet
+// with equal second derivatives, so which one takes a pair at q = 1 to float
+// accuracy does not show.
+struct Kern {
+    double w, s;
+};
+template <bool NEAR, bool W>
+__device__ __forceinline__ Kern cubic(const PairConst& C, double d2) {
+    const double y1 = inv_root_40(d2);
+    const double r = d2 * y1;
+    const double dist = fma(fma(-r, r, d2), half_of(y1), r);
+    const double q = __double2hiint(y1) == 0x7FF00000 ? 0.0 : dist * C.inv_h;
+    Kern k{0.0, 0.0};
+    if (NEAR) {
+        if (W) k.w = fma(q * q, fma(C.w3, q, C.w2), C.w0q);
+        k.s = fma(C.s1q, q, C.s1);
+    } else {
+        const double y = fma(y1, fma(-r, half_of(y1), 0.5), y1);
+        const double t = 2.0 - q, t2 = t * t;
+        const bool in = __double2hiint(t) >= 0;  // q <= 2
+        if (W) k.w = in ? (C.w6 * t) * t2 : 0.0;
+        k.s = in ? (C.s2 * y) * t2 : 0.0;
+    }
+    return k;
+}
+
+// Neighbours of each particle (find_neighbours, GridFind.cpp:112-189): a block
+// takes 32 consecutive particles, one warp per stencil cell, so the lanes of a
+// warp read the same few cells in step. The float test on the cell-relative
+// offsets decides outside the guard band around the cutoff, the reference's
+// double test inside it and for particles outside their cell (clamped, or
+// beyond the key's bits), whose x the reorder set to NaN (+inf: non-existent).
+// near: the neighbours at up to one h. Then the neighbours, and the owned ones,
+// in the cells before this one (saturated: a number past the slots is not stored).
+// Issue-bound: a dozen instructions per candidate. A group of lanes per
+// particle instead, a cell a lane, ran at 14 (3D: 9) lanes of 32: 124 us on the
+// 409k flume, 2.8 ms on 385k particles in 3D.
+template <int DIM>
+__global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_masks(DevParams P, Sorted G) {
+    using M = Pm<DIM>;
+    using T = typename M::T;
+    __shared__ uint32_t counts[M::nc][32];
+    const uint32_t lane = threadIdx.x & 31u;
+    const int c = threadIdx.x >> 5;
+    const uint32_t k = blockIdx.x * 32u + lane;
+    const bool active = k < P.n;
+    T mask = 0, near = 0;
+    uint32_t first = 0;
+    bool over = false;
+    if (active) {
+        const float4 pj = G.P4[k];
+        uint32_t cell;
+        bool wraps;
+        // (a non-existent particle has none: its x is infinite)
+        if (stencil_cell<DIM>(P, G.key[k], c, cell, wraps) && __float_as_int(pj.x) != 0x7F800000) {
+            const uint32_t s = G.cell_start[cell], end = G.cell_end[cell];
+            const uint32_t e = s != kEmpty ? end : s;
+            first = s;
+            // of two cells that meet by a wrapped coordinate only one sees the other: such
+            // pairs are not stored
+            over = e - s > (wraps ? 0u : M::bits);
+            if (!over) {
+                const MixedF& F = P.mf;
+                const float h2 = F.h * F.h;
+                const float3 sh = stencil_shift<DIM>(c);
+                const float shx = sh.x * F.cell - pj.x, shy = sh.y * F.cell - pj.y;
+                const float shz = DIM == 3 ? sh.z * F.cell - pj.z : 0.0f;
+                T bit = 1;
+#pragma unroll 4
+                for (uint32_t i = s; i < e; i++, bit <<= 1) {
+                    const float4 pi = G.P4[i];
+                    const float dx = pi.x + shx, dy = pi.y + shy, dz = DIM == 3 ? pi.z + shz : 0.0f;
+                    const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
+                    if (d2 < F.cut2_lo) mask |= bit;
+                    if (d2 < h2) near |= bit;
+                    if (!(d2 < F.cut2_lo) && !(d2 >= F.cut2_hi)) {
+                        const D3 a = row<DIM>(G.pr, i), b = row<DIM>(G.pr, k);
+                        const double r2 = exact_dist2<DIM>(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y),
+                                                           DIM == 3 ? __dsub_rn(a.z, b.z) : 0.0);
+                        if (r2 < P.cut2 && G.itype[i] != P.type_non_existent) {
+                            mask |= bit;
+                            if (r2 < P.h * P.h) near |= bit;
+                        }
+                    }
+                }
+                if (c == M::nc / 2) mask &= ~((T)1 << (k - s));  // not itself
+            }
+        }
+    }
+    // at most 27 x 64 neighbours, and owned ones, in 12 bits each
+    const uint32_t cnt = M::popc(mask);
+    const uint32_t own = c == M::nc / 2 ? M::popc(mask & ~(((T)2 << ((k - first) & (M::bits - 1))) - 1))
+                                        : (first > k ? cnt : 0u);
+    counts[c][lane] = cnt | own << 12 | (over ? 0x80000000u : 0u);
+    __syncthreads();
+    if (!active) return;
+    uint32_t before = 0;
+    for (int b = 0; b < c; b++) before += counts[b][lane] & 0x7FFFFFFFu;
+    const uint32_t own_before = before >> 12;
+    before &= 0xFFFu;
+    M::masks(G)[(size_t)c * P.n + k] = mask;
+    M::nears(G)[(size_t)c * P.n + k] = near;
+    G.pfirst[(size_t)c * P.n + k] = first;
+    G.pbefore[(size_t)c * P.n + k] = (uint8_t)min(before, 255u);
+    if (G.pown) G.pown[(size_t)c * P.n + k] = (uint8_t)min(own_before, 255u);
+    if (c == M::nc - 1) {
+        uint32_t word = 0;
+        for (int b = 0; b < M::nc; b++) word |= (counts[b][lane] >> 31) << b;
+        M::masks(G)[(size_t)M::nc * P.n + k] = (T)word;
+        G.pcount[k] = before + cnt;
+    }
+}
+
+// The walk of the two pair passes: a warp takes 32 consecutive particles (and,
+// of `slices` warps sharing them, every slices-th stencil cell), each lane hands
+// out its particle's owned pairs (the neighbours with a larger sorted index) one
+// at a time onto a small stack, and whenever 32 are there the warp evaluates
+// them, one a lane. SPLIT: two stacks, for the two branches of the kernel, so
+// that a warp runs one of them. ORD: number the owned pairs of a particle too.
+// All lanes call f(word pair, lane has a pair, near as a constant) together;
+// pair_of() reads the words.
+constexpr int kStack = 64;  // up to 31 waiting and 32 pushed
+struct Pair {
+    uint32_t k, i;   // sorted indices, k < i
+    uint32_t rank;   // i's number among k's neighbours (255: that or more)
+    uint32_t order;  // and among the owned ones
+    int c;           // i's cell in k's stencil
+    uint32_t bit;    // k's bit in its own cell
+};
+// k0: the first particle of the warp.
+__device__ __forceinline__ Pair pair_of(uint2 e, uint32_t k0) {
+    return {k0 + (e.y & 31u), e.x, (e.y >> 16) & 255u, e.y >> 24, (int)((e.y >> 5) & 31u), (e.y >> 10) & 63u};
+}
+__device__ __forceinline__ uint32_t warp_first() { return (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; }
+template <int DIM, bool SPLIT, bool ORD, class F>
+__device__ __forceinline__ void walk_pairs(const DevParams& P, const Sorted& G, uint2* stacks, F&& f) {
+    using M = Pm<DIM>;
+    using T = typename M::T;
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const uint32_t k0 = warp_first(), k = k0 + lane;
+    if (k0 >= P.n) return;
+    uint2* const far_stack = stacks + (threadIdx.x >> 5) * (SPLIT ? 2 * kStack : kStack);
+    uint2* const near_stack = far_stack + kStack;
+    const int step = (int)gridDim.y;
+    const size_t n = P.n;
+    // a particle whose own cell is searched in place stores nothing
+    const bool active = k < P.n && !((M::masks(G)[(size_t)M::nc * n + k] >> (M::nc / 2)) & 1u);
+    const uint32_t bit = active ? k - G.pfirst[(size_t)(M::nc / 2) * n + k] : 0u;
+    // the lanes go through the cells together, the next cell's words loaded ahead
+    // (each lane at its own pace, a load after another by some lane in most rounds,
+    // took 165 us for the 2D terms of the 409k flume and 2.4 ms for 385k in 3D)
+    T m_next = 0, close_next = 0;
+    uint32_t first_next = 0, before_next = 0, own_next = 0;
+    auto fetch = [&](int c) {
+        m_next = 0;
+        if (!active || c >= M::nc) return;
+        const size_t at = (size_t)c * n + k;
+        m_next = M::masks(G)[at];
+        first_next = G.pfirst[at];
+        before_next = G.pbefore[at];
+        if (SPLIT) close_next = M::nears(G)[at];
+        if (ORD) own_next = G.pown[at];
+    };
+    uint32_t held = 0, held_near = 0;
+    fetch((int)blockIdx.y);
+    for (int c = (int)blockIdx.y; c < M::nc; c += step) {
+        const T all = m_next, close = close_next;
+        const uint32_t first = first_next, before = before_next;
+        uint32_t order = own_next;
+        fetch(c + step);
+        T bits = all;
+        if (c == M::nc / 2) bits &= ~(((T)2 << bit) - 1);  // without itself and the particles before it
+        else if (first < k) bits = 0;
+        for (;;) {
+            const bool has = bits != 0;
+            bool near = false;
+            uint2 e;
+            if (has) {
+                const uint32_t b = M::lowest(bits);
+                const T lower = ((T)1 << b) - 1;
+                bits &= bits - 1;
+                near = SPLIT && ((close >> b) & 1u);
+                const uint32_t rank = min(before + M::popc(all & lower), 255u);
+                e = make_uint2(first + b, lane | (uint32_t)c << 5 | bit << 10 | rank << 16 | min(order, 255u) << 24);
+                order++;
+            }
+            const uint32_t who = __ballot_sync(0xFFFFFFFFu, has && !near);
+            const uint32_t who_near = SPLIT ? __ballot_sync(0xFFFFFFFFu, near) : 0u;
+            if ((who | who_near) == 0) break;
+            if (has) {
+                if (near) near_stack[held_near + __popc(who_near & below)] = e;
+                else far_stack[held + __popc(who & below)] = e;
+            }
+            held += __popc(who);
+            held_near += __popc(who_near);
+            __syncwarp();
+            if (held >= 32) {
+                held -= 32;
+                f(far_stack[held + lane], true, std::false_type{});
+                __syncwarp();
+            }
+            if (SPLIT && held_near >= 32) {
+                held_near -= 32;
+                f(near_stack[held_near + lane], true, std::true_type{});
+                __syncwarp();
+            }
+        }
+    }
+    f(far_stack[lane], lane < held, std::false_type{});
+    if (SPLIT) f(near_stack[lane], lane < held_near, std::true_type{});
+}
+
+// The rank of k among i's neighbours: k is bit `bit` of i's stencil cell opposite c.
+template <int DIM>
+__device__ __forceinline__ uint32_t rank_of(const DevParams& P, const Sorted& G, uint32_t i, int c, uint32_t bit) {
+    using M = Pm<DIM>;
+    const size_t at = (size_t)(M::nc - 1 - c) * P.n + i;
+    const typename M::T m = M::masks(G)[at];
+    return G.pbefore[at] + M::popc(m & (((typename M::T)1 << bit) - 1));
+}
+
+// The viscous part of the coefficient (artificial_viscosity_part,
+// ArtificialViscosity.h:29-65) added to pf: Pi_ij for an approaching pair, with
+// one quotient for its two divisions. vr = (v_j - v_i).(r_j - r_i).
+__device__ __forceinline__ double add_visc(const PairConst& C, double pf, double vr, double d2, double rhos) {
+    if (__double2hiint(vr) >= 0) return pf;
+    const double x = (d2 + C.etq_h2) * rhos;
+    const double r = inverse_40(x);
+    const double e = fma(-x, r, 1.0);
+    const double u = vr * r;
+    const double w = fma(u, e, u);
+    double f = C.av_c;  // -2 h alpha c; 2 h (beta mu - alpha c) with a bulk term
+    if (C.bulk) f = fma(C.av_beta2h, C.h * rhos * w, f);
+    return fma(f, w, pf);
+}
+
+// Lennard-Jones coefficient of a fluid particle's boundary neighbour
+// (external_force_part, ExtForce.h:15-60). Few pairs: the IEEE forms, since the
+// twelfth power multiplies their error.
+__device__ __noinline__ double lj_coef(double rr0, double D, double d2) {
+    const double dist = sqrt(d2);
+    if (!(dist < rr0)) return 0.0;
+    const double rn = rr0 / dist;
+    const double rn2 = rn * rn, rn4 = rn2 * rn2, rn8 = rn4 * rn4;
+    return D * (rn8 * rn4 - rn4) / d2;
+}
+__device__ __forceinline__ bool lj_pair(const DevParams& P, int32_t tk, int32_t ti) {
+    return P.repulsive && ((tk > 0 && ti < 0) || (ti > 0 && tk < 0));
+}
+
+__device__ __forceinline__ double dot2(D3 a, D3 b) { return fma(a.x, b.x, a.y * b.y); }
+template <int DIM>
+__device__ __forceinline__ double dot(D3 a, D3 b) {
+    return DIM == 3 ? fma(a.z, b.z, dot2(a, b)) : dot2(a, b);
+}
+
+// Coefficients of r_i - r_k in the accelerations of k and of i (they differ by
+// the Lennard-Jones part, which only the fluid particle of the two feels).
+template <int DIM>
+__device__ __forceinline__ void force_coefs(const DevParams& P, const PairConst& C, double s, double d2,
+                                            D3 d, D3 vk, D3 vi, double rhok, double rhoi, double prk, double pri,
+                                            int32_t tk, int32_t ti, double& ck, double& ci) {
+    double pf = prk + pri;
+    if (C.visc) {
+        const double vr = dot<DIM>({vi.x - vk.x, vi.y - vk.y, DIM == 3 ? vi.z - vk.z : 0.0}, d);
+        pf = add_visc(C, pf, vr, d2, rhok + rhoi);
+    }
+    ck = ci = s * pf;
+    if (lj_pair(P, tk, ti)) {
+        const double fl = lj_coef(C.lj_rr0, C.lj_D, d2);
+        if (tk > 0) ck -= fl;
+        else ci -= fl;
+    }
+}
+
+// density_con's terms of a pair (Density.h:63-114): the rate is the same for
+// both sides, the delta-SPH part divides by the neighbour's density.
+template <int DIM>
+__device__ __forceinline__ void rate_terms(const DevParams& P, const PairConst& C, const Sorted& G, uint32_t k,
+                                           uint32_t i, double s, double d2, D3 d, double& tk, double& ti) {
+    const D3 a = row<DIM>(G.pd, k), b = row<DIM>(G.pd, i);
+    tk = ti = dot<DIM>({b.x - a.x, b.y - a.y, DIM == 3 ? b.z - a.z : 0.0}, d) * s;
+    if (P.density_treatment == 2) {
+        const double2 qk = reinterpret_cast<const double2*>(G.pe)[k], qi = reinterpret_cast<const double2*>(G.pe)[i];
+        const double f = C.dhc2 * (qi.x - qk.x) * s;  // -2 dhc m (rho_i - rho_k) s
+        tk = fma(f, qi.y, tk);
+        ti = fma(-f, qk.y, ti);
+        // coincident particles: the reference's (diff.dwdr) / dist^2 is 0/0
+        if ((__double_as_longlong(d2) << 1) == 0) tk = ti = __longlong_as_double(0x7FF8000000000000ll);
+    }
+}
+
+__device__ __forceinline__ double flip(double x) {
+    return __hiloint2double(__double2hiint(x) ^ 0x80000000, __double2loint(x));
+}
+// The stored terms of a neighbour, one record: 2D summation density (ax, ay);
+// else (ax, ay, az, rate), a whole 32-byte sector, since one side's is a
+// scattered store.
+template <int DIM, bool CONT>
+constexpr int kRec = DIM == 3 || CONT ? 4 : 2;
+template <int DIM, bool CONT>
+__device__ __forceinline__ void put_record(const Sorted& G, size_t at, D3 f, double rate) {
+    double2* const p = reinterpret_cast<double2*>(G.pf + at * kRec<DIM, CONT>);
+    if (kRec<DIM, CONT> == 2)
+        p[0] = make_double2(f.x, f.y);
+    else
+        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(f.x), "d"(f.y), "d"(f.z), "d"(rate)
+                     : "memory");
+}
+// Both sides: the products are made once unless the coefficients differ.
+template <int DIM, bool CONT>
+__device__ __forceinline__ void put_forces(const Sorted& G, uint32_t cap, uint32_t rk, uint32_t ri, size_t ak,
+                                           size_t ai, double ck, double ci, bool differ, D3 d, double tk, double ti) {
+    D3 f{ck * d.x, ck * d.y, DIM == 3 ? ck * d.z : 0.0};
+    if (rk < cap) put_record<DIM, CONT>(G, ak, f, tk);
+    if (differ) f = {ci * d.x, ci * d.y, DIM == 3 ? ci * d.z : 0.0};
+    if (ri < cap) put_record<DIM, CONT>(G, ai, {flip(f.x), flip(f.y), DIM == 3 ? flip(f.z) : 0.0}, ti);
+}
+
+// Each pair once. Summation density: m W into both columns, m s kept by the
+// owner with the other side's rank. Continuity density: the rates and the
+// accelerations into both columns (they wait for no sum).
+// FP64 operations a pair: 2D summation 12 in the near branch of the kernel, 16
+// in the far one; 3D continuity about 40.
+template <int DIM, bool CONT>
+__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_terms(DevParams P, Sorted G) {
+    extern __shared__ uint2 pair_stack[];
+    const PairConst& C = P.pc;
+    const uint32_t cap = C.cap;
+    const size_t n = P.n;
+    walk_pairs<DIM, true, !CONT>(P, G, pair_stack, [&](const uint2 e, bool active, auto near) {
+        constexpr bool NEAR = decltype(near)::value;
+        if (!active) return;
+        const Pair q = pair_of(e, warp_first());
+        const uint32_t k = q.k, i = q.i, rk = q.rank;
+        const uint32_t ri = rank_of<DIM>(P, G, i, q.c, q.bit);
+        const size_t ak = rk * n + k, ai = ri * n + i;
+        if (CONT) {
+            D3 a, b, va, vb;
+            double rhok, rhoi, prk, pri;
+            force_rows<DIM>(G, k, a, va, rhok, prk);
+            force_rows<DIM>(G, i, b, vb, rhoi, pri);
+            const int32_t yk = G.itype[k], yi = G.itype[i];
+            const D3 d{b.x - a.x, b.y - a.y, DIM == 3 ? b.z - a.z : 0.0};
+            const double d2 = dot<DIM>(d, d);
+            const Kern kk = cubic<NEAR, false>(C, d2);
+            double tk, ti, ck, ci;
+            rate_terms<DIM>(P, C, G, k, i, kk.s, d2, d, tk, ti);
+            force_coefs<DIM>(P, C, kk.s, d2, d, va, vb, rhok, rhoi, prk, pri, yk, yi, ck, ci);
+            put_forces<DIM, true>(G, cap, rk, ri, ak, ai, ck, ci, lj_pair(P, yk, yi), d, tk, ti);
+        } else {
+            const D3 a = row<DIM>(G.pr, k), b = row<DIM>(G.pr, i);
+            const D3 d{b.x - a.x, b.y - a.y, DIM == 3 ? b.z - a.z : 0.0};
+            const Kern kk = cubic<NEAR, true>(C, dot<DIM>(d, d));
+            if (rk < cap) G.pw[ak] = kk.w;
+            if (ri < cap) G.pw[ai] = kk.w;
+            if (q.order < cap) {
+                G.ps[q.order * n + k] = kk.s;
+                G.prank[q.order * n + k] = (uint8_t)min(ri, 255u);
+            }
+        }
+    });
+}
+
+// The kernel of a pair that stores none.
+__device__ __forceinline__ Kern cubic_any(const PairConst& C, double d2) {
+    return d2 < C.h * C.h ? cubic<true, true>(C, d2) : cubic<false, true>(C, d2);
+}
+
+// The accelerations, each pair once (summation density). A pair that recedes
+// (no viscosity) is done after 10 FP64 operations in 2D; the others (and the
+// wall pairs) go on to a second stack, and 32 of them at a time take the 12
+// more: half the pairs, where one pass costs every warp both (20 a pair, 205 us
+// on the 409k flume).
+template <int DIM>
+struct Approach {  // a warp's second stack
+    uint2 e[kStack];
+    double dx[kStack], dy[kStack], dz[DIM == 3 ? kStack : 1], vr[kStack];
+};
+template <int DIM>
+__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_forces(DevParams P, Sorted G) {
+    extern __shared__ double2 pair_shared[];
+    Approach<DIM>& A = reinterpret_cast<Approach<DIM>*>(pair_shared)[threadIdx.x >> 5];
+    uint2* const stacks = reinterpret_cast<uint2*>(reinterpret_cast<Approach<DIM>*>(pair_shared) + (blockDim.x >> 5));
+    const PairConst& C = P.pc;
+    const uint32_t cap = C.cap, lane = threadIdx.x & 31u;
+    const size_t n = P.n;
+    uint32_t held = 0;
+    auto second = [&](uint32_t at) {
+        const Pair q = pair_of(A.e[at], warp_first());
+        const uint32_t k = q.k, i = q.i, rk = q.rank;
+        const D3 d{A.dx[at], A.dy[at], DIM == 3 ? A.dz[at] : 0.0};
+        const double vr = A.vr[at];
+        D3 a, va;
+        double rhok, rhoi, prk, pri;
+        force_rows<DIM>(G, k, a, va, rhok, prk);
+        force_rows<DIM>(G, i, a, va, rhoi, pri);
+        const int32_t tk = G.itype[k], ti = G.itype[i];
+        const double d2 = dot<DIM>(d, d);
+        double s;
+        uint32_t ri;
+        if (q.order < cap) {
+            s = G.ps[q.order * n + k];
+            ri = G.prank[q.order * n + k];
+        } else {
+            s = cubic_any(C, d2).s;
+            ri = rank_of<DIM>(P, G, i, q.c, q.bit);
+        }
+        double pf = prk + pri;
+        if (C.visc) pf = add_visc(C, pf, vr, d2, rhok + rhoi);
+        double ck = s * pf, ci = ck;
+        const bool lj = lj_pair(P, tk, ti);
+        if (lj) {
+            const double fl = lj_coef(C.lj_rr0, C.lj_D, d2);
+            if (tk > 0) ck -= fl;
+            else ci -= fl;
+        }
+        put_forces<DIM, false>(G, cap, rk, ri, rk * n + k, ri * n + i, ck, ci, lj, d, 0.0, 0.0);
+    };
+    walk_pairs<DIM, false, true>(P, G, stacks, [&](const uint2 e, bool active, auto) {
+        bool go_on = false;
+        D3 d{0.0, 0.0, 0.0};
+        double vr = 0.0;
+        if (active) {
+            const Pair q = pair_of(e, warp_first());
+            const uint32_t k = q.k, i = q.i, rk = q.rank;
+            D3 a, b, va, vb;
+            double rhok, rhoi, prk, pri;
+            force_rows<DIM>(G, k, a, va, rhok, prk);
+            force_rows<DIM>(G, i, b, vb, rhoi, pri);
+            d = {b.x - a.x, b.y - a.y, DIM == 3 ? b.z - a.z : 0.0};
+            go_on = q.order >= cap || lj_pair(P, G.itype[k], G.itype[i]);
+            if (C.visc) {
+                vr = dot<DIM>({vb.x - va.x, vb.y - va.y, DIM == 3 ? vb.z - va.z : 0.0}, d);
+                go_on = go_on || __double2hiint(vr) < 0;
+            }
+            if (!go_on) {
+                const size_t ao = q.order * n + k;
+                const uint32_t ri = G.prank[ao];
+                const double c = G.ps[ao] * (prk + pri);
+                put_forces<DIM, false>(G, cap, rk, ri, rk * n + k, ri * n + i, c, c, false, d, 0.0, 0.0);
+            }
+        }
+        const uint32_t who = __ballot_sync(0xFFFFFFFFu, go_on);
+        if (go_on) {
+            const uint32_t at = held + __popc(who & ((1u << lane) - 1u));
+            A.e[at] = e;
+            A.dx[at] = d.x;
+            A.dy[at] = d.y;
+            if (DIM == 3) A.dz[at] = d.z;
+            A.vr[at] = vr;
+        }
+        held += __popc(who);
+        __syncwarp();
+        if (held >= 32) {
+            held -= 32;
+            second(held + lane);
+            __syncwarp();
+        }
+    });
+    if (lane < held) second(lane);
+}
+
+// The neighbours of k whose values are not stored: ranks from `first` on, and
+// the cells searched in place. f(i, r_i - r_k, squared distance).
+template <int DIM, class F>
+__device__ __forceinline__ void unstored_neighbours(const DevParams& P, const Sorted& G, uint32_t k, uint32_t over,
+                                                    uint32_t first, F&& f) {
+    using M = Pm<DIM>;
+    const uint32_t key = G.key[k];
+    const D3 a = row<DIM>(G.pr, k);
+    uint32_t rank = 0;
+    for (int c = 0; c < M::nc; c++) {
+        uint32_t cell;
+        bool wraps;
+        if ((over >> c) & 1u) {
+            stencil_cell<DIM>(P, key, c, cell, wraps);
+            for (uint32_t i = G.cell_start[cell]; i < G.cell_end[cell]; i++) {
+                if (i == k || G.itype[i] == P.type_non_existent) continue;
+                const D3 b = row<DIM>(G.pr, i);
+                const D3 d{__dsub_rn(b.x, a.x), __dsub_rn(b.y, a.y), DIM == 3 ? __dsub_rn(b.z, a.z) : 0.0};
+                const double d2 = exact_dist2<DIM>(d.x, d.y, d.z);
+                if (d2 < P.cut2) f(i, d, d2);
+            }
+            continue;
+        }
+        typename M::T m = M::masks(G)[(size_t)c * P.n + k];
+        if (m == 0) continue;
+        const uint32_t base = G.pfirst[(size_t)c * P.n + k];
+        for (; m; m &= m - 1, rank++) {
+            if (rank < first) continue;
+            const uint32_t i = base + M::lowest(m);
+            const D3 b = row<DIM>(G.pr, i);
+            const D3 d{b.x - a.x, b.y - a.y, DIM == 3 ? b.z - a.z : 0.0};
+            f(i, d, dot<DIM>(d, d));
+        }
+    }
+}
+
+// What of k's neighbours is stored: the number of slots; whether others remain.
+template <int DIM>
+__device__ __forceinline__ bool stored_slots(const DevParams& P, const Sorted& G, uint32_t k, uint32_t& over,
+                                             uint32_t& slots) {
+    using M = Pm<DIM>;
+    over = (uint32_t)M::masks(G)[(size_t)M::nc * P.n + k];
+    const uint32_t cnt = G.pcount[k];
+    slots = (over >> (M::nc / 2)) & 1u ? 0u : min(cnt, P.pc.cap);
+    return over != 0 || cnt > slots;
+}
+
+// density_sum + EOS (Density.h:25-61, EOS.cpp:31-34) from the stored values:
+// streams 8 bytes per neighbour.
+template <int DIM>
+__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_density(DevParams P, State S, Sorted G,
+                                                                   StepScalars* __restrict__ scal,
+                                                                   uint32_t* __restrict__ flags) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t cnt = 0;
+    if (k < P.n) {
+        const PairConst& C = P.pc;
+        uint32_t over, slots;
+        const bool more = stored_slots<DIM>(P, G, k, over, slots);
+        double acc = C.w0;
+        const double* const w = G.pw + k;
+#pragma unroll 8
+        for (uint32_t s = 0; s < slots; s++) acc += w[(size_t)s * P.n];
+        cnt = slots;
+        if (more && G.itype[k] != P.type_non_existent) {
+            unstored_neighbours<DIM>(P, G, k, over, slots, [&](uint32_t, D3, double d2) {
+                acc += cubic_any(C, d2).w;
+                cnt++;
+            });
+        }
+        if (cnt > P.max_nb - 1) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
+        const double p = eos_p(P, acc);
+        const double x = acc * acc, r = inverse_40(x), u = p * r;
+        const double pr2 = fma(u, fma(-x, r, 1.0), u);
+        if (DIM == 3) {
+            G.pr[(size_t)k * 4 + 3] = acc;
+            G.pv[(size_t)k * 4 + 3] = pr2;
+        } else {
+            reinterpret_cast<double2*>(G.pq)[k] = make_double2(acc, pr2);
+        }
+        const uint32_t id = G.id[k];
+        S.rho[id] = acc;
+        S.p[id] = p;
+    }
+    warp_sum_add(&scal->pairs, cnt);
+}
+
+// update_acceleration's sums (UpdateAcceleration.cpp:33-125), and density_con's
+// with continuity density, from the stored terms: one addition per component
+// and a record of 16 or 32 bytes per neighbour, streamed.
+template <int DIM, bool CONT>
+__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_sum(DevParams P, State S, Sorted G,
+                                                               StepScalars* __restrict__ scal,
+                                                               uint32_t* __restrict__ flags) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t cnt = 0;
+    if (k < P.n) {
+        const PairConst& C = P.pc;
+        const size_t n = P.n;
+        uint32_t over, slots;
+        const bool more = stored_slots<DIM>(P, G, k, over, slots);
+        double ax = 0.0, ay = -P.g, az = 0.0, rate = 0.0;
+        constexpr int R = kRec<DIM, CONT>;
+        const double2* const rec = reinterpret_cast<const double2*>(G.pf + (size_t)k * R);
+#pragma unroll 4
+        for (uint32_t s = 0; s < slots; s++) {
+            const double2* const p = rec + s * n * (R / 2);
+            const double2 f = p[0];
+            ax += f.x;
+            ay += f.y;
+            if (R == 4) {
+                const double2 g = p[R / 2 - 1];
+                if (DIM == 3) az += g.x;
+                if (CONT) rate += g.y;
+            }
+        }
+        cnt = slots;
+        if (more && G.itype[k] != P.type_non_existent) {
+            D3 r, v;
+            double rho, pr2;
+            force_rows<DIM>(G, k, r, v, rho, pr2);
+            const int32_t tk = G.itype[k];
+            unstored_neighbours<DIM>(P, G, k, over, slots, [&](uint32_t i, D3 d, double d2) {
+                D3 ri, vi;
+                double rhoi, pri, ck, ci;
+                force_rows<DIM>(G, i, ri, vi, rhoi, pri);
+                const Kern kk = cubic_any(C, d2);
+                force_coefs<DIM>(P, C, kk.s, d2, d, v, vi, rho, rhoi, pr2, pri, tk, G.itype[i], ck, ci);
+                ax = fma(d.x, ck, ax);
+                ay = fma(d.y, ck, ay);
+                if (DIM == 3) az = fma(d.z, ck, az);
+                if (CONT) {
+                    double t, ti;
+                    rate_terms<DIM>(P, C, G, k, i, kk.s, d2, d, t, ti);
+                    rate += t;
+                }
+                cnt++;
+            });
+        }
+        const uint32_t id = G.id[k];
+        S.ax[id] = ax;
+        S.ay[id] = ay;
+        if (DIM == 3) S.az[id] = az;
+        if (CONT) {
+            S.drho[id] = rate;
+            if (cnt > P.max_nb - 1) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
+        }
+    }
+    if (CONT) warp_sum_add(&scal->pairs, cnt);
+}
+
+// Warps that share 32 particles' stencil cells in the pair passes: one where the
+// particles alone give every SM a dozen warps; a third or a ninth of the cells
+// each below that, where one warp's pairs in a row would be the whole step's time.
+int pair_slices(uint32_t n) {
+    const uint32_t warps = (n + 31) / 32;
+    return warps >= 1824 ? 1 : (warps >= 608 ? 3 : 9);
+}
+
+}  // namespace
+
+template <int DIM>
+void launch_pair_masks(const DevParams& P, const Sorted& G, cudaStream_t st) {
+    k_pair_masks<DIM><<<(P.n + 31) / 32, 32 * Pm<DIM>::nc, 0, st>>>(P, G);
+}
+template <int DIM>
+void launch_pair_terms(const DevParams& P, const Sorted& G, cudaStream_t st, int threads) {
+    const dim3 grid((P.n + threads - 1) / threads, pair_slices(P.n));
+    const size_t sh = (size_t)(threads / 32) * 2 * kStack * sizeof(uint2);
+    if (P.density_treatment != 0) k_pair_terms<DIM, true><<<grid, threads, sh, st>>>(P, G);
+    else k_pair_terms<DIM, false><<<grid, threads, sh, st>>>(P, G);
+}
+template <int DIM>
+void launch_pair_density(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
+                         cudaStream_t st) {
+    k_pair_density<DIM><<<(P.n + 127) / 128, 128, 0, st>>>(P, S, G, scal, flags);
+}
+template <int DIM>
+void launch_pair_forces(const DevParams& P, const Sorted& G, cudaStream_t st, int threads) {
+    const dim3 grid((P.n + threads - 1) / threads, pair_slices(P.n));
+    const size_t sh = (size_t)(threads / 32) * (sizeof(Approach<DIM>) + kStack * sizeof(uint2));
+    k_pair_forces<DIM><<<grid, threads, sh, st>>>(P, G);
+}
+template <int DIM>
+void launch_pair_sum(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
+                     cudaStream_t st) {
+    if (P.density_treatment != 0) k_pair_sum<DIM, true><<<(P.n + 127) / 128, 128, 0, st>>>(P, S, G, scal, flags);
+    else k_pair_sum<DIM, false><<<(P.n + 127) / 128, 128, 0, st>>>(P, S, G, scal, flags);
+}
+
+#define RRSPH_INSTANTIATE(D)                                                                                    \
+    template void launch_pair_masks<D>(const DevParams&, const Sorted&, cudaStream_t);                          \
+    template void launch_pair_terms<D>(const DevParams&, const Sorted&, cudaStream_t, int);                     \
+    template void launch_pair_density<D>(const DevParams&, const State&, const Sorted&, StepScalars*, uint32_t*, \
+                                         cudaStream_t);                                                         \
+    template void launch_pair_forces<D>(const DevParams&, const Sorted&, cudaStream_t, int);                    \
+    template void launch_pair_sum<D>(const DevParams&, const State&, const Sorted&, StepScalars*, uint32_t*,    \
+                                     cudaStream_t);
+RRSPH_INSTANTIATE(2)
+RRSPH_INSTANTIATE(3)
+#undef RRSPH_INSTANTIATE
+
+}  // namespace rrsph

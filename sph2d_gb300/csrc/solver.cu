@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../host/error.hpp"
@@ -45,6 +46,36 @@ int dev_alloc(rrsph_solver* s, T** ptr, size_t count) {
     s->allocations.push_back(p);
     *ptr = static_cast<T*>(p);
     return RRSPH_OK;
+}
+
+// The arrays of the stored-pair FP64 step, all of them or none.
+bool alloc_pairs(rrsph_solver* s) {
+    auto& G = s->G;
+    const size_t n = s->P.n, cap = s->P.pc.cap, w = s->dim == 3 ? 4 : 2;
+    const bool cont = s->P.density_treatment != 0;
+    const size_t before = s->allocations.size();
+    auto get = [&](auto** ptr, size_t count) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, count * sizeof(**ptr)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        s->allocations.push_back(p);
+        *ptr = static_cast<std::remove_reference_t<decltype(*ptr)>>(p);
+        return true;
+    };
+    const bool ok = get(&G.pr, w * n) && get(&G.pv, w * n) && (s->dim == 3 || get(&G.pq, 2 * n)) &&
+                    (!cont || get(&G.pd, w * n)) && (s->P.density_treatment != 2 || get(&G.pe, 2 * n)) &&
+                    get(&G.pnear, (s->dim == 3 ? 2 * 27 : 9) * n) && get(&G.pbefore, (s->dim == 3 ? 27 : 9) * n) &&
+                    get(&G.pfirst, (s->dim == 3 ? 27 : 9) * n) && get(&G.pcount, n) && (cont || get(&G.pw, cap * n)) &&
+                    get(&G.pf, (s->dim == 3 || cont ? 4 : 2) * cap * n) &&
+                    (cont || (get(&G.pown, (s->dim == 3 ? 27 : 9) * n) && get(&G.ps, cap * n) && get(&G.prank, cap * n)));
+    if (ok) return true;
+    while (s->allocations.size() > before) {
+        cudaFree(s->allocations.back());
+        s->allocations.pop_back();
+    }
+    return false;
 }
 
 // Host copies of the smoothing-kernel factors and W (SmoothingKernel.h).
@@ -93,6 +124,7 @@ int fill_dev_params(const rrsph_params& p, rrsph::DevParams& P) {
     P.mass = p.mass;
     P.g = p.g;
     P.rho0 = p.rho0;
+    P.inv_rho0 = 1.0 / p.rho0;
     const double c_sqr = p.eos_sound_vel_method == 0 ? 200 * p.g * p.depth * p.eos_sound_vel_coef : p.eos_sound_vel;
     P.c_eos = std::sqrt(c_sqr);
     P.B = c_sqr * p.rho0 / 7;
@@ -167,7 +199,37 @@ int fill_dev_params(const rrsph_params& p, rrsph::DevParams& P) {
     M.ap_inv_wdelta = (float)(1.0 / P.ap_wdelta);
     M.avel_coef2 = (float)(2.0 * P.avg_vel_coef);
     M.dhc = (float)P.delta_sph_dhc;
+    rrsph::PairConst& C = P.pc;
+    C.inv_h = P.inv_h;
+    C.h = P.h;
+    {   // the products rounded once
+        const long double mf = (long double)P.mass * P.kf[1], ih = 1.0L / P.h;
+        C.w0q = (double)(mf * 2.0L / 3.0L);
+        C.w2 = (double)-mf;
+        C.w3 = (double)(mf * 0.5L);
+        C.w6 = (double)(mf / 6.0L);
+        C.s1 = (double)(-2.0L * mf * ih * ih);
+        C.s1q = (double)(1.5L * mf * ih * ih);
+        C.s2 = (double)(-0.5L * mf * ih);
+    }
+    C.w0 = P.mass * P.w0_density;
+    C.etq_h2 = P.etq_h2;
+    C.av_c = -2.0 * P.h * (P.av_alpha * P.c_av);
+    C.av_beta2h = 2.0 * P.h * P.av_beta;
+    C.lj_rr0 = P.lj_rr0;
+    C.lj_D = P.lj_D;
+    C.dhc2 = -2.0 * P.delta_sph_dhc;
+    C.visc = P.art_visc;
+    C.bulk = P.av_beta != 0.0;
+    C.cap = std::min<uint32_t>(P.dim == 3 ? rrsph::kPairCap3 : rrsph::kPairCap2, P.max_nb);
     return RRSPH_OK;
+}
+
+// Whether the loop's FP64 step may evaluate each pair once: the common method
+// set (the stored values hold no artificial pressure, XSPH velocity or
+// viscosity maximum, and are written for the cubic kernel and form 2).
+bool pair_method(const rrsph::DevParams& P) {
+    return P.all_cubic && P.intf_form == 2 && !P.art_pressure && !P.avg_vel && !(P.dt_method == 2 && P.dt_reduce);
 }
 
 int key_bits(uint64_t max_cells) {
@@ -218,7 +280,9 @@ template <int DIM>
 void enqueue_grid(rrsph_solver* s, int predict, rrsph::StepScalars* scal, rrsph::GatherSrc fsrc) {
     rrsph::launch_keys<DIM>(s->P, s->S, s->G, scal, predict, s->flags, s->stream);
     sort_grid(s, s->stream);
-    rrsph::launch_reorder<DIM>(s->P, s->S, s->G, fsrc, s->precision == RRSPH_PRECISION_MIXED, s->stream);
+    rrsph::launch_reorder<DIM>(s->P, s->S, s->G, fsrc,
+                               s->precision == RRSPH_PRECISION_MIXED ? rrsph::kReorderMixed : rrsph::kReorderFp64,
+                               s->stream);
     s->launches += 2;
 }
 
@@ -289,10 +353,10 @@ void enqueue_verlet_rebuild(rrsph_solver* s, cudaStream_t st) {
     const bool cont = s->P.density_treatment != 0;
     rrsph::GatherSrc fsrc{s->S.vpx, s->S.vpy, s->S.vpz, cont ? s->S.rho_pred : s->S.rho, nullptr, 1};
     if (s->dim == 3) {
-        rrsph::launch_reorder<3>(s->P, s->S, s->G, fsrc, 1, st);
+        rrsph::launch_reorder<3>(s->P, s->S, s->G, fsrc, rrsph::kReorderMixed, st);
         rrsph::launch_verlet_build<3>(s->P, s->S, s->G, st);
     } else {
-        rrsph::launch_reorder<2>(s->P, s->S, s->G, fsrc, 1, st);
+        rrsph::launch_reorder<2>(s->P, s->S, s->G, fsrc, rrsph::kReorderMixed, st);
         rrsph::launch_verlet_build<2>(s->P, s->S, s->G, st);
     }
     s->launches += 3;
@@ -400,12 +464,29 @@ void enqueue_step(rrsph_solver* s, int par, cudaEvent_t* events, bool with_keys)
     if (events) cudaEventRecord(events[1], s->stream);
     sort_grid(s, s->stream);
     if (events) cudaEventRecord(events[2], s->stream);
-    rrsph::launch_reorder<DIM>(s->P, s->S, s->G, fsrc, s->precision == RRSPH_PRECISION_MIXED, s->stream);
+    rrsph::launch_reorder<DIM>(s->P, s->S, s->G, fsrc,
+                               s->precision == RRSPH_PRECISION_MIXED ? rrsph::kReorderMixed
+                               : s->pairs64                          ? rrsph::kReorderPairs
+                                                                     : rrsph::kReorderFp64,
+                               s->stream);
     if (events) cudaEventRecord(events[3], s->stream);
-    enqueue_density<DIM>(s, cur);
+    if (s->pairs64) {
+        rrsph::launch_pair_masks<DIM>(s->P, s->G, s->stream);
+        rrsph::launch_pair_terms<DIM>(s->P, s->G, s->stream, s->gather_threads[0]);
+        if (!cont) rrsph::launch_pair_density<DIM>(s->P, s->S, s->G, cur, s->flags, s->stream);
+        s->launches += cont ? 2 : 3;
+    } else {
+        enqueue_density<DIM>(s, cur);
+    }
     if (s->mark_density) cudaEventRecordWithFlags(s->ev_density, s->stream, cudaEventRecordExternal);
     if (events) cudaEventRecord(events[4], s->stream);
-    enqueue_forces<DIM>(s, RRSPH_TERM_ALL, cur, 0, 1);
+    if (s->pairs64) {
+        if (!cont) rrsph::launch_pair_forces<DIM>(s->P, s->G, s->stream, s->gather_threads[1]);
+        rrsph::launch_pair_sum<DIM>(s->P, s->S, s->G, cur, s->flags, s->stream);
+        s->launches += cont ? 1 : 2;
+    } else {
+        enqueue_forces<DIM>(s, RRSPH_TERM_ALL, cur, 0, 1);
+    }
     if (events) cudaEventRecord(events[5], s->stream);
     rrsph::launch_whole_step<DIM>(s->P, s->S, s->G, cur, nxt, s->flags, 1, s->stream);
     if (events) cudaEventRecord(events[6], s->stream);
@@ -518,6 +599,8 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
         if (d3) A(S.coff4, n); else A(S.coff2, n);
         A(G.P4, n);
         if (cont) { A(G.vdx, n); A(G.vdy, n); if (d3) A(G.vdz, n); A(G.rhod, n); }
+        // 1.2 KB (3D: 5.7 KB) a particle; without room for them the directed gathers run
+        if (pair_method(s->P)) s->pairs64 = alloc_pairs(s);
     } else {
         if (d3) { A(S.coff4, n); A(S.vpf4, n); } else { A(S.coff2, n); A(S.vpf2, n); }
         if (n < rrsph::verlet_max_particles(s->dim)) {  // neighbour reuse

@@ -75,6 +75,7 @@ struct rrsph_solver {
     uint64_t timed_steps = 0;
     rrsph_impl::AdjointRun* adj = nullptr;
     int gather_threads[2] = {rrsph::kGatherThreads, rrsph::kGatherThreads};  // density, forces block sizes
+    bool pairs64 = false;  // the loop's FP64 step evaluates each pair once (kernels_pairs64.cu)
     // neighbour reuse of the FP32-mixed step
     bool verlet = false;
     double verlet_skin = kDefaultSkin3;        // skin, in units of hsml (set at creation by dimension)
