@@ -42,6 +42,7 @@ struct Sorted {
     uint32_t *keys_in, *ids_in;       // key pass output (id order)
     uint32_t *keys_a, *ids_a, *keys_b, *ids_b;
     uint32_t* sort_scratch;
+    uint32_t* scattered;              // counting sort: the ids grouped by cell, which the reorder puts in order (else null)
     uint32_t *key, *id;               // sorted result (points into a or b)
     uint32_t *cell_start, *cell_end;  // [max_cells]
     // FP64 gathers

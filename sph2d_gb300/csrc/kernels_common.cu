@@ -27,7 +27,7 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
     key_pass<DIM, 2>(P, S, G, i, S.rx[i], S.ry[i], DIM == 3 ? S.rz[i] : 0.0, flags);
 }
 
-// Gathers the state into cell order and records each cell's [start, end) in
+// Gathers the state into cell order and (after the radix sort) records each cell's [start, end) in
 // the sorted arrays (the cells_start table of make_grid, GridFind.cpp:77-87).
 // R: 0 = FP64 gathers; 1 = the mixed loop with summation density; 2 = the
 // mixed loop with continuity density; 3 = mixed, outside the loop (the
@@ -36,12 +36,23 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
 // pressure too, which waits for no sum).
 template <int DIM, int R>
 __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.n) return;
-    const uint32_t key = G.key[k];
-    const uint32_t id = G.id[k];
-    if (k == 0 || G.key[k - 1] != key) G.cell_start[key] = k;
-    if (k == P.n - 1 || G.key[k + 1] != key) G.cell_end[key] = k + 1;
+    uint32_t key, id;
+    if (G.scattered) {  // after the counting sort: the place among the cell's ids; the table is written
+        id = G.scattered[k];
+        key = G.keys_in[id];
+        const uint32_t s = G.cell_start[key], e = G.cell_end[key];
+        k = s;
+        for (uint32_t j = s; j < e; j++) k += G.scattered[j] < id ? 1u : 0u;
+        G.key[k] = key;
+        G.id[k] = id;
+    } else {
+        key = G.key[k];
+        id = G.id[k];
+        if (k == 0 || G.key[k - 1] != key) G.cell_start[key] = k;
+        if (k == P.n - 1 || G.key[k + 1] != key) G.cell_end[key] = k + 1;
+    }
     const int32_t t = S.itype[id];
     if (R == 4) {
         // what the neighbour masks' float test reads: an x of +inf (a non-existent

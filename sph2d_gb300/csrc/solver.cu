@@ -252,9 +252,10 @@ void set_verlet_params(rrsph_solver* s) {
     s->P.vl_cut2 = (float)(c * c * (1.0 + 1e-4));
     s->P.vl_half_skin2 = (float)(0.25 * skin * skin * (1.0 - 1e-4));
     s->P.vl_skin_edge = (float)(skin * 1.01);
-    // reset + sort (3 per 8-bit pass) + reorder + build (a step that reuses the
+    // reset + sort (3, or 3 per 8-bit pass) + reorder + build (a step that reuses the
     // lists launches nothing for them: the key pass wrote its cell-order copies)
-    s->vl_extra_launches = 3ull + 3ull * (unsigned long long)((s->sort_bits + 7) / 8);
+    s->vl_extra_launches = 3ull + (s->G.scattered ? 3ull : 3ull * (unsigned long long)((s->sort_bits + 7) / 8)) +
+                           (s->P.keep_cells && !s->G.scattered ? 1ull : 0ull);
 }
 
 int check_handle(rrsph_solver* s, const char* fn) {
@@ -264,12 +265,16 @@ int check_handle(rrsph_solver* s, const char* fn) {
     return RRSPH_OK;
 }
 
-// The stable sort of the key pass's (cell, id) pairs into (keys_a, ids_a),
-// whatever the number of passes: the grid stays there after the step, while
-// the whole step's key pass rewrites (keys_in, ids_in) for the next one.
+// The sort of the key pass's (cell, id) pairs; with the reorder after it the
+// grid is in (keys_a, ids_a), where it stays after the step, while the whole
+// step's key pass rewrites (keys_in, ids_in) for the next one.
 void sort_grid(rrsph_solver* s, cudaStream_t st) {
-    rrsph::radix_sort_pairs_into(s->G.keys_in, s->G.ids_in, s->G.keys_a, s->G.ids_a, s->G.keys_b, s->G.ids_b,
-                                 s->G.sort_scratch, s->P.n, s->sort_bits, st, &s->launches);
+    if (s->G.scattered)
+        rrsph::cell_sort(s->G.keys_in, s->G.keys_b, s->G.scattered, s->G.cell_start, s->G.cell_end, s->G.sort_scratch,
+                         s->P.n, s->P.max_cells, st, &s->launches);
+    else
+        rrsph::radix_sort_pairs_into(s->G.keys_in, s->G.ids_in, s->G.keys_a, s->G.ids_a, s->G.keys_b, s->G.ids_b,
+                                     s->G.sort_scratch, s->P.n, s->sort_bits, st, &s->launches);
     s->G.key = s->G.keys_a;
     s->G.id = s->G.ids_a;
 }
@@ -329,10 +334,11 @@ void set_verlet_copies(rrsph_solver* s, int read, int write) {
 bool tiles_active(const rrsph_solver* s) {
     return RRSPH_DENSITY_CELL_TILES && s->verlet && s->dim == 2 && s->P.density_treatment == 0 && s->P.all_cubic;
 }
-// The key pass keeps or clears cell-table entries as the density pass needs;
-// on a change the table is cleared wholesale (no entry of another grid stays).
+// The key pass keeps or clears cell-table entries as the density pass needs
+// (the counting sort rewrites the whole table: kept); on a change the table is
+// cleared wholesale (no entry of another grid stays).
 int set_keep_cells(rrsph_solver* s) {
-    const int keep = tiles_active(s) ? 1 : 0;
+    const int keep = s->G.scattered || tiles_active(s) ? 1 : 0;
     if (keep != s->P.keep_cells) {
         s->P.keep_cells = keep;
         RRSPH_CUDA_TRY(cudaMemsetAsync(s->G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream));
@@ -342,14 +348,11 @@ int set_keep_cells(rrsph_solver* s) {
 
 void enqueue_verlet_rebuild(rrsph_solver* s, cudaStream_t st) {
     rrsph::launch_verlet_reset(s->S.vl_rebuild, s->S.vl_gone, s->vl_builds, st);
-    if (s->P.keep_cells) {  // the previous build's table stayed in place: clear it for the reorder
+    if (s->P.keep_cells && !s->G.scattered) {  // the previous build's table stayed in place: clear it for the reorder
         rrsph::launch_clear_cells(s->G.cell_start, s->P.max_cells, st);
         s->launches++;
     }
-    rrsph::radix_sort_pairs_into(s->G.keys_in, s->G.ids_in, s->G.keys_a, s->G.ids_a, s->G.keys_b, s->G.ids_b,
-                                 s->G.sort_scratch, s->P.n, s->sort_bits, st, &s->launches);
-    s->G.key = s->G.keys_a;
-    s->G.id = s->G.ids_a;
+    sort_grid(s, st);
     const bool cont = s->P.density_treatment != 0;
     rrsph::GatherSrc fsrc{s->S.vpx, s->S.vpy, s->S.vpz, cont ? s->S.rho_pred : s->S.rho, nullptr, 1};
     if (s->dim == 3) {
@@ -585,8 +588,11 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
     A(S.rho, n); A(S.p, n); A(S.drho, n); A(S.rho_pred, n); A(S.mu, n);
     A(S.itype, n); A(S.key_of, n); A(S.itype_changed, 1);
     A(G.keys_in, n); A(G.ids_in, n); A(G.keys_a, n); A(G.ids_a, n); A(G.keys_b, n); A(G.ids_b, n);
-    A(G.sort_scratch, rrsph::sort_scratch_words((uint32_t)n));
-    A(G.cell_start, (size_t)s->P.max_cells); A(G.cell_end, (size_t)s->P.max_cells);
+    const bool counting = rrsph::cell_sort_fits(s->P.max_cells, n);
+    const size_t table = counting ? (size_t)rrsph::cell_tiles(s->P.max_cells) * rrsph::kCountTile : s->P.max_cells;
+    A(G.sort_scratch, counting ? rrsph::cell_sort_words(s->P.max_cells) : rrsph::sort_scratch_words((uint32_t)n));
+    A(G.cell_start, table); A(G.cell_end, table);
+    if (counting) G.scattered = G.ids_b;
     A(G.rx, n); A(G.ry, n); if (d3) A(G.rz, n);
     A(G.itype, n);
     if (!mixed) {
@@ -659,17 +665,19 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
         }
         s->verlet = true;
         s->verlet_skin = s->dim == 3 ? kDefaultSkin3 : kDefaultSkin2;
-        set_verlet_params(s);
-        s->P.keep_cells = tiles_active(s) ? 1 : 0;  // the table is cleared wholesale below
     }
+    s->P.keep_cells = G.scattered || tiles_active(s) ? 1 : 0;  // the table is cleared wholesale below
+    if (s->verlet) set_verlet_params(s);
     if (cudaMallocHost(&s->h_scal, sizeof(rrsph::StepScalars)) != cudaSuccess ||
         cudaMallocHost(&s->h_flags, sizeof(uint32_t)) != cudaSuccess ||
         cudaHostAlloc(&s->h_report, sizeof(rrsph::HostReport), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void**)&s->d_report, s->h_report, 0) != cudaSuccess)
         return fail(set_error(RRSPH_ERR_OUT_OF_MEMORY, "rrsph_create: pinned host allocation failed"));
     std::memset(s->h_report, 0, sizeof(rrsph::HostReport));
-    // empty cell table, zeroed state
-    if (cudaMemsetAsync(G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream) != cudaSuccess ||
+    // empty cell table, zeroed counts and state
+    if ((counting && cudaMemsetAsync(G.sort_scratch, 0, rrsph::cell_sort_words(s->P.max_cells) * sizeof(uint32_t),
+                                     s->stream) != cudaSuccess) ||
+        cudaMemsetAsync(G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream) != cudaSuccess ||
         cudaMemsetAsync(S.key_of, 0xFF, n * sizeof(uint32_t), s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->scal, 0, 2 * sizeof(rrsph::StepScalars), s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->flags, 0, sizeof(uint32_t), s->stream) != cudaSuccess ||
@@ -1159,7 +1167,7 @@ template <int DIM>
 void enqueue_component_grid(rrsph_solver* s, bool with_p) {
     s->keys_ready = false;  // this grid's keys were made without the predictor
     s->nlist_valid = false;  // and it replaces the grid the last step's list refers to
-    if (s->P.keep_cells)     // the last build's table is still in place
+    if (s->P.keep_cells && !s->G.scattered)  // the last build's table is still in place
         cudaMemsetAsync(s->G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream);
     if (s->S.vl_rebuild) cudaMemsetAsync(s->S.vl_rebuild, 0xFF, sizeof(uint32_t), s->stream);
     rrsph::GatherSrc fsrc{s->S.vx, s->S.vy, s->S.vz, s->S.rho, with_p ? s->S.p : nullptr, 0};
@@ -1367,7 +1375,7 @@ extern "C" int rrsph_kernel_launches(rrsph_solver* s, uint64_t* launches) {
         int rc = rrsph_neighbour_rebuilds(s, &builds);
         if (rc) return rc;
     }
-    *launches = s->launches + builds * (s->vl_extra_launches + (s->P.keep_cells ? 1ull : 0ull));
+    *launches = s->launches + builds * s->vl_extra_launches;
     return RRSPH_OK;
 }
 
@@ -1396,11 +1404,9 @@ extern "C" int rrsph_set_neighbour_reuse(rrsph_solver* s, int enable, double ski
     drop_graphs(s);
     s->verlet = enable != 0;
     s->nlist_valid = false;
-    if (enable) {
-        s->verlet_skin = skin_over_h;
-        set_verlet_params(s);
-    }
+    if (enable) s->verlet_skin = skin_over_h;
     if ((rc = set_keep_cells(s)) != 0) return rc;
+    if (enable) set_verlet_params(s);
     if (s->S.vl_rebuild) RRSPH_CUDA_TRY(cudaMemsetAsync(s->S.vl_rebuild, 0xFF, sizeof(uint32_t), s->stream));
     s->keys_ready = false;
     return RRSPH_OK;

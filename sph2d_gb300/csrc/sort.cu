@@ -1,4 +1,6 @@
-// sort.cu — stable LSD radix sort of (cell key, particle id) pairs.
+// sort.cu — the grid's sorts of particles by (cell, id): a counting sort over
+// the cell table (cell_sort) where the table is small enough, else a stable LSD
+// radix sort of (cell key, particle id) pairs, described here.
 //
 // Replaces the reference's serial counting sort over max_cells
 // (sources/RRSPH_OMP/src/GridFind.cpp:47-88) and the OpenCL bitonic sort
@@ -20,6 +22,7 @@ namespace rrsph {
 namespace {
 
 constexpr int kWarps = kSortThreads / 32;
+constexpr uint32_t kEmptyCell = 0xFFFFFFFFu;  // kEmpty (common.cuh)
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -141,7 +144,81 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t* __rest
     }
 }
 
+// ------------------------------------------- counting sort over the cells --
+
+// A place in its cell for every particle (in the order the atomics arrive), and
+// the particles per tile of cells: neighbouring ids mostly share a tile, so a
+// warp adds each tile's once.
+__global__ void k_cell_count(const uint32_t* __restrict__ keys, uint32_t* __restrict__ place,
+                             uint32_t* __restrict__ cells, uint32_t* __restrict__ tile_sums, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < n;
+    const uint32_t key = valid ? keys[i] : 0u;
+    if (valid) place[i] = atomicAdd(&cells[key], 1u);
+    const uint32_t tile = valid ? key / kCountTile : 0xFFFFFFFFu;
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, tile);
+    if (valid && (__ffs(peers) - 1) == (int)(threadIdx.x & 31u)) atomicAdd(&tile_sums[tile], (uint32_t)__popc(peers));
+}
+
+// Exclusive prefix of the counts over all cells, written as the cell table (an
+// empty cell starts at kEmpty, as after the radix sort); the counts are cleared
+// on the way. A block owns one tile of cells and adds up the tile sums before
+// its own itself (at most 64 words a thread, from L2), so no block waits for
+// another.
+__global__ void __launch_bounds__(kCountTile / 4) k_cell_table(uint4* __restrict__ cells,
+                                                               const uint32_t* __restrict__ tile_sums,
+                                                               uint4* __restrict__ cell_start,
+                                                               uint4* __restrict__ cell_end) {
+    constexpr uint32_t threads = kCountTile / 4, warps = threads / 32;
+    __shared__ uint32_t part[warps], base_part[warps];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const size_t at = (size_t)blockIdx.x * threads + threadIdx.x;
+    const uint4 a = cells[at];
+    uint32_t base = 0;
+#pragma unroll 4
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += threads) base += tile_sums[t];
+    const uint32_t own = a.x + a.y + a.z + a.w;
+    if (own) cells[at] = make_uint4(0u, 0u, 0u, 0u);
+    base = __reduce_add_sync(0xFFFFFFFFu, base);
+    uint32_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+    }
+    if (lane == 0) base_part[warp] = base;
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    uint32_t s = incl - own;
+#pragma unroll
+    for (uint32_t w = 0; w < warps; w++) s += base_part[w] + (w < warp ? part[w] : 0u);
+    const uint32_t s1 = s + a.x, s2 = s1 + a.y, s3 = s2 + a.z;
+    cell_start[at] = make_uint4(a.x ? s : kEmptyCell, a.y ? s1 : kEmptyCell, a.z ? s2 : kEmptyCell,
+                                a.w ? s3 : kEmptyCell);
+    if (own) cell_end[at] = make_uint4(s1, s2, s3, s3 + a.w);
+}
+
+__global__ void k_cell_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
+                               const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ scattered, uint32_t n,
+                               uint32_t* __restrict__ tile_sums, uint32_t tiles) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = i; t < tiles; t += gridDim.x * blockDim.x) tile_sums[t] = 0u;
+    if (i < n) scattered[cell_start[keys[i]] + place[i]] = i;
+}
+
 }  // namespace
+
+void cell_sort(const uint32_t* keys, uint32_t* place, uint32_t* scattered, uint32_t* cell_start, uint32_t* cell_end,
+               uint32_t* counts, uint32_t n, uint32_t max_cells, cudaStream_t stream, unsigned long long* launches) {
+    const uint32_t tiles = cell_tiles(max_cells), blocks = (n + 255) / 256;
+    uint32_t* const tile_sums = counts + (size_t)tiles * kCountTile;
+    k_cell_count<<<blocks, 256, 0, stream>>>(keys, place, counts, tile_sums, n);
+    k_cell_table<<<tiles, kCountTile / 4, 0, stream>>>(reinterpret_cast<uint4*>(counts), tile_sums,
+                                                       reinterpret_cast<uint4*>(cell_start),
+                                                       reinterpret_cast<uint4*>(cell_end));
+    k_cell_scatter<<<blocks, 256, 0, stream>>>(keys, place, cell_start, scattered, n, tile_sums, tiles);
+    if (launches) *launches += 3;
+}
 
 void radix_sort_pairs_into(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
                            uint32_t* keys_tmp, uint32_t* vals_tmp, uint32_t* counts, uint32_t n, int bits,
