@@ -419,7 +419,9 @@ typedef struct rrsph_wave_maker {
  * ensemble packed into one particle set (count = 0 restores the params' wave
  * maker). Ranges must not overlap. */
 int rrsph_set_wave_makers(rrsph_solver* s, uint32_t count, const rrsph_wave_maker* makers);
-/* Block sizes of the density and force gathers (multiples of 32, <= 256). */
+/* Block sizes of the density and force gathers (multiples of 32, <= 256). The
+ * gathers that split a particle's list over four warps (few particles, FP32-mixed
+ * with neighbour reuse) keep their own. */
 int rrsph_set_gather_threads(rrsph_solver* s, uint32_t density_threads, uint32_t force_threads);
 /* Autotuner: times `steps` steps on the uploaded state for every pair of
  * candidate gather block sizes (64, 128, 256), keeps the fastest and puts the

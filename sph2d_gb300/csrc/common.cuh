@@ -94,6 +94,7 @@ struct DevParams {
     // neighbour reuse (mixed step): list cutoff (cell + skin)^2, (skin / 2)^2, and
     // the distance from a cell edge within which the list looks two cells away
     float vl_cut2, vl_half_skin2, vl_skin_edge;
+    int vl_split;           // warps per 32 particles of its two gathers
     // 1: the key pass leaves the cell table of the last list build in place
     // (the cell-tile density pass reads it on reuse steps); each rebuild then
     // clears the table wholesale before the reorder writes the new one

@@ -96,6 +96,8 @@ struct Sorted {
     // vcount[k] = candidates (kListOver: too many, searched instead). This
     // step's neighbours (the candidates within the cutoff, in list order) in the
     // same slab layout: nlist, ncount[k] of them; words past ncount are stale.
+    // With split gathers (vl_split = 4) sub-list u of a particle takes the groups
+    // u, u + 4, ... and ncount[k] holds four counts of 8 bits.
     uint32_t* vlist;
     uint32_t* vcount;
     uint32_t* nlist;
@@ -170,6 +172,7 @@ void launch_clear_cells(uint32_t* cell_start, uint32_t max_cells, cudaStream_t s
 template <int DIM>
 void launch_nlist_export(const DevParams& P, const Sorted& G, uint32_t* counts, uint32_t* list, uint32_t max_per,
                          uint32_t* flags, cudaStream_t st);
+int verlet_split(int dim, uint32_t n);
 template <int DIM>
 void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
                            cudaStream_t st, int threads);

@@ -194,6 +194,32 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, Sta
     }
 }
 
+// The split gathers (L > 1): a block of L warps takes 32 particles, warp `sub`
+// their list groups sub, sub + L, ..., and the first warp adds the partial sums up
+// and goes on alone. With few particles a thread walking its whole list is one
+// long chain of dependent loads on a nearly empty chip. A warp's neighbours go to
+// the slab groups it reads (sub + L j), so no warp waits for another's count; the
+// L counts share the particle's word.
+template <int L>
+constexpr uint32_t kCountBits = 32 / L;
+template <int L>
+__device__ __forceinline__ uint32_t sub_count(uint32_t word, uint32_t sub) {
+    return L == 1 ? word : (word >> (sub * kCountBits<L>)) & ((1u << (kCountBits<L> & 31u)) - 1u);
+}
+// Slab offset of neighbour e of warp `sub` (in words, from the particle's uint4).
+template <int L>
+__device__ __forceinline__ size_t slab_at(uint32_t n, uint32_t sub, uint32_t e) {
+    return (size_t)(L == 1 ? e >> 2 : sub + L * (e >> 2)) * 4 * n + (e & 3u);
+}
+// The word of a list of c entries stored in consecutive groups.
+template <int L>
+__device__ __forceinline__ uint32_t packed_counts(uint32_t c) {
+    if (L == 1) return c;
+    uint32_t word = 0;
+    for (uint32_t g = 0; 4 * g < c; g++) word += min(4u, c - 4 * g) << ((g % L) * kCountBits<L>);
+    return word;
+}
+
 // One candidate's contribution to the density gather: W (summation) or the
 // continuity rate with its delta-SPH term (density_con, Density.h:63-114,
 // the same arithmetic as k_density_mixed).
@@ -220,7 +246,7 @@ __device__ __forceinline__ float density_term(const MixedF& M, int skf, float f,
 // neighbours, written to nlist for the force pass. A particle whose list
 // overflowed searches the stencil cells (the grid is rebuilt every step while
 // one does) and writes its neighbours too.
-template <int DIM, int SKF, bool CONT>
+template <int DIM, int SKF, bool CONT, int L>
 __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams P, State S, Sorted G,
                                                                      StepScalars* __restrict__ scal,
                                                                      uint32_t* __restrict__ flags) {
@@ -228,20 +254,20 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
     constexpr uint32_t IDX = Vl<DIM>::index;
     // the force gather may launch now: it waits for this grid at its start (griddepcontrol.wait)
     asm volatile("griddepcontrol.launch_dependents;");
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = k < P.n;
-    uint32_t cnt = 0;
+    const uint32_t lane = threadIdx.x & 31u, sub = L > 1 ? threadIdx.x >> 5 : 0u;
+    const uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
+    bool active = k < P.n;
+    uint32_t cnt = 0, word = 0;
+    Kahan acc{0.0f, 0.0f};
     if (active) {
         const MixedF& M = P.mf;
-        const uint32_t id = G.id[k];
         const float4 pj = G.P4[k];
         const int32_t tj = __float_as_int(pj.w);
         const int skf = SKF ? SKF : P.density_skf;
         const float f = M.kf[skf];
         const bool delta = CONT && P.density_treatment == 2;
         const float4 vdj = CONT ? G.VD4[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        Kahan acc{0.0f, 0.0f};
-        uint32_t* const nslab = G.nlist + (size_t)k * 4;  // neighbour e at nslab[(e / 4) * 4n + e % 4]
+        uint32_t* const nslab = G.nlist + (size_t)k * 4;  // neighbour e at nslab[slab_at(e)]
         if (tj != P.type_non_existent) {
             const uint32_t vc = G.vcount[k];
             if (vc != kListOver) {
@@ -253,9 +279,10 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
                 // the body has no branch but the rare guard-band test, and each group's
                 // sum is added with compensation
                 // (list words are read once a step: streaming loads keep L1 for the neighbours' data)
-                uint4 w = vc ? __ldcs(slab) : make_uint4(kVlNone, kVlNone, kVlNone, kVlNone);
-                for (uint32_t e0 = 0; e0 < vc; e0 += kVlBatch) {
-                    const uint4 wn = e0 + kVlBatch < vc ? __ldcs(slab + (size_t)((e0 >> 2) + 1) * P.n) : w;
+                uint4 w = 4 * sub < vc ? __ldcs(slab + (size_t)sub * P.n)
+                                       : make_uint4(kVlNone, kVlNone, kVlNone, kVlNone);
+                for (uint32_t e0 = 4 * sub; e0 < vc; e0 += kVlBatch * L) {
+                    const uint4 wn = e0 + kVlBatch * L < vc ? __ldcs(slab + (size_t)((e0 >> 2) + L) * P.n) : w;
                     const uint32_t en[kVlBatch] = {w.x, w.y, w.z, w.w};
                     float4 pb[kVlBatch];
 #pragma unroll
@@ -276,13 +303,14 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
                         const float4 vdi = CONT && in ? G.VD4[en[j] & IDX] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         const float t = density_term<DIM, SKF, CONT>(M, skf, f, dx, dy, dz, d2, vdi, vdj, delta);
                         part += in ? t : 0.0f;
-                        if (in) nslab[(size_t)(cnt >> 2) * 4 * P.n + (cnt & 3u)] = en[j];
+                        if (in) nslab[slab_at<L>(P.n, sub, cnt)] = en[j];
                         cnt += in;
                     }
                     acc.add(M.mass * part);
                     w = wn;
                 }
-            } else {
+                word = cnt;
+            } else if (sub == 0) {
                 constexpr int NC = DIM == 3 ? 27 : 9;
                 const Stencil<DIM> st(P, G.key[k]);
 #pragma unroll 1
@@ -307,16 +335,41 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
                         // this step's neighbour list too (the grid is this step's: the stencil
                         // offsets are within one cell)
                         if (cnt < (uint32_t)CAP)
-                            nslab[(size_t)(cnt >> 2) * 4 * P.n + (cnt & 3u)] = i | vl_code<DIM>(sx, sy, sz);
+                            nslab[slab_at<1>(P.n, 0, cnt)] = i | vl_code<DIM>(sx, sy, sz);
                         cnt++;
                         const float4 vdi = CONT ? G.VD4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         part += density_term<DIM, SKF, CONT>(M, skf, f, dx, dy, dz, d2, vdi, vdj, delta);
                     }
                     acc.add(M.mass * part);
                 }
+                word = packed_counts<L>(min(cnt, (uint32_t)CAP));
             }
         }
-        G.ncount[k] = cnt < (uint32_t)CAP ? cnt : (uint32_t)CAP;
+    }
+    if (L > 1) {
+        __shared__ float ps[L][32], pc[L][32];
+        __shared__ uint32_t pn[L][32];
+        ps[sub][lane] = acc.s;
+        pc[sub][lane] = acc.c;
+        pn[sub][lane] = cnt;
+        __syncthreads();
+        if (sub != 0) return;
+        if (active) {
+            // (an over-full list was searched by this warp alone, its counts packed)
+            const bool listed = G.vcount[k] != kListOver;
+#pragma unroll
+            for (int u = 1; u < L; u++) {
+                acc.add(ps[u][lane]);
+                acc.c += pc[u][lane];
+                cnt += pn[u][lane];
+                if (listed) word |= pn[u][lane] << ((uint32_t)u * kCountBits<L>);
+            }
+        }
+    }
+    if (active) {
+        const MixedF& M = P.mf;
+        const uint32_t id = G.id[k];
+        G.ncount[k] = L == 1 ? min(cnt, (uint32_t)CAP) : word;
         if (cnt > P.max_nb - 1) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
         if (!CONT) {
             // rho - rho0 = sum - (rho0 - m W(0)): the two are within a factor of two,
@@ -533,20 +586,24 @@ __global__ void __launch_bounds__(kTileWarps * 32) k_density_tiles(DevParams P, 
 // are not the ones the key pass writes (P4n, V4n, VD4n), and the list of every
 // particle is complete (the density pass wrote the neighbours of overflowed
 // lists too, which needs at most Vl<DIM>::cap neighbours per particle).
-template <int DIM, int SKF, bool STD, int WV>
-__global__ void __launch_bounds__(kMaxGatherThreads, 4) k_forces_verlet(DevParams P, State S, Sorted G,
+template <int DIM, int SKF, bool STD, int WV, int L>
+__global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_forces_verlet(DevParams P, State S, Sorted G,
                                                                     StepScalars* __restrict__ scal,
                                                                     StepScalars* __restrict__ next,
                                                                     uint32_t* __restrict__ flags) {
     constexpr uint32_t IDX = Vl<DIM>::index;
     // launched while the density gather finishes: wait for it (and its writes) first
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, sub = L > 1 ? threadIdx.x >> 5 : 0u;
+    const uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = k < P.n;
     double amag = 0, arvmu_d = 0;
+    Kahan ax{0, 0}, ay{0, 0}, az{0, 0};
+    Kahan avx{0, 0}, avy{0, 0}, avz{0, 0};
+    float arvmu = 0.0f;
+    const bool avel = !STD && P.avg_vel;
     if (active) {
         const MixedF& M = P.mf;
-        const uint32_t id = G.id[k];
         const float4 pj4 = G.P4[k];
         const int32_t tj = __float_as_int(pj4.w);
         ForceAcc<DIM, SKF> F{P, G, G.V4[k], G.PR[k], 0.0f, false, false, false, false, false, 0, 0,
@@ -555,22 +612,21 @@ __global__ void __launch_bounds__(kMaxGatherThreads, 4) k_forces_verlet(DevParam
         F.ext = P.repulsive && tj > 0;
         F.intf = true;
         F.visc = P.art_visc;
-        F.avel = P.avg_vel;
+        F.avel = avel;
         F.form1 = P.intf_form == 1;
         F.intf_skf = SKF ? SKF : P.intf_skf;
         F.av_skf = SKF ? SKF : P.av_skf;
-        Kahan ax{0, 0}, ay{0, 0}, az{0, 0};
-        Kahan avx{0, 0}, avy{0, 0}, avz{0, 0};
         if (tj != P.type_non_existent) {
             const uint32_t vc = G.vcount[k];
             if (WV != 0 || vc != kListOver) {
                 // this step's neighbours, four list words per load (the lanes of a
                 // warp load neighbouring uint4s), their data two at a time
-                const uint32_t nc = G.ncount[k];
+                const uint32_t nc = sub_count<L>(G.ncount[k], sub);
                 const uint4* nslab = reinterpret_cast<const uint4*>(G.nlist) + k;  // group g at nslab[g * n]
                 const float bx = -2.0f * M.cell - pj4.x, by = -2.0f * M.cell - pj4.y, bz = -2.0f * M.cell - pj4.z;
                 for (uint32_t e0 = 0; e0 < nc; e0 += 4) {
-                    const uint4 w = __ldcs(nslab + (size_t)(e0 >> 2) * P.n);  // streaming, as in the density pass
+                    // streaming, as in the density pass
+                    const uint4 w = __ldcs(nslab + (size_t)(L == 1 ? e0 >> 2 : sub + L * (e0 >> 2)) * P.n);
                     const uint32_t eg[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                     for (int h = 0; h < 4; h += kVlForceBatch<DIM, STD>) {
@@ -625,7 +681,7 @@ __global__ void __launch_bounds__(kMaxGatherThreads, 4) k_forces_verlet(DevParam
                         }
                     }
                 }
-            } else {
+            } else if (sub == 0) {
                 constexpr int NC = DIM == 3 ? 27 : 9;
                 const Stencil<DIM> st(P, G.key[k]);
 #pragma unroll 1
@@ -661,17 +717,52 @@ __global__ void __launch_bounds__(kMaxGatherThreads, 4) k_forces_verlet(DevParam
                 }
             }
         }
+        arvmu = F.arvmu;
+    }
+    if (L > 1) {  // the other warps' sums, then the first warp goes on alone
+        constexpr int Q = (DIM == 3 ? 3 : 2) * (STD ? 1 : 2);
+        __shared__ float part[L - 1 ? L - 1 : 1][2 * Q + 1][32];
+        auto each = [&](auto&& f) {
+            f(0, ax);
+            f(1, ay);
+            if (DIM == 3) f(2, az);
+            if (!STD) {
+                f(DIM, avx);
+                f(DIM + 1, avy);
+                if (DIM == 3) f(5, avz);
+            }
+        };
+        if (sub != 0) {
+            each([&](int q, const Kahan& a) {
+                part[sub - 1][2 * q][lane] = a.s;
+                part[sub - 1][2 * q + 1][lane] = a.c;
+            });
+            part[sub - 1][2 * Q][lane] = arvmu;
+        }
+        __syncthreads();
+        if (sub != 0) return;
+#pragma unroll
+        for (int u = 0; u < L - 1; u++) {
+            each([&](int q, Kahan& a) {
+                a.add(part[u][2 * q][lane]);
+                a.c += part[u][2 * q + 1][lane];
+            });
+            arvmu = fmaxf(arvmu, part[u][2 * Q][lane]);
+        }
+    }
+    if (active) {
+        const uint32_t id = G.id[k];
         const double axd = ax.value(), ayd = ay.value() - P.g;  // gravity along y (ExtForce.h), 2D and 3D
         const double azd = DIM == 3 ? az.value() : 0.0;
         S.ax[id] = axd;
         S.ay[id] = ayd;
         if (DIM == 3) S.az[id] = azd;
-        if (F.avel) {
+        if (avel) {
             S.avx[id] = avx.value();
             S.avy[id] = avy.value();
             if (DIM == 3) S.avz[id] = avz.value();
         }
-        arvmu_d = F.arvmu;
+        arvmu_d = arvmu;
         if (P.dt_reduce) amag = sqrt(axd * axd + ayd * ayd + azd * azd);
         if (WV != 0) {
             const double dt = step_dt<(WV & kVarRare) != 0>(P, scal, flags, k == 0);
@@ -701,10 +792,17 @@ void launch_verlet_build(const DevParams& P, const State& S, const Sorted& G, cu
     constexpr int kBuildThreads = 128;
     k_vl_build<DIM><<<(P.n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, st>>>(P, S, G);
 }
+// Warps per 32 particles of the two gathers (DevParams::vl_split, fixed when a
+// solver is created): four where a thread per particle leaves the SMs a few warps
+// each, else one. us per step with 1 / 4 (8 is no faster): 2D, 6k particles 32.5 /
+// 25.6, 22k 36.9 / 27.8, 33k 38.9 / 34.8, 43k 39.5 / 40.8, 66k 40.9 / 45.7; 3D,
+// 72k 105 / 90, 194k 207 / 211. (A block keeps the registers of the warps that
+// are done while its first warp finishes the step.)
+int verlet_split(int dim, uint32_t n) { return n <= (dim == 3 ? 128000u : 36000u) ? 4 : 1; }
+
 template <int DIM>
 void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
                            cudaStream_t st, int threads) {
-    const unsigned blocks = (P.n + threads - 1) / threads;
     const bool cont = P.density_treatment != 0;
 #if RRSPH_DENSITY_CELL_TILES
     if (DIM == 2 && !cont && P.all_cubic) {
@@ -713,13 +811,21 @@ void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, 
         return;
     }
 #endif
+#define RRSPH_DV(SKF, CONT)                                                                                           \
+    do {                                                                                                              \
+        if (P.vl_split == 4)                                                                                          \
+            k_density_verlet<DIM, SKF, CONT, 4><<<(P.n + 31) / 32, 128, 0, st>>>(P, S, G, scal, flags);               \
+        else                                                                                                          \
+            k_density_verlet<DIM, SKF, CONT, 1><<<(P.n + threads - 1) / threads, threads, 0, st>>>(P, S, G, scal, flags); \
+    } while (0)
     if (P.all_cubic) {
-        if (cont) k_density_verlet<DIM, 1, true><<<blocks, threads, 0, st>>>(P, S, G, scal, flags);
-        else k_density_verlet<DIM, 1, false><<<blocks, threads, 0, st>>>(P, S, G, scal, flags);
+        if (cont) RRSPH_DV(1, true);
+        else RRSPH_DV(1, false);
     } else {
-        if (cont) k_density_verlet<DIM, 0, true><<<blocks, threads, 0, st>>>(P, S, G, scal, flags);
-        else k_density_verlet<DIM, 0, false><<<blocks, threads, 0, st>>>(P, S, G, scal, flags);
+        if (cont) RRSPH_DV(0, true);
+        else RRSPH_DV(0, false);
     }
+#undef RRSPH_DV
 }
 // A launch that may start while the stream's previous kernel finishes
 // (programmatic dependent launch); the kernel waits for it with
@@ -741,15 +847,20 @@ void launch_after(void (*kernel)(Params...), unsigned blocks, int threads, cudaS
 template <int DIM>
 void launch_forces_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal,
                           StepScalars* scal_next, uint32_t* flags, cudaStream_t st, int threads, int whole) {
-    const unsigned blocks = (P.n + threads - 1) / threads;
     const bool std_terms = P.all_cubic && P.intf_form != 1 && P.art_visc && !P.art_pressure && !P.avg_vel;
     const int wv = whole ? (kVarMixed | (P.density_treatment != 0 ? kVarCont : 0) |
                             (P.avg_vel || P.dt_method == 2 ? kVarRare : 0))
                          : 0;
 // the force gather follows the density gather with a programmatic dependency:
 // its blocks launch as the density gather's last blocks run, then wait for it
-#define RRSPH_FV(SKF, STD, WV) \
-    launch_after(k_forces_verlet<DIM, SKF, STD, WV>, blocks, threads, st, P, S, G, scal, scal_next, flags)
+#define RRSPH_FV(SKF, STD, WV)                                                                                       \
+    do {                                                                                                             \
+        if (P.vl_split == 4)                                                                                         \
+            launch_after(k_forces_verlet<DIM, SKF, STD, WV, 4>, (P.n + 31) / 32, 128, st, P, S, G, scal, scal_next, flags); \
+        else                                                                                                         \
+            launch_after(k_forces_verlet<DIM, SKF, STD, WV, 1>, (P.n + threads - 1) / threads, threads, st, P, S, G, \
+                         scal, scal_next, flags);                                                                    \
+    } while (0)
 #define RRSPH_FV_WV(SKF, STD)                                                          \
     do {                                                                               \
         switch (wv) {                                                                  \
@@ -769,6 +880,12 @@ void launch_forces_verlet(const DevParams& P, const State& S, const Sorted& G, S
 
 namespace {
 
+// sub_count with the split as a value.
+__device__ __forceinline__ uint32_t split_count(uint32_t word, uint32_t sub, uint32_t split) {
+    const uint32_t bits = 32u / split;
+    return split == 1 ? word : (word >> (sub * bits)) & ((1u << bits) - 1u);
+}
+
 // The neighbour list the last density pass of the reuse step wrote (nlist,
 // ncount: build slots with cell codes, in list order), as particle ids: row
 // G.id[k] of `list` gets the ids of slot k's entries.
@@ -777,16 +894,21 @@ __global__ void k_nlist_export(DevParams P, Sorted G, uint32_t* __restrict__ cou
                                uint32_t max_per, uint32_t* __restrict__ flags) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.n) return;
-    const uint32_t id = G.id[k], c = G.ncount[k];
+    const uint32_t id = G.id[k], split = (uint32_t)P.vl_split, word = G.ncount[k];
+    uint32_t c = 0;
+    for (uint32_t u = 0; u < split; u++) c += split_count(word, u, split);
     counts[id] = c;
     // a searched (over-full) particle stores at most the list capacity: a full
     // row may have lost entries, which this copy cannot show
     const bool clipped = c == (uint32_t)Vl<DIM>::cap && G.vcount[k] == kListOver;
     if (c > max_per || clipped) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
     const uint32_t* const nslab = G.nlist + (size_t)k * 4;
-    const uint32_t m = c < max_per ? c : max_per;
-    for (uint32_t e = 0; e < m; e++)
-        list[(size_t)id * max_per + e] = G.id[nslab[(size_t)(e >> 2) * 4 * P.n + (e & 3u)] & Vl<DIM>::index];
+    uint32_t e = 0;
+    for (uint32_t u = 0; u < split; u++) {
+        const uint32_t m = split_count(word, u, split);
+        for (uint32_t j = 0; j < m && e < max_per; j++, e++)
+            list[(size_t)id * max_per + e] = G.id[nslab[(size_t)(u + split * (j >> 2)) * 4 * P.n + (j & 3u)] & Vl<DIM>::index];
+    }
 }
 
 }  // namespace

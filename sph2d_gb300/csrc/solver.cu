@@ -667,7 +667,10 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
         s->verlet_skin = s->dim == 3 ? kDefaultSkin3 : kDefaultSkin2;
     }
     s->P.keep_cells = G.scattered || tiles_active(s) ? 1 : 0;  // the table is cleared wholesale below
-    if (s->verlet) set_verlet_params(s);
+    if (s->verlet) {
+        s->P.vl_split = tiles_active(s) ? 1 : rrsph::verlet_split(s->dim, (uint32_t)n);
+        set_verlet_params(s);
+    }
     if (cudaMallocHost(&s->h_scal, sizeof(rrsph::StepScalars)) != cudaSuccess ||
         cudaMallocHost(&s->h_flags, sizeof(uint32_t)) != cudaSuccess ||
         cudaHostAlloc(&s->h_report, sizeof(rrsph::HostReport), cudaHostAllocMapped) != cudaSuccess ||
