@@ -121,6 +121,7 @@ struct StepScalars {
     unsigned long long pairs;      // directed pairs found by the density gather of this step
     unsigned long long nwm_off;    // 1 once a one-shot wave maker (wall disappear) has fired
     unsigned long long pairs_total;  // pairs summed over the steps since upload
+    double piston_vx;          // the params' piston at `time` (piston_block, before the whole step)
 };
 
 // ------------------------------------------- FP64-free double handling --

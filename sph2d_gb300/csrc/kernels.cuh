@@ -21,6 +21,8 @@ struct State {
     uint32_t* key_of;          // cell key used by the last grid build, per id
     int32_t* wave_tank;        // piston of each particle in wave_law, -1 for none (null: the params' wave maker)
     const PistonLaw* wave_law; // wave-maker table
+    double* wave_vx;           // its pistons' velocities of this step (piston_block)
+    uint32_t wave_count;
     // FP32-mixed step only (null otherwise), written by the key pass, id order:
     float2* coff2;             // 2D: offset of r from its cell's lower edge
     float4* coff4;             // 3D: the same (x, y, z)
@@ -132,7 +134,7 @@ void launch_forces_fp64(const DevParams& P, const State& S, const Sorted& G, uin
                         uint32_t* flags, int write_mu, cudaStream_t st, int threads, int use_masks = 0);
 // The stored-pair FP64 step (kernels_pairs64.cu) on a grid reordered with kReorderPairs.
 template <int DIM>
-void launch_pair_masks(const DevParams& P, const Sorted& G, cudaStream_t st);
+void launch_pair_masks(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, cudaStream_t st);
 template <int DIM>
 void launch_pair_terms(const DevParams& P, const Sorted& G, cudaStream_t st, int threads);
 template <int DIM>
@@ -150,9 +152,10 @@ template <int DIM>
 void launch_forces_mixed(const DevParams& P, const State& S, const Sorted& G, uint32_t terms, StepScalars* scal,
                          uint32_t* flags, int write_mu, int use_masks, cudaStream_t st, int threads);
 // whole_step; with next_keys also the next step's predict_half_step and key pass.
+// pistons: a kernel of the step has evaluated the piston velocities (piston_block).
 template <int DIM>
 void launch_whole_step(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal_cur,
-                       StepScalars* scal_next, uint32_t* flags, int next_keys, cudaStream_t st);
+                       StepScalars* scal_next, uint32_t* flags, int next_keys, cudaStream_t st, bool pistons = false);
 
 // Neighbour reuse (the FP32-mixed step): the candidate lists
 // are built with the cutoff widened by a skin and reused while no particle has

@@ -159,13 +159,13 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
 // advances the step scalars into scal_next (time += dt, step + 1).
 template <int DIM, int V>
 __global__ void k_whole(DevParams P, State S, Sorted G, const StepScalars* __restrict__ scal,
-                        StepScalars* __restrict__ next, uint32_t* __restrict__ flags, int next_keys) {
+                        StepScalars* __restrict__ next, uint32_t* __restrict__ flags, int next_keys, bool pre) {
     constexpr bool RARE = (V & kVarRare) != 0;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const double dt = step_dt<RARE>(P, scal, flags, i == 0);
     if (i == 0) advance_scalars(P, scal, next, dt);
     if (i >= P.n) return;
-    whole_particle<DIM, V>(P, S, G, i, dt, scal, flags, next_keys, S.ax[i], S.ay[i], DIM == 3 ? S.az[i] : 0.0);
+    whole_particle<DIM, V>(P, S, G, i, dt, scal, flags, next_keys, pre, S.ax[i], S.ay[i], DIM == 3 ? S.az[i] : 0.0);
 }
 
 // cells_start[c] = lower bound of c in the sorted keys, c in [0, max_cells].
@@ -475,13 +475,13 @@ void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherS
 }
 template <int DIM>
 void launch_whole_step(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal_cur,
-                       StepScalars* scal_next, uint32_t* flags, int next_keys, cudaStream_t st) {
+                       StepScalars* scal_next, uint32_t* flags, int next_keys, cudaStream_t st, bool pistons) {
     const int v = (P.density_treatment != 0 ? kVarCont : 0) | (P.avg_vel || P.dt_method == 2 ? kVarRare : 0) |
                   ((DIM == 2 ? S.vpf2 != nullptr : S.vpf4 != nullptr) ? kVarMixed : 0);
     const unsigned b = blocks_for(P.n, 256);
     switch (v) {
 #define RRSPH_WHOLE(V) \
-    case V: k_whole<DIM, V><<<b, 256, 0, st>>>(P, S, G, scal_cur, scal_next, flags, next_keys); break;
+    case V: k_whole<DIM, V><<<b, 256, 0, st>>>(P, S, G, scal_cur, scal_next, flags, next_keys, pistons); break;
         RRSPH_WHOLE(0) RRSPH_WHOLE(1) RRSPH_WHOLE(2) RRSPH_WHOLE(3)
         RRSPH_WHOLE(4) RRSPH_WHOLE(5) RRSPH_WHOLE(6) RRSPH_WHOLE(7)
 #undef RRSPH_WHOLE
@@ -510,7 +510,7 @@ void launch_pack(const DevParams& P, State S, double* r, double* v, uint32_t str
                                  cudaStream_t);                                                                \
     template void launch_reorder<D>(const DevParams&, const State&, const Sorted&, GatherSrc, int, cudaStream_t); \
     template void launch_whole_step<D>(const DevParams&, const State&, const Sorted&, StepScalars*,            \
-                                       StepScalars*, uint32_t*, int, cudaStream_t);                            \
+                                       StepScalars*, uint32_t*, int, cudaStream_t, bool);                      \
     template void launch_neighbour_list<D>(const DevParams&, const Sorted&, uint32_t*, uint32_t*, uint32_t,    \
                                            uint32_t*, cudaStream_t);                                           \
     template void launch_unpack<D>(const DevParams&, State, const double*, const double*, uint32_t, cudaStream_t); \

@@ -30,6 +30,7 @@
 // a mask has bits, are evaluated in place by both particles.
 #include "kernels.cuh"
 #include "neighbour.cuh"
+#include "piston.cuh"
 
 #include <type_traits>
 
@@ -217,7 +218,12 @@ __device__ __forceinline__ Kern cubic(const PairConst& C, double d2) {
 // particle instead, a cell a lane, ran at 14 (3D: 9) lanes of 32: 124 us on the
 // 409k flume, 2.8 ms on 385k particles in 3D.
 template <int DIM>
-__global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_masks(DevParams P, Sorted G) {
+__global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_masks(DevParams P, State S, Sorted G,
+                                                                                        StepScalars* scal) {
+    if (blockIdx.x * 32u >= P.n) {  // the extra block
+        piston_block(P, S, scal);
+        return;
+    }
     using M = Pm<DIM>;
     using T = typename M::T;
     __shared__ uint32_t counts[M::nc][32];
@@ -804,8 +810,9 @@ int pair_slices(uint32_t n) {
 }  // namespace
 
 template <int DIM>
-void launch_pair_masks(const DevParams& P, const Sorted& G, cudaStream_t st) {
-    k_pair_masks<DIM><<<(P.n + 31) / 32, 32 * Pm<DIM>::nc, 0, st>>>(P, G);
+void launch_pair_masks(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, cudaStream_t st) {
+    const unsigned extra = has_pistons(P, S) ? 1 : 0;
+    k_pair_masks<DIM><<<(P.n + 31) / 32 + extra, 32 * Pm<DIM>::nc, 0, st>>>(P, S, G, scal);
 }
 template <int DIM>
 void launch_pair_terms(const DevParams& P, const Sorted& G, cudaStream_t st, int threads) {
@@ -833,7 +840,7 @@ void launch_pair_sum(const DevParams& P, const State& S, const Sorted& G, StepSc
 }
 
 #define RRSPH_INSTANTIATE(D)                                                                                    \
-    template void launch_pair_masks<D>(const DevParams&, const Sorted&, cudaStream_t);                          \
+    template void launch_pair_masks<D>(const DevParams&, const State&, const Sorted&, StepScalars*, cudaStream_t); \
     template void launch_pair_terms<D>(const DevParams&, const Sorted&, cudaStream_t, int);                     \
     template void launch_pair_density<D>(const DevParams&, const State&, const Sorted&, StepScalars*, uint32_t*, \
                                          cudaStream_t);                                                         \

@@ -10,6 +10,7 @@
 // reference's: the same cutoff test). Each particle's build cell stays its
 // reference cell for the cell-relative offsets until the next build.
 #include "mixed_common.cuh"
+#include "piston.cuh"
 #include "step_particle.cuh"
 
 namespace rrsph {
@@ -254,9 +255,13 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
     constexpr uint32_t IDX = Vl<DIM>::index;
     // the force gather may launch now: it waits for this grid at its start (griddepcontrol.wait)
     asm volatile("griddepcontrol.launch_dependents;");
+    if (L > 1 && blockIdx.x * 32u >= P.n) {  // the extra block
+        piston_block(P, S, scal);
+        return;
+    }
     const uint32_t lane = threadIdx.x & 31u, sub = L > 1 ? threadIdx.x >> 5 : 0u;
     const uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = k < P.n;
+    const bool active = k < P.n;
     uint32_t cnt = 0, word = 0;
     Kahan acc{0.0f, 0.0f};
     if (active) {
@@ -586,24 +591,46 @@ __global__ void __launch_bounds__(kTileWarps * 32) k_density_tiles(DevParams P, 
 // are not the ones the key pass writes (P4n, V4n, VD4n), and the list of every
 // particle is complete (the density pass wrote the neighbours of overflowed
 // lists too, which needs at most Vl<DIM>::cap neighbours per particle).
+__device__ __forceinline__ void fetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// The rows whole_particle and its key pass read of particle id.
+template <int DIM>
+__device__ __forceinline__ void fetch_whole(const State& S, uint32_t id) {
+    fetch_l1(S.rx + id);
+    fetch_l1(S.ry + id);
+    fetch_l1(S.vx + id);
+    fetch_l1(S.vy + id);
+    if (DIM == 3) {
+        fetch_l1(S.rz + id);
+        fetch_l1(S.vz + id);
+        fetch_l1(S.boff4 + id);
+    } else {
+        fetch_l1(S.boff + id);
+    }
+    fetch_l1(S.itype + id);
+    fetch_l1(S.key_of + id);
+    fetch_l1(S.bcxy + id);
+    fetch_l1(S.slot + id);
+}
 template <int DIM, int SKF, bool STD, int WV, int L>
 __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_forces_verlet(DevParams P, State S, Sorted G,
                                                                     StepScalars* __restrict__ scal,
                                                                     StepScalars* __restrict__ next,
                                                                     uint32_t* __restrict__ flags) {
     constexpr uint32_t IDX = Vl<DIM>::index;
-    // launched while the density gather finishes: wait for it (and its writes) first
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t lane = threadIdx.x & 31u, sub = L > 1 ? threadIdx.x >> 5 : 0u;
-    const uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = k < P.n;
+    // the warps of a split block meet below: its lanes past the end redo the last particle
+    if (L > 1) k = min(k, P.n - 1u);
     double amag = 0, arvmu_d = 0;
-    Kahan ax{0, 0}, ay{0, 0}, az{0, 0};
-    Kahan avx{0, 0}, avy{0, 0}, avz{0, 0};
-    float arvmu = 0.0f;
-    const bool avel = !STD && P.avg_vel;
-    if (active) {
+    // launched while the density gather finishes: wait for it and its writes; the
+    // split gather first fetches what that does not write (this particle's rows of
+    // the whole step, into L1)
+    if (WV != 0 && L > 1 && sub == 0) fetch_whole<DIM>(S, G.id[k]);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (L > 1 || active) {
         const MixedF& M = P.mf;
+        const uint32_t id = G.id[k];
         const float4 pj4 = G.P4[k];
         const int32_t tj = __float_as_int(pj4.w);
         ForceAcc<DIM, SKF> F{P, G, G.V4[k], G.PR[k], 0.0f, false, false, false, false, false, 0, 0,
@@ -612,10 +639,12 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
         F.ext = P.repulsive && tj > 0;
         F.intf = true;
         F.visc = P.art_visc;
-        F.avel = avel;
+        F.avel = P.avg_vel;
         F.form1 = P.intf_form == 1;
         F.intf_skf = SKF ? SKF : P.intf_skf;
         F.av_skf = SKF ? SKF : P.av_skf;
+        Kahan ax{0, 0}, ay{0, 0}, az{0, 0};
+        Kahan avx{0, 0}, avy{0, 0}, avz{0, 0};
         if (tj != P.type_non_existent) {
             const uint32_t vc = G.vcount[k];
             if (WV != 0 || vc != kListOver) {
@@ -717,57 +746,55 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
                 }
             }
         }
-        arvmu = F.arvmu;
-    }
-    if (L > 1) {  // the other warps' sums, then the first warp goes on alone
-        constexpr int Q = (DIM == 3 ? 3 : 2) * (STD ? 1 : 2);
-        __shared__ float part[L - 1 ? L - 1 : 1][2 * Q + 1][32];
-        auto each = [&](auto&& f) {
-            f(0, ax);
-            f(1, ay);
-            if (DIM == 3) f(2, az);
-            if (!STD) {
-                f(DIM, avx);
-                f(DIM + 1, avy);
-                if (DIM == 3) f(5, avz);
+        if (L > 1) {  // the other warps' sums, then the first warp goes on alone
+            constexpr int Q = (DIM == 3 ? 3 : 2) * (STD ? 1 : 2);
+            __shared__ float part[L - 1 ? L - 1 : 1][2 * Q + 1][32];
+            auto each = [&](auto&& f) {
+                f(0, ax);
+                f(1, ay);
+                if (DIM == 3) f(2, az);
+                if (!STD) {
+                    f(DIM, avx);
+                    f(DIM + 1, avy);
+                    if (DIM == 3) f(5, avz);
+                }
+            };
+            if (sub != 0) {
+                each([&](int q, const Kahan& a) {
+                    part[sub - 1][2 * q][lane] = a.s;
+                    part[sub - 1][2 * q + 1][lane] = a.c;
+                });
+                part[sub - 1][2 * Q][lane] = F.arvmu;
             }
-        };
-        if (sub != 0) {
-            each([&](int q, const Kahan& a) {
-                part[sub - 1][2 * q][lane] = a.s;
-                part[sub - 1][2 * q + 1][lane] = a.c;
-            });
-            part[sub - 1][2 * Q][lane] = arvmu;
-        }
-        __syncthreads();
-        if (sub != 0) return;
+            __syncthreads();
+            if (sub != 0) return;
 #pragma unroll
-        for (int u = 0; u < L - 1; u++) {
-            each([&](int q, Kahan& a) {
-                a.add(part[u][2 * q][lane]);
-                a.c += part[u][2 * q + 1][lane];
-            });
-            arvmu = fmaxf(arvmu, part[u][2 * Q][lane]);
+            for (int u = 0; u < L - 1; u++) {
+                each([&](int q, Kahan& a) {
+                    a.add(part[u][2 * q][lane]);
+                    a.c += part[u][2 * q + 1][lane];
+                });
+                F.arvmu = fmaxf(F.arvmu, part[u][2 * Q][lane]);
+            }
         }
-    }
-    if (active) {
-        const uint32_t id = G.id[k];
-        const double axd = ax.value(), ayd = ay.value() - P.g;  // gravity along y (ExtForce.h), 2D and 3D
-        const double azd = DIM == 3 ? az.value() : 0.0;
-        S.ax[id] = axd;
-        S.ay[id] = ayd;
-        if (DIM == 3) S.az[id] = azd;
-        if (avel) {
-            S.avx[id] = avx.value();
-            S.avy[id] = avy.value();
-            if (DIM == 3) S.avz[id] = avz.value();
-        }
-        arvmu_d = arvmu;
-        if (P.dt_reduce) amag = sqrt(axd * axd + ayd * ayd + azd * azd);
-        if (WV != 0) {
-            const double dt = step_dt<(WV & kVarRare) != 0>(P, scal, flags, k == 0);
-            if (k == 0) advance_scalars(P, scal, next, dt);
-            whole_particle<DIM, WV>(P, S, G, id, dt, scal, flags, 1, axd, ayd, azd);
+        if (L == 1 || active) {
+            const double axd = ax.value(), ayd = ay.value() - P.g;  // gravity along y (ExtForce.h), 2D and 3D
+            const double azd = DIM == 3 ? az.value() : 0.0;
+            S.ax[id] = axd;
+            S.ay[id] = ayd;
+            if (DIM == 3) S.az[id] = azd;
+            if (F.avel) {
+                S.avx[id] = avx.value();
+                S.avy[id] = avy.value();
+                if (DIM == 3) S.avz[id] = avz.value();
+            }
+            arvmu_d = F.arvmu;
+            if (P.dt_reduce) amag = sqrt(axd * axd + ayd * ayd + azd * azd);
+            if (WV != 0) {
+                const double dt = step_dt<(WV & kVarRare) != 0>(P, scal, flags, k == 0);
+                if (k == 0) advance_scalars(P, scal, next, dt);
+                whole_particle<DIM, WV>(P, S, G, id, dt, scal, flags, 1, L > 1, axd, ayd, azd);
+            }
         }
     }
     if (P.dt_method == 2 && P.dt_reduce) {
@@ -804,6 +831,7 @@ template <int DIM>
 void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
                            cudaStream_t st, int threads) {
     const bool cont = P.density_treatment != 0;
+    const unsigned extra = has_pistons(P, S) ? 1 : 0;
 #if RRSPH_DENSITY_CELL_TILES
     if (DIM == 2 && !cont && P.all_cubic) {
         constexpr int tt = kTileWarps * 32;
@@ -814,7 +842,7 @@ void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, 
 #define RRSPH_DV(SKF, CONT)                                                                                           \
     do {                                                                                                              \
         if (P.vl_split == 4)                                                                                          \
-            k_density_verlet<DIM, SKF, CONT, 4><<<(P.n + 31) / 32, 128, 0, st>>>(P, S, G, scal, flags);               \
+            k_density_verlet<DIM, SKF, CONT, 4><<<(P.n + 31) / 32 + extra, 128, 0, st>>>(P, S, G, scal, flags);       \
         else                                                                                                          \
             k_density_verlet<DIM, SKF, CONT, 1><<<(P.n + threads - 1) / threads, threads, 0, st>>>(P, S, G, scal, flags); \
     } while (0)

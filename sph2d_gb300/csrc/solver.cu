@@ -431,8 +431,9 @@ int enqueue_step_verlet(rrsph_solver* s, int par, cudaEvent_t* events, bool with
     else rrsph::launch_forces_verlet<2>(s->P, s->S, s->G, cur, nxt, s->flags, st, s->gather_threads[1], fuse ? 1 : 0);
     if (events) cudaEventRecord(events[5], st);
     if (!fuse) {
-        if (d3) rrsph::launch_whole_step<3>(s->P, s->S, s->G, cur, nxt, s->flags, 1, st);
-        else rrsph::launch_whole_step<2>(s->P, s->S, s->G, cur, nxt, s->flags, 1, st);
+        const bool pistons = s->P.vl_split > 1;  // the split density gather's
+        if (d3) rrsph::launch_whole_step<3>(s->P, s->S, s->G, cur, nxt, s->flags, 1, st, pistons);
+        else rrsph::launch_whole_step<2>(s->P, s->S, s->G, cur, nxt, s->flags, 1, st, pistons);
     }
     if (events) cudaEventRecord(events[6], st);
     s->launches += fuse ? 2 : 3;
@@ -474,7 +475,7 @@ void enqueue_step(rrsph_solver* s, int par, cudaEvent_t* events, bool with_keys)
                                s->stream);
     if (events) cudaEventRecord(events[3], s->stream);
     if (s->pairs64) {
-        rrsph::launch_pair_masks<DIM>(s->P, s->G, s->stream);
+        rrsph::launch_pair_masks<DIM>(s->P, s->S, s->G, cur, s->stream);
         rrsph::launch_pair_terms<DIM>(s->P, s->G, s->stream, s->gather_threads[0]);
         if (!cont) rrsph::launch_pair_density<DIM>(s->P, s->S, s->G, cur, s->flags, s->stream);
         s->launches += cont ? 2 : 3;
@@ -491,7 +492,7 @@ void enqueue_step(rrsph_solver* s, int par, cudaEvent_t* events, bool with_keys)
         enqueue_forces<DIM>(s, RRSPH_TERM_ALL, cur, 0, 1);
     }
     if (events) cudaEventRecord(events[5], s->stream);
-    rrsph::launch_whole_step<DIM>(s->P, s->S, s->G, cur, nxt, s->flags, 1, s->stream);
+    rrsph::launch_whole_step<DIM>(s->P, s->S, s->G, cur, nxt, s->flags, 1, s->stream, s->pairs64);
     if (events) cudaEventRecord(events[6], s->stream);
     s->launches += 2;
 }
@@ -1497,10 +1498,14 @@ extern "C" int rrsph_set_wave_makers(rrsph_solver* s, uint32_t count, const rrsp
         if ((rc = dev_alloc(s, &s->S.wave_tank, n)) != 0) return rc;
     }
     rrsph::PistonLaw* table = nullptr;
+    double* vx = nullptr;
     if ((rc = dev_alloc(s, &table, std::max<size_t>(count, 1))) != 0) return rc;
+    if ((rc = dev_alloc(s, &vx, std::max<size_t>(count, 1))) != 0) return rc;
     RRSPH_CUDA_TRY(cudaMemcpy(s->S.wave_tank, owner.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
     if (count) RRSPH_CUDA_TRY(cudaMemcpy(table, laws.data(), count * sizeof(rrsph::PistonLaw), cudaMemcpyHostToDevice));
     s->S.wave_law = table;
+    s->S.wave_vx = vx;
+    s->S.wave_count = count;
     if (!count) s->S.wave_tank = nullptr;  // an empty table restores the params' wave maker
     return RRSPH_OK;
 }

@@ -8,6 +8,7 @@
 
 #include "kernels.cuh"
 #include "neighbour.cuh"
+#include "piston.cuh"
 
 namespace rrsph {
 namespace {
@@ -161,54 +162,6 @@ __device__ __forceinline__ void predict(const DevParams& P, const State& S, uint
 }
 
 
-// Piston velocity of dynamic_boundaries (RRSPH_OMP/src/WaveMaker.cpp:34-82)
-// for one set of wave-maker parameters.
-__device__ inline double piston_law_vx(int nwm, double phase, double freq, double H, double k, double depth,
-                                double time_start, double time) {
-    const double delta = phase - freq * time_start;
-    const double omega = freq;
-    const double kd = k * depth;
-    const double sh = sinh(kd), ch = cosh(kd);
-    const double m1 = 2 * (sh * sh) / (sh * ch + kd);
-    const double S0 = H / m1;
-    double vx = 0.5 * S0 * omega * cos(omega * time + delta);
-    if (nwm == 3) {
-        const double e2_1 = (H * H) / (32 * depth);
-        const double e2_2 = 3 * ch / (sh * sh * sh) - 2 / m1;
-        vx += 2 * omega * (e2_1 + e2_2) * cos(2 * omega * time + 2 * delta);
-    }
-    return vx;
-}
-
-// The params' piston, or X'(t) of the Fourier piston X(t) = sum_k c_k
-// sin(k omega t) when one is set.
-__device__ inline double piston_vx(const DevParams& P, double time) {
-    if (P.fourier_n > 0) {
-        double vx = 0;
-        for (int k = 1; k <= P.fourier_n; k++) {
-            const double phi = k * P.fourier_omega * cos(k * P.fourier_omega * time);
-            vx += P.fourier_coef[k - 1] * phi;
-        }
-        return vx;
-    }
-    return piston_law_vx(P.nwm, P.nwm_phase, P.nwm_freq, P.nwm_H, P.nwm_k, P.depth, P.nwm_time_start, time);
-}
-
-// Piston velocity of nwm_solitary_rayleigh (WaveMaker.cpp:84-134).
-__device__ inline double solitary_vx(const DevParams& P, double time) {
-    const double H = P.nwm_H, h = P.depth, g = P.g;
-    const double k = sqrt(3 * H / (4 * (h * h) * (H + h)));
-    const double c = sqrt(g * (H + h));
-    const double Tf = 2 / (k * c) * (3.8 + H / h);
-    const double tau = k * c * (time - Tf);
-    const double u = tanh(tau);
-    const double top = k * H * (h + H - H * (u * u)) + 2 * k * ((H * u) * (H * u));
-    const double b = k * (h + H - H * (u * u));
-    const double dxdu = top / (b * b);
-    const double th = tanh(tau);
-    return dxdu * (1 - th * th) * (k * c);
-}
-
 // dt of the step: scal->dt, or update_dt (UpdateAcceleration.cpp:15-29) under
 // DT_CORRECTION_DYNAMIC (with the step's maxima when dt_reduce is set). One
 // thread (first) reports a never-ending dt.
@@ -243,12 +196,13 @@ __device__ __forceinline__ void advance_scalars(const DevParams& P, const StepSc
 
 // The per-particle part of k_whole: make_waves for particle i, whole_step,
 // the boundary check and (next_keys) the next step's predictor + key pass,
-// with the acceleration (ax, ay, az) of this step's force evaluation.
+// with the acceleration (ax, ay, az) of this step's force evaluation. pre: the
+// piston velocities of the step are in scal and S.wave_vx (piston_block).
 template <int DIM, int V>
 __device__ __forceinline__ void whole_particle(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
                                                double dt, const StepScalars* __restrict__ scal,
-                                               uint32_t* __restrict__ flags, int next_keys, double ax, double ay,
-                                               double az) {
+                                               uint32_t* __restrict__ flags, int next_keys, bool pre, double ax,
+                                               double ay, double az) {
     constexpr bool CONT = (V & kVarCont) != 0, RARE = (V & kVarRare) != 0;
     constexpr int M = (V & kVarMixed) ? 1 : 0;
     const double time = scal->time;
@@ -259,14 +213,14 @@ __device__ __forceinline__ void whole_particle(const DevParams& P, const State& 
         if (w >= 0) {
             const PistonLaw L = S.wave_law[w];
             if (time >= L.time_start) {
-                const double vx = piston_law_vx(L.nwm, L.phase, L.freq, L.H, L.k, L.depth, L.time_start, time);
+                const double vx = pre ? S.wave_vx[w] : table_vx(L, time);
                 S.rx[i] = S.rx[i] + vx * dt;
                 S.vx[i] = vx;
             }
         }
     } else if (waves && P.nwm_valid && i >= P.nwm_start && i < P.nwm_end) {
         if (P.nwm == 2 || P.nwm == 3 || P.nwm == 5) {
-            const double vx = P.nwm == 5 ? solitary_vx(P, time) : piston_vx(P, time);
+            const double vx = pre ? scal->piston_vx : params_vx(P, time);
             S.rx[i] = S.rx[i] + vx * dt;
             S.vx[i] = vx;
         } else if (P.nwm == 4) {
