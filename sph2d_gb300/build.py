@@ -28,7 +28,7 @@ LIB = PKG / "librrsph_cuda.so"
 RUNNER = PKG / "rrsph_run"
 
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
-CU_SOURCES = ["sort.cu", "kernels_common.cu", "kernels_fp64.cu", "kernels_pairs64.cu", "kernels_mixed.cu", "kernels_reuse.cu", "solver.cu",
+CU_SOURCES = ["sort.cu", "kernels_common.cu", "kernels_fp64.cu", "kernels_pairs64.cu", "kernels_mixed.cu", "kernels_reuse.cu", "kernels_reuse_cell.cu", "solver.cu",
               "sort_noalloc.cu", "run_loop.cu", "adjoint.cu"]
 CPP_SOURCES = ["params.cpp", "layers.cpp"]
 

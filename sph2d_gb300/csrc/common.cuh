@@ -27,6 +27,24 @@ struct MixedF {
     float dhc;                  // delta-SPH: coef * h * c
 };
 
+// Constants of the mixed step with neighbour reuse (kernels_reuse.cu). Its sums
+// run over the kernel without its factors and are multiplied once at their end by
+// factors kept as two floats. These are products of the float constants of the
+// stencil-search gathers (MixedF), and the separations are scaled to metres before
+// anything else, so that the two differ by random rounding only.
+struct F2 {
+    float hi, lo;
+};
+struct ReuseF {
+    float u;             // position unit in metres
+    F2 w;                // m f: of W / f
+    F2 a;                // m f / (2 h^2): of an acceleration or rate sum
+    F2 m;                // m: the same for other kernels
+    float far;           // h: (q > 1) / distance of the kernel gradient over that factor
+    float visc, bulk;    // -2 alpha c h, 2 beta h
+    float lj_D, lj_r2;   // Lennard-Jones over the acceleration's factor; its squared range
+};
+
 // Constants of the stored-pair FP64 sums (kernels_pairs64.cu), the mass and the
 // cubic kernel's factors multiplied in.
 struct PairConst {
@@ -91,15 +109,15 @@ struct DevParams {
     int dt_reduce;          // 1: true max reduction
     double cfl, never_ending_dt;
     int all_cubic;          // every smoothing kernel choice is the cubic spline
-    // neighbour reuse (mixed step): list cutoff (cell + skin)^2, (skin / 2)^2, and
+    // neighbour reuse (mixed step): on; list cutoff (cell + skin)^2, (skin / 2)^2, and
     // the distance from a cell edge within which the list looks two cells away
+    int reuse;
     float vl_cut2, vl_half_skin2, vl_skin_edge;
     int vl_split;           // warps per 32 particles of its two gathers
-    // 1: the key pass leaves the cell table of the last list build in place
-    // (the cell-tile density pass reads it on reuse steps); each rebuild then
-    // clears the table wholesale before the reorder writes the new one
+    // 1: the key pass leaves the cell table in place (the counting sort rewrites it whole)
     int keep_cells;
     MixedF mf;
+    ReuseF rf;
     PairConst pc;
 };
 
@@ -248,12 +266,19 @@ __device__ inline uint64_t cell_coord(double r, double rmin, double cell) {
 // fraction is more than 2^-30 from an integer its truncation is the
 // quotient's; every other case (outside the geometry, near a cell edge, not
 // finite) takes the exact division. below: r < rmin or r is NaN.
+// fix: (r - rmin) / cell in units of 2^-27, rounded down, modulo 2^32; its whole
+// cells are c's. far: below the grid by more than a cell, beyond what the key's
+// bits hold, or NaN: fix and off do not tell it from a particle of the grid.
+constexpr int kFixBits = 27;
 struct CellSplit {
     uint64_t c;
     float off;   // r - (rmin + c cell), in float
-    bool below;
+    uint32_t fix;
+    bool below, far;
 };
-__device__ inline CellSplit cell_split(double r, double rmin, double cell, double inv_cell, float cellf) {
+template <bool FIX>
+__device__ inline CellSplit cell_split(double r, double rmin, double cell, double inv_cell, float cellf,
+                                       uint32_t cmax = 0) {
     const double q = __dmul_rn(__dsub_rn(r, rmin), inv_cell);
     const long long bits = __double_as_longlong(q);
     if (bits > 0) {
@@ -265,14 +290,23 @@ __device__ inline CellSplit cell_split(double r, double rmin, double cell, doubl
             const unsigned long long top = frac >> (F - 30);
             if (top != 0 && top != (1ull << 30) - 1) {
                 const float f = (float)(uint32_t)(frac >> (F - 24)) * 5.9604644775390625e-8f;  // * 2^-24
-                return {m >> F, f * cellf, false};
+                const uint64_t c = m >> F;
+                return {c, f * cellf, FIX ? (uint32_t)(m >> (F - kFixBits)) : 0u, false, FIX && c > cmax};
             }
         } else if (e < 0 && e >= -30 && !(e == -1 && (m >> 23) == (1ull << 30) - 1)) {
-            return {0, (float)q * cellf, false};
+            return {0, (float)q * cellf, FIX ? (uint32_t)(m >> (52 - e - kFixBits)) : 0u, false, false};
         }
     }
     const uint64_t c = cell_coord(r, rmin, cell);
-    return {c, (float)(r - (rmin + (double)c * cell)), !(r >= rmin)};
+    const double off = r - (rmin + (double)c * cell);
+    CellSplit s{c, (float)off, 0u, !(r >= rmin), false};
+    if (FIX) {
+        const double one = (double)(1 << kFixBits), in = off * inv_cell;
+        s.far = c > cmax || !(in >= -1.0);
+        if (s.below) s.fix = fabs(in) < 1e10 ? (uint32_t)(long long)floor(in * one) : 0u;
+        else s.fix = ((uint32_t)c << kFixBits) + (uint32_t)fmin(fmax(in * one, 0.0), one - 1.0);
+    }
+    return s;
 }
 
 // Neighbour-cell coordinate steps (GridUtils.h:158-163).

@@ -29,14 +29,39 @@ struct State {
     float2* vpf2;              // 2D: v_predict in float
     float4* vpf4;              // 3D: the same (x, y, z)
     // mixed step with neighbour reuse (null otherwise), id order:
-    uint32_t* cxy;             // cell coordinates of the current position, x | y << 16 (3D: x | y << 10 | z << 20)
-    uint32_t* bcxy;            // cell coordinates at the last list build
+    int2* fix2;                // 2D: fixed-point position (Pos)
+    int4* fix4;                // 3D: the same (x, y, z)
+    int2* bfix2;               // 2D: the same at the last list build
+    int4* bfix4;               // 3D
+    uint32_t* bcxy;            // kReuseCell: cell coordinates at the last list build, x | y << 16
+    float2* boff;              // kReuseCell: offset from that cell's edges at the last list build
     uint32_t* slot;            // cell-order index at the last list build
-    float2* boff;              // 2D: offset from that cell's edges at the last list build
-    float4* boff4;             // 3D: the same (x, y, z)
+    uint32_t* vl_far;          // non-zero: some particle is outside the grid (CellSplit::far); [1]: at the last rebuild
     uint32_t* vl_rebuild;      // non-zero: the next step rebuilds the grid and the lists
-    uint32_t* vl_gone;         // the last build: bit 0 left out non-existent particles, bit 1 overflowed a list
+    uint32_t* vl_gone;         // the last build: bit 0 left out non-existent particles, bit 1 searched particles
     uint32_t* itype_changed;   // non-zero once a step changed a particle's type since the last upload
+};
+
+// A position in fixed point: 2^27 units a cell from the grid's origin, modulo 2^32
+// (32 cells): the difference of two words is the separation of particles less
+// than 16 cells apart. code carries the particle's kind in a float that is added to
+// a squared distance: 0 fluid, -0 boundary, the smallest subnormal for other
+// types; +inf absent (non-existent); NaN, low bits as before, for a particle
+// outside the grid, which no list holds.
+struct __align__(16) Pos {
+    int x, y, z;
+    float code;
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t bits() const { return __float_as_uint(code); }
+    __device__ __forceinline__ bool absent() const { return bits() == 0x7F800000u; }
+    __device__ __forceinline__ bool unlisted() const { return (bits() & 0x7FC00000u) == 0x7FC00000u; }
+    __device__ __forceinline__ bool fluid() const { return (bits() & 0x80000001u) == 0u; }
+    __device__ __forceinline__ bool boundary() const { return (int)bits() < 0; }
+    static __device__ __forceinline__ float code_of(int32_t type, int32_t type_absent, bool far) {
+        if (type == type_absent) return __uint_as_float(0x7F800000u);
+        return __uint_as_float((type > 0 ? 0u : (type < 0 ? 0x80000000u : 1u)) | (far ? 0x7FC00000u : 0u));
+    }
+#endif
 };
 
 // Per-step cell-ordered copies and the grid.
@@ -61,10 +86,12 @@ struct Sorted {
     float4* V4;    // velocity the forces use + density the forces use
     float4* VD4;   // v + (rho - rho0) for density_con
     float2* PR;    // pressure p and p / rho^2 (rho = the density the forces use)
-    // mixed step with neighbour reuse: the P4 / V4 (/ VD4 with continuity
-    // density) of the next step, which the key pass writes at each particle's
-    // build slot (the two buffers alternate)
-    float4* P4n;
+    // mixed step with neighbour reuse: positions (in P4's buffer), with a row n of
+    // an absent particle; and the positions / V4 (/ VD4 with continuity density) of
+    // the next step, which the key pass writes at each particle's build slot (the
+    // two buffers alternate)
+    Pos* pos;
+    Pos* posn;
     float4* V4n;
     float4* VD4n;
     // Neighbour masks written by the density pass for the force pass (the FP64
@@ -90,16 +117,14 @@ struct Sorted {
     double* ps;        // [cap][n], summation density: kernel gradient of owned pair number o
     uint8_t* prank;    // [cap][n]: its owner's number among the neighbours of the other particle
     // mixed step with neighbour reuse: up to kVerletCap2 (2D) / kVerletCap3 (3D)
-    // candidates per particle, sorted index | cell code << 27 (3D: << 25) with
-    // code = (dx + 2) * 5 + (dy + 2) (3D: ((dx + 2) * 5 + (dy + 2)) * 5 + (dz + 2))
-    // for the candidate's cell offset, stored in slabs of four: entries 4g..4g+3
-    // of particle k are the uint4 at (uint4*)list + g * n + k (the lanes of a
-    // warp read neighbouring uint4s), the last group padded with kVlNone;
-    // vcount[k] = candidates (kListOver: too many, searched instead). This
-    // step's neighbours (the candidates within the cutoff, in list order) in the
-    // same slab layout: nlist, ncount[k] of them; words past ncount are stale.
-    // With split gathers (vl_split = 4) sub-list u of a particle takes the groups
-    // u, u + 4, ... and ncount[k] holds four counts of 8 bits.
+    // candidates per particle as sorted indices, stored in slabs of four: entries
+    // 4g..4g+3 of particle k are the uint4 at (uint4*)vlist + g * n + k (the lanes of
+    // a warp read neighbouring uint4s), the last group padded with index n (an absent
+    // particle); vcount[k] = candidates, or kListOver: the particle is searched
+    // instead. This step's neighbours (the candidates within the cutoff, in list
+    // order) in the same slab layout: nlist, ncount[k] of them; words past ncount are
+    // stale. With split gathers (vl_split = 4) sub-list u of a particle takes the
+    // groups u, u + 4, ... and ncount[k] holds four counts of 8 bits.
     uint32_t* vlist;
     uint32_t* vcount;
     uint32_t* nlist;
@@ -118,7 +143,7 @@ template <int DIM>
 void launch_keys(const DevParams& P, const State& S, Sorted& G, StepScalars* scal, int predict, uint32_t* flags,
                  cudaStream_t st);
 // for_whom: the gathers the cell-order copies are for.
-enum : int { kReorderFp64 = 0, kReorderMixed = 1, kReorderPairs = 2 };
+enum : int { kReorderFp64 = 0, kReorderMixed = 1, kReorderPairs = 2, kReorderReuse = 3 };
 template <int DIM>
 void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int for_whom,
                     cudaStream_t st);
@@ -161,7 +186,8 @@ void launch_whole_step(const DevParams& P, const State& S, const Sorted& G, Step
 // are built with the cutoff widened by a skin and reused while no particle has
 // moved more than half the skin since the build (kernels_reuse.cu).
 void launch_verlet_decide(cudaGraphConditionalHandle h, const uint32_t* rebuild, cudaStream_t st);
-void launch_verlet_reset(uint32_t* rebuild, uint32_t* gone, unsigned long long* builds, cudaStream_t st);
+void launch_verlet_reset(uint32_t* rebuild, uint32_t* gone, uint32_t* far, unsigned long long* builds,
+                         cudaStream_t st);
 // After an upload: the lists stay valid unless the last build left out a
 // non-existent particle (which may exist now); moves are checked by the key pass.
 void launch_verlet_upload_check(uint32_t* rebuild, const uint32_t* gone, cudaStream_t st);
@@ -223,12 +249,6 @@ template <int DIM>
 void launch_download_direct(const DevParams& P, const State& S, double* r, double* v, double* rho, double* p,
                             int32_t* itype, uint32_t stride, cudaStream_t st, const uint32_t* itype_if = nullptr);
 
-// Compile-time variant: the cell-tile density pass of the 2D mixed step with
-// neighbour reuse (summation density, cubic kernel) instead of the
-// candidate-list pass (kernels_reuse.cu).
-#ifndef RRSPH_DENSITY_CELL_TILES
-#define RRSPH_DENSITY_CELL_TILES 0
-#endif
 // Stored values per particle of the FP64 pair sums: about 20 neighbours in 2D
 // and 80 in 3D (120 to 160 beside the half-spaced walls); more are evaluated in place.
 constexpr uint32_t kPairCap2 = 48;
@@ -236,10 +256,14 @@ constexpr uint32_t kPairCap3 = 160;
 constexpr int kVerletCap2 = 64;         // candidate-list entries per particle, 2D
 constexpr int kVerletCap3 = 256;        // and 3D
 inline int verlet_cap(int dim) { return dim == 3 ? kVerletCap3 : kVerletCap2; }
-// particles a list entry can index (the cell code takes the top bits)
+// particles the reuse step takes
 inline uint64_t verlet_max_particles(int dim) { return dim == 3 ? (1ull << 25) : (1ull << 27); }
+// DevParams::reuse: fixed-point positions (kernels_reuse.cu), or cell-relative
+// floats (kernels_reuse_cell.cu: 2D with split gathers), whose list entries hold a
+// cell code above a 27-bit index.
+enum : int { kReuseFixed = 1, kReuseCell = 2 };
+constexpr uint32_t kCellEntryIndex = (1u << 27) - 1u;
 constexpr uint32_t kListOver = 0xFFFFFFFFu;
-constexpr uint32_t kVlNone = 0xFFFFFFFFu;  // padding of a list row (never an entry)
 constexpr int kGatherThreads = 128;     // default block size of the pair gathers
 constexpr int kMaxGatherThreads = 256;
 

@@ -32,7 +32,8 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
 // R: 0 = FP64 gathers; 1 = the mixed loop with summation density; 2 = the
 // mixed loop with continuity density; 3 = mixed, outside the loop (the
 // velocities, density and pressure given by F, double copies for exports);
-// 4 = the stored-pair FP64 step (packed rows; with continuity density the
+// 5, 6 = the mixed loop with neighbour reuse, as 1 and 2 but with fixed-point
+// positions; 4 = the stored-pair FP64 step (packed rows; with continuity density the
 // pressure too, which waits for no sum).
 template <int DIM, int R>
 __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
@@ -115,9 +116,31 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
         }
         return;
     }
-    // FP32-mixed: cell-relative offsets the key pass computed from the same positions
-    float ox, oy, oz = 0.0f;
-    if (DIM == 2) {
+    // FP32-mixed: cell-relative offsets, or the fixed-point position, that the key pass
+    // computed from the same positions
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+    if (R == 5 || R == 6) {
+        Pos q{0, 0, 0, 0.0f};
+        if (DIM == 2) {
+            const int2 f = S.fix2[id];
+            q.x = f.x;
+            q.y = f.y;
+        } else {
+            const int4 f = S.fix4[id];
+            q.x = f.x;
+            q.y = f.y;
+            q.z = f.z;
+        }
+        bool far = false;
+        if (S.vl_far[1]) {  // some particle is outside the grid: this one?
+            constexpr uint32_t cmax = DIM == 3 ? 0x3FFu : 0xFFFFu;
+            far = cell_split<true>(S.rx[id], P.xmin, P.cell, P.inv_cell, P.mf.cell, cmax).far ||
+                  cell_split<true>(S.ry[id], P.ymin, P.cell, P.inv_cell, P.mf.cell, cmax).far;
+            if (DIM == 3) far = far || cell_split<true>(S.rz[id], P.zmin, P.cell, P.inv_cell, P.mf.cell, cmax).far;
+        }
+        q.code = Pos::code_of(t, P.type_non_existent, far);
+        G.pos[k] = q;
+    } else if (DIM == 2) {
         const float2 o = S.coff2[id];
         ox = o.x;
         oy = o.y;
@@ -127,7 +150,7 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
         oy = o.y;
         oz = o.z;
     }
-    G.P4[k] = make_float4(ox, oy, oz, __int_as_float(t));
+    if (R != 5 && R != 6) G.P4[k] = make_float4(ox, oy, oz, __int_as_float(t));
     float fvx, fvy, fvz = 0.0f, frho = 0.0f;  // the loop's summation density writes .w itself
     if (R != 3) {  // v_predict in float from the predictor
         if (DIM == 2) {
@@ -140,7 +163,7 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
             fvy = v.y;
             fvz = v.z;
         }
-        if (R == 2) frho = d2f(F.rho[id]);
+        if (R == 2 || R == 6) frho = d2f(F.rho[id]);
     } else {
         fvx = d2f(F.vx[id]);
         fvy = d2f(F.vy[id]);
@@ -149,7 +172,7 @@ __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
         if (F.p) G.PR[k] = make_float2(d2f(F.p[id]), d2f(F.p[id] / (F.rho[id] * F.rho[id])));
     }
     G.V4[k] = make_float4(fvx, fvy, fvz, frho);
-    if (R == 2 || (R == 3 && P.density_treatment != 0))  // rho - rho0 keeps rho_i - rho_j accurate in float
+    if (R == 2 || R == 6 || (R == 3 && P.density_treatment != 0))  // rho - rho0 keeps rho_i - rho_j accurate in float
         G.VD4[k] = vd4_of<DIM>(S.vx[id], S.vy[id], DIM == 3 ? S.vz[id] : 0.0, S.rho[id] - P.rho0);
 }
 
@@ -469,6 +492,8 @@ void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherS
     const unsigned b = blocks_for(P.n, 256);
     if (for_whom == kReorderPairs) k_reorder<DIM, 4><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else if (for_whom == kReorderFp64) k_reorder<DIM, 0><<<b, 256, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderReuse && P.density_treatment == 0) k_reorder<DIM, 5><<<b, 256, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderReuse) k_reorder<DIM, 6><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else if (!fsrc.loop) k_reorder<DIM, 3><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else if (P.density_treatment == 0) k_reorder<DIM, 1><<<b, 256, 0, st>>>(P, S, G, fsrc);
     else k_reorder<DIM, 2><<<b, 256, 0, st>>>(P, S, G, fsrc);

@@ -7,11 +7,22 @@
 // when the grid was last built; while no particle has moved more than skin/2
 // since then, every pair within the cutoff is in the lists, and each step
 // tests the list instead of the 3^dim stencil cells (the pair set is the
-// reference's: the same cutoff test). Each particle's build cell stays its
-// reference cell for the cell-relative offsets until the next build.
-#include "mixed_common.cuh"
-#include "piston.cuh"
-#include "step_particle.cuh"
+// reference's: the same cutoff test).
+//
+// Positions are fixed point, kFixOne units a cell, modulo 2^32 (kernels.cuh,
+// Pos): the separation of two particles within 16 cells of each other is the
+// difference of their words whatever cells they are in, so a list entry is a bare
+// index and a pair's separation costs a subtraction and a conversion per axis.
+// The density pass writes the candidates that are neighbours as a second list for
+// the force pass, four entries a store. (Cell-relative floats with a cell code per
+// entry, decoded by both passes, and single-word list stores took 95 and 100
+// instructions a pair, and the stores three quarters of the density pass's L2
+// traffic. One bit a candidate instead of a second list left the force gather
+// with 23 of 32 lanes: 68 us on the flume.) us per step, before and after: 409k
+// flume 123.6 / 116, 1.06M 3D dam break 824 / 718, 928k ensemble 254 / 235, 43k
+// delta-SPH dam break 39.4 / 36.1. The 16-byte neighbour loads bound both passes
+// now: L1 79 % busy in the density pass, loads in flight in the force pass.
+#include "reuse.cuh"
 
 namespace rrsph {
 
@@ -23,53 +34,103 @@ constexpr int kVlBatch = 4;       // list entries the density gather loads toget
 template <int DIM, bool STD>
 constexpr int kVlForceBatch = DIM == 2 && STD ? 4 : 2;
 
-// List entry = sorted index | cell code << Vl<DIM>::shift, with the code of
-// the candidate's cell offset (dx, dy[, dz]) in [-2, 2]^dim:
-// (dx + 2) * 5 + (dy + 2) in 2D, ((dx + 2) * 5 + (dy + 2)) * 5 + (dz + 2) in 3D.
 template <int DIM>
 struct Vl {
     static constexpr int cap = DIM == 3 ? kVerletCap3 : kVerletCap2;
-    static constexpr int shift = DIM == 3 ? 25 : 27;
-    static constexpr uint32_t index = (1u << shift) - 1u;
     static constexpr uint32_t cmax = DIM == 3 ? 0x3FFu : kMaxCellCoord2;  // largest cell coordinate of a key
 };
 
-template <int DIM>
-__device__ __forceinline__ uint32_t vl_code(int dx, int dy, int dz) {
-    const int c = DIM == 3 ? ((dx + 2) * 5 + (dy + 2)) * 5 + (dz + 2) : (dx + 2) * 5 + (dy + 2);
-    return (uint32_t)c << Vl<DIM>::shift;
+// The split gathers (L > 1): a block of L warps takes 32 particles, warp `sub`
+// their list groups sub, sub + L, ..., and the first warp adds the partial sums up
+// and goes on alone. With few particles a thread walking its whole list is one
+// long chain of dependent loads on a nearly empty chip.
+// A warp's neighbours go to the slab groups it reads (sub + L j), so no warp waits
+// for another's count; the L counts share the particle's word.
+template <int L>
+constexpr uint32_t kCountBits = 32 / L;
+template <int L>
+__device__ __forceinline__ uint32_t sub_count(uint32_t word, uint32_t sub) {
+    return L == 1 ? word : (word >> (sub * kCountBits<L>)) & ((1u << (kCountBits<L> & 31u)) - 1u);
 }
-// The offset of an entry's code, shifted by +2 per axis (0..4).
-template <int DIM>
-__device__ __forceinline__ void vl_offset(uint32_t en, uint32_t& cx, uint32_t& cy, uint32_t& cz) {
-    const uint32_t c = en >> Vl<DIM>::shift;
-    if (DIM == 3) {
-        cx = c / 25u;
-        const uint32_t r = c - 25u * cx;
-        cy = r / 5u;
-        cz = r - 5u * cy;
-    } else {
-        cx = (c * 13u) >> 6;  // c / 5, exact for c < 32
-        cy = c - 5u * cx;
-        cz = 0;
-    }
+// The word of a list of c entries stored in consecutive groups.
+template <int L>
+__device__ __forceinline__ uint32_t packed_counts(uint32_t c) {
+    if (L == 1) return c;
+    uint32_t word = 0;
+    for (uint32_t g = 0; 4 * g < c; g++) word += min(4u, c - 4 * g) << ((g % L) * kCountBits<L>);
+    return word;
 }
 
-// The cubic W(q) of kernel_wf as selects: every lane runs the same instructions.
-__device__ __forceinline__ float cubic_wf_sel(float f, float q) {
-    const float t = 2.0f - q;
-    const float w1 = f * ((2.0f / 3.0f - q * q) + q * q * q * 0.5f);
-    const float w2 = f * ((1.0f / 6.0f) * (t * t * t));
-    return q <= 1.0f ? w1 : (q <= 2.0f ? w2 : 0.0f);
+// Separation of two positions in metres, exact before the conversion.
+template <int DIM>
+__device__ __forceinline__ float3 separation(const Pos& i, const Pos& j, float u) {
+    auto diff = [](int a, int b) { return (float)(int)((uint32_t)a - (uint32_t)b); };
+    return make_float3(diff(i.x, j.x) * u, diff(i.y, j.y) * u, DIM == 3 ? diff(i.z, j.z) * u : 0.0f);
 }
+// Squared distance, + the neighbour's code: nothing for a live particle, infinite
+// or NaN (never below a cutoff) for one that is absent or not listed.
+template <int DIM>
+__device__ __forceinline__ float distance2(float3 d, float code) {
+    return DIM == 3 ? fmaf(d.x, d.x, fmaf(d.y, d.y, fmaf(d.z, d.z, code))) : fmaf(d.x, d.x, fmaf(d.y, d.y, code));
+}
+// The reference's cutoff test in double (inside the guard band, and for a
+// particle outside the grid): rare, so the positions come from the id-order state.
+template <int DIM>
+__device__ __noinline__ bool exact_pair(const DevParams& P, const State& S, uint32_t a, uint32_t b) {
+    const double dx = __dsub_rn(S.rx[a], S.rx[b]), dy = __dsub_rn(S.ry[a], S.ry[b]);
+    const double dz = DIM == 3 ? __dsub_rn(S.rz[a], S.rz[b]) : 0.0;
+    return exact_dist2<DIM>(dx, dy, dz) < P.cut2;
+}
+// The stencil search's test of particle i (sorted) against k: an absent one never,
+// one outside the grid in double.
+template <int DIM>
+__device__ __forceinline__ bool searched_pair(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
+                                              uint32_t k, const Pos& pi, const Pos& pk) {
+    if (pi.absent()) return false;
+    if (pi.unlisted() || pk.unlisted()) return exact_pair<DIM>(P, S, G.id[i], G.id[k]);
+    const float d2 = distance2<DIM>(separation<DIM>(pi, pk, P.rf.u), pi.code);
+    if (d2 < P.mf.cut2_lo) return true;
+    return d2 < P.mf.cut2_hi && exact_pair<DIM>(P, S, G.id[i], G.id[k]);
+}
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// The cubic spline: W / f with q = |r| / h ...
+__device__ __forceinline__ float cubic_w(float q) {
+    const float t = 2.0f - q;
+    const float far = (1.0f / 6.0f) * (t * (t * t));
+    const float near = fmaf(q * q, fmaf(0.5f, q, -1.0f), 2.0f / 3.0f);
+    return q <= 1.0f ? near : far;
+}
+// ... and s with dW/dr = diff s f / (2 h^2) (rs: 1 / distance).
+__device__ __forceinline__ float cubic_s(const ReuseF& U, float q, float rs) {
+    const float t = 2.0f - q;
+    const float far = -(rs * U.far) * (t * t);
+    const float near = fmaf(3.0f, q, -4.0f);
+    return q <= 1.0f ? near : far;
+}
+// 1 / distance, of coincident particles large enough to give q = 0.
+__device__ __forceinline__ float inv_distance(float d2) { return rsqrtf(fmaxf(d2, 1e-30f)); }
+
+// A compensated sum times a factor, as an unevaluated sum of two floats.
+__device__ __forceinline__ F2 scaled(const Kahan& a, F2 f) {
+    const float hi = a.s * f.hi;
+    return {hi, fmaf(a.s, f.hi, -hi) + (a.s * f.lo - a.c * f.hi)};
+}
+__device__ __forceinline__ double value(F2 v) { return f2d(v.hi) + f2d(v.lo); }
 
 __global__ void k_vl_decide(cudaGraphConditionalHandle h, const uint32_t* __restrict__ rebuild) {
     cudaGraphSetConditional(h, *rebuild ? 1u : 0u);
 }
 __global__ void k_vl_reset(uint32_t* __restrict__ rebuild, uint32_t* __restrict__ gone,
-                           unsigned long long* __restrict__ builds) {
+                           uint32_t* __restrict__ far, unsigned long long* __restrict__ builds) {
     *rebuild = 0u;
     *gone = 0u;
+    far[1] = far[0];  // for this rebuild; the next key pass raises its own
+    far[0] = 0u;
     *builds += 1ull;
 }
 // After an upload: a flag raised by the key pass that ran for the replaced
@@ -98,39 +159,47 @@ __device__ __forceinline__ float gap_to_cell(int d, float p, float cell) {
 
 // After this step's grid (sort + reorder): each particle's candidates, four
 // entries gathered in registers and stored as one uint4 into the group's slab
-// (the lanes of a warp store neighbouring uint4s), in cell order x outer.
+// (the lanes of a warp store neighbouring uint4s), in cell order x outer, the last
+// group padded with the row of an absent particle (index n). A particle outside
+// the grid gets no list: it is searched, as is one with too many candidates.
 template <int DIM>
 __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, State S, Sorted G) {
     constexpr int CAP = Vl<DIM>::cap;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.n) return;
-    const MixedF& M = P.mf;
+    const ReuseF& U = P.rf;
+    const float cell = P.mf.cell;
     const uint32_t id = G.id[k], key = G.key[k];
-    const float4 pj = G.P4[k];
+    const Pos pj = G.pos[k];
     uint32_t cx, cy, cz = 0;
     if (DIM == 3) {
         cx = third_bits(key);
         cy = third_bits(key >> 1);
         cz = third_bits(key >> 2);
-        S.bcxy[id] = cx | (cy << 10) | (cz << 20);
-        S.boff4[id] = make_float4(pj.x, pj.y, pj.z, 0.0f);
+        S.bfix4[id] = make_int4(pj.x, pj.y, pj.z, 0);
     } else {
         cx = second_bits(key);
         cy = second_bits(key >> 1);
-        S.bcxy[id] = cx | (cy << 16);
-        S.boff[id] = make_float2(pj.x, pj.y);
+        S.bfix2[id] = make_int2(pj.x, pj.y);
     }
     S.slot[id] = k;
     uint4* const slab = reinterpret_cast<uint4*>(G.vlist) + k;  // group g at slab[g * n]
-    uint4 buf = make_uint4(kVlNone, kVlNone, kVlNone, kVlNone);
+    uint4 buf = make_uint4(P.n, P.n, P.n, P.n);
     uint32_t nl = 0;
-    if (__float_as_int(pj.w) == P.type_non_existent) atomicOr(S.vl_gone, 1u);
-    if (__float_as_int(pj.w) != P.type_non_existent) {
+    if (pj.absent()) atomicOr(S.vl_gone, 1u);
+    // offset from the lower edges of the key's cell
+    const float px = (float)(int)((uint32_t)pj.x - (cx << kFixBits)) * U.u;
+    const float py = (float)(int)((uint32_t)pj.y - (cy << kFixBits)) * U.u;
+    const float pz = DIM == 3 ? (float)(int)((uint32_t)pj.z - (cz << kFixBits)) * U.u : 0.0f;
+    // searched: a particle outside the grid, which no list holds, and where there is
+    // one also those less than a cell below the grid's edge, which may meet it
+    const bool outside = !pj.absent() && (pj.unlisted() || (S.vl_far[1] && (px < 0.0f || py < 0.0f || pz < 0.0f)));
+    if (!pj.absent() && !outside) {
         const float edge = P.vl_skin_edge;
         int x0, x1, y0, y1, z0 = 0, z1 = 0;
-        vl_window<DIM>(pj.x, cx, M.cell, edge, x0, x1);
-        vl_window<DIM>(pj.y, cy, M.cell, edge, y0, y1);
-        if (DIM == 3) vl_window<DIM>(pj.z, cz, M.cell, edge, z0, z1);
+        vl_window<DIM>(px, cx, cell, edge, x0, x1);
+        vl_window<DIM>(py, cy, cell, edge, y0, y1);
+        if (DIM == 3) vl_window<DIM>(pz, cz, cell, edge, z0, z1);
 #pragma unroll 1
         for (int dx = x0; dx <= x1; dx++) {
 #pragma unroll 1
@@ -141,37 +210,30 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, Sta
                     // particle holds no candidate: the distance from the particle
                     // to the cell's nearest side, per axis (the window's corner and
                     // far diagonal cells mostly)
-                    const float gx = gap_to_cell(dx, pj.x, M.cell), gy = gap_to_cell(dy, pj.y, M.cell);
-                    const float gz = DIM == 3 ? gap_to_cell(dz, pj.z, M.cell) : 0.0f;
+                    const float gx = gap_to_cell(dx, px, cell), gy = gap_to_cell(dy, py, cell);
+                    const float gz = DIM == 3 ? gap_to_cell(dz, pz, cell) : 0.0f;
                     if (gx * gx + gy * gy + gz * gz >= P.vl_cut2) continue;
-                    const uint32_t cell = DIM == 3 ? split3_32(cx + dx) | (split3_32(cy + dy) << 1) |
-                                                         (split3_32(cz + dz) << 2)
-                                                   : split2_32(cx + dx) | (split2_32(cy + dy) << 1);
-                    if (cell >= P.max_cells) continue;
-                    const uint32_t s = G.cell_start[cell];
+                    const uint32_t c = DIM == 3 ? split3_32(cx + dx) | (split3_32(cy + dy) << 1) |
+                                                      (split3_32(cz + dz) << 2)
+                                                : split2_32(cx + dx) | (split2_32(cy + dy) << 1);
+                    if (c >= P.max_cells) continue;
+                    const uint32_t s = G.cell_start[c];
                     if (s == kEmpty) continue;
-                    const uint32_t e = G.cell_end[cell];
-                    const float shx = (float)dx * M.cell - pj.x;
-                    const float shy = (float)dy * M.cell - pj.y;
-                    const float shz = DIM == 3 ? (float)dz * M.cell - pj.z : 0.0f;
-                    const uint32_t code = vl_code<DIM>(dx, dy, dz);
+                    const uint32_t e = G.cell_end[c];
                     // the cell's particles four at a time: their loads issue together (an
                     // index past the cell's end loads its last particle and is skipped)
                     for (uint32_t i0 = s; i0 < e; i0 += kVlBatch) {
-                        float4 q[kVlBatch];
+                        Pos q[kVlBatch];
 #pragma unroll
-                        for (int u = 0; u < kVlBatch; u++) q[u] = G.P4[min(i0 + u, e - 1u)];
+                        for (int u = 0; u < kVlBatch; u++) q[u] = G.pos[min(i0 + u, e - 1u)];
 #pragma unroll
                         for (int u = 0; u < kVlBatch; u++) {
                             const uint32_t i = i0 + u;
-                            // past the cell's end, itself, or non-existent (stays so): no candidate
-                            if (i >= e || i == k || __float_as_int(q[u].w) == P.type_non_existent) continue;
-                            const float ddx = q[u].x + shx, ddy = q[u].y + shy, ddz = DIM == 3 ? q[u].z + shz : 0.0f;
-                            const float d2 = DIM == 3 ? ddx * ddx + ddy * ddy + ddz * ddz : ddx * ddx + ddy * ddy;
-                            if (d2 < P.vl_cut2) {
+                            if (i >= e || i == k) continue;
+                            if (distance2<DIM>(separation<DIM>(q[u], pj, U.u), q[u].code) < P.vl_cut2) {
                                 if (nl < (uint32_t)CAP) {
                                     // shifted in: the group's entries in order once its fourth arrives
-                                    buf = make_uint4(buf.y, buf.z, buf.w, i | code);
+                                    buf = make_uint4(buf.y, buf.z, buf.w, i);
                                     if ((nl & 3u) == 3u) slab[(size_t)(nl >> 2) * P.n] = buf;
                                 }
                                 nl++;
@@ -184,75 +246,53 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, Sta
     }
     if (nl < (uint32_t)CAP && (nl & 3u)) {  // the padded last group: its m entries to the front
         const uint32_t m = nl & 3u;
-        buf = m == 1u ? make_uint4(buf.w, kVlNone, kVlNone, kVlNone)
-                      : (m == 2u ? make_uint4(buf.z, buf.w, kVlNone, kVlNone) : make_uint4(buf.y, buf.z, buf.w, kVlNone));
+        buf = m == 1u ? make_uint4(buf.w, P.n, P.n, P.n)
+                      : (m == 2u ? make_uint4(buf.z, buf.w, P.n, P.n) : make_uint4(buf.y, buf.z, buf.w, P.n));
         slab[(size_t)(nl >> 2) * P.n] = buf;
     }
-    G.vcount[k] = nl <= (uint32_t)CAP ? nl : kListOver;
-    if (nl > (uint32_t)CAP) {  // its search needs a fresh grid each step
+    const bool search = outside || nl > (uint32_t)CAP;
+    G.vcount[k] = search ? kListOver : nl;
+    if (search) {  // needs a fresh grid each step
         atomicOr(S.vl_rebuild, 1u);
         atomicOr(S.vl_gone, 2u);
     }
 }
 
-// The split gathers (L > 1): a block of L warps takes 32 particles, warp `sub`
-// their list groups sub, sub + L, ..., and the first warp adds the partial sums up
-// and goes on alone. With few particles a thread walking its whole list is one
-// long chain of dependent loads on a nearly empty chip. A warp's neighbours go to
-// the slab groups it reads (sub + L j), so no warp waits for another's count; the
-// L counts share the particle's word.
-template <int L>
-constexpr uint32_t kCountBits = 32 / L;
-template <int L>
-__device__ __forceinline__ uint32_t sub_count(uint32_t word, uint32_t sub) {
-    return L == 1 ? word : (word >> (sub * kCountBits<L>)) & ((1u << (kCountBits<L> & 31u)) - 1u);
-}
-// Slab offset of neighbour e of warp `sub` (in words, from the particle's uint4).
-template <int L>
-__device__ __forceinline__ size_t slab_at(uint32_t n, uint32_t sub, uint32_t e) {
-    return (size_t)(L == 1 ? e >> 2 : sub + L * (e >> 2)) * 4 * n + (e & 3u);
-}
-// The word of a list of c entries stored in consecutive groups.
-template <int L>
-__device__ __forceinline__ uint32_t packed_counts(uint32_t c) {
-    if (L == 1) return c;
-    uint32_t word = 0;
-    for (uint32_t g = 0; 4 * g < c; g++) word += min(4u, c - 4 * g) << ((g % L) * kCountBits<L>);
-    return word;
-}
-
-// One candidate's contribution to the density gather: W (summation) or the
-// continuity rate with its delta-SPH term (density_con, Density.h:63-114,
-// the same arithmetic as k_density_mixed).
+// One neighbour's term of the density gather, to be multiplied by term_factor():
+// W (summation) or the continuity rate with its delta-SPH term (density_con,
+// Density.h:63-114).
 template <int DIM, int SKF, bool CONT>
-__device__ __forceinline__ float density_term(const MixedF& M, int skf, float f, float dx, float dy, float dz,
-                                              float d2, float4 vdi, float4 vdj, bool delta) {
-    const float inv_dist = rsqrtf(d2);
-    const float q = d2 * inv_dist * M.inv_h;
-    if (!CONT) return SKF == 1 ? cubic_wf_sel(f, q) : kernel_wf(skf, f, q);
-    const float sc = SKF == 1 ? cubic_dwdr_sel(f, q, inv_dist, M.inv_h)
-                              : kernel_dwdr_scalef(skf, f, q, inv_dist, M.inv_h);
-    float vcc = (vdi.x - vdj.x) * dx + (vdi.y - vdj.y) * dy;
-    if (DIM == 3) vcc += (vdi.z - vdj.z) * dz;
+__device__ __forceinline__ float density_term(const DevParams& P, float3 d, float d2, float4 vdi, float4 vdj) {
+    const MixedF& M = P.mf;
+    const ReuseF& U = P.rf;
+    const float rs = inv_distance(d2);
+    const float q = d2 * rs * M.inv_h;
+    const int skf = SKF ? SKF : P.density_skf;
+    if (!CONT) return SKF == 1 ? cubic_w(q) : kernel_wf(skf, M.kf[skf], q);
+    const float sc = SKF == 1 ? cubic_s(U, q, rs) : kernel_dwdr_scalef(skf, M.kf[skf], q, rs, M.inv_h);
+    float vcc = (vdi.x - vdj.x) * d.x + (vdi.y - vdj.y) * d.y;
+    if (DIM == 3) vcc += (vdi.z - vdj.z) * d.z;
     float term = vcc * sc;
-    if (delta) {
+    if (P.density_treatment == 2) {
         const float rho_factor = __fdividef(vd4_drho<DIM>(vdi, vdj), M.rho0 + vdi.w);
-        term += 2.0f * M.dhc * (rho_factor * -sc);
+        term -= d2 > 0.0f ? 2.0f * M.dhc * (rho_factor * sc) : 0.0f;
     }
     return term;
 }
+template <int SKF, bool CONT>
+__device__ __forceinline__ F2 term_factor(const ReuseF& U) {
+    return SKF != 1 ? U.m : (CONT ? U.a : U.w);
+}
 
 // density_sum (Density.h:25-61) + EOS, or density_con (Density.h:63-114), over
-// the candidate list: the entries within the cutoff are this step's
-// neighbours, written to nlist for the force pass. A particle whose list
-// overflowed searches the stencil cells (the grid is rebuilt every step while
-// one does) and writes its neighbours too.
+// the candidate list; the candidates within the cutoff are this step's
+// neighbours, written to nlist for the force pass. A particle that is searched
+// instead (the grid is rebuilt every step while one is) writes its neighbours too.
 template <int DIM, int SKF, bool CONT, int L>
 __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams P, State S, Sorted G,
                                                                      StepScalars* __restrict__ scal,
                                                                      uint32_t* __restrict__ flags) {
     constexpr int CAP = Vl<DIM>::cap;
-    constexpr uint32_t IDX = Vl<DIM>::index;
     // the force gather may launch now: it waits for this grid at its start (griddepcontrol.wait)
     asm volatile("griddepcontrol.launch_dependents;");
     if (L > 1 && blockIdx.x * 32u >= P.n) {  // the extra block
@@ -265,90 +305,102 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
     uint32_t cnt = 0, word = 0;
     Kahan acc{0.0f, 0.0f};
     if (active) {
-        const MixedF& M = P.mf;
-        const float4 pj = G.P4[k];
-        const int32_t tj = __float_as_int(pj.w);
-        const int skf = SKF ? SKF : P.density_skf;
-        const float f = M.kf[skf];
-        const bool delta = CONT && P.density_treatment == 2;
+        const float u = P.rf.u, lo = P.mf.cut2_lo, hi = P.mf.cut2_hi;
+        const Pos pj = G.pos[k];
         const float4 vdj = CONT ? G.VD4[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        uint32_t* const nslab = G.nlist + (size_t)k * 4;  // neighbour e at nslab[slab_at(e)]
-        if (tj != P.type_non_existent) {
-            const uint32_t vc = G.vcount[k];
-            if (vc != kListOver) {
-                const uint4* slab = reinterpret_cast<const uint4*>(G.vlist) + k;  // group g at slab[g * n]
-                // shift of offset code (cx, cy, cz) = (cx - 2, cy - 2, cz - 2) cells, relative to this particle
-                const float bx = -2.0f * M.cell - pj.x, by = -2.0f * M.cell - pj.y, bz = -2.0f * M.cell - pj.z;
-                // groups of four entries (one load, the next group's issued before this
-                // one's particles are loaded), then their particles, loaded together;
-                // the body has no branch but the rare guard-band test, and each group's
-                // sum is added with compensation
-                // (list words are read once a step: streaming loads keep L1 for the neighbours' data)
-                uint4 w = 4 * sub < vc ? __ldcs(slab + (size_t)sub * P.n)
-                                       : make_uint4(kVlNone, kVlNone, kVlNone, kVlNone);
-                for (uint32_t e0 = 4 * sub; e0 < vc; e0 += kVlBatch * L) {
-                    const uint4 wn = e0 + kVlBatch * L < vc ? __ldcs(slab + (size_t)((e0 >> 2) + L) * P.n) : w;
+        const uint32_t vc = pj.absent() ? 0u : G.vcount[k];
+        if (vc != kListOver) {
+            const uint4* const slab = reinterpret_cast<const uint4*>(G.vlist) + k;  // group g at slab[g * n]
+            const uint32_t groups = (vc + 3u) >> 2;
+            // groups of four entries (one load, the next group's issued before this
+            // one's particles are loaded), then their particles, loaded together; the
+            // body has no branch but the rare guard-band test, and each group's sum is
+            // added with compensation (list words are read once a step: streaming
+            // loads keep L1 for the neighbours' data)
+            // neighbours wait in a ring of eight words in shared memory until there are
+            // four to store: no branch per candidate
+            uint4* const out = reinterpret_cast<uint4*>(G.nlist) + (size_t)sub * P.n + k;  // this warp's group j at out[L j n]
+            extern __shared__ uint32_t list_ring[];
+            uint32_t* const ring = list_ring + threadIdx.x;  // word e & 7 at ring[(e & 7) blockDim.x]
+            uint32_t stored = 0;
+            auto store4 = [&]() {
+                const uint32_t* const q = ring + (stored & 4u) * blockDim.x;
+                out[(size_t)(L * (stored >> 2)) * P.n] = make_uint4(q[0], q[blockDim.x], q[2 * blockDim.x], q[3 * blockDim.x]);
+                stored += 4;
+            };
+            uint4 w = make_uint4(P.n, P.n, P.n, P.n);
+            if (sub < groups) w = __ldcs(slab + (size_t)sub * P.n);
+            for (uint32_t g = sub; g < groups; g += L) {
+                    const uint4 wn = g + L < groups ? __ldcs(slab + (size_t)(g + L) * P.n) : w;
                     const uint32_t en[kVlBatch] = {w.x, w.y, w.z, w.w};
-                    float4 pb[kVlBatch];
+                    Pos pb[kVlBatch];
 #pragma unroll
-                    for (int j = 0; j < kVlBatch; j++)
-                        pb[j] = en[j] != kVlNone ? G.P4[en[j] & IDX] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    for (int j = 0; j < kVlBatch; j++) pb[j] = G.pos[en[j]];
+                    float3 d[kVlBatch];
+                    float d2[kVlBatch];
+                    bool in[kVlBatch], band = false;
+#pragma unroll
+                    for (int j = 0; j < kVlBatch; j++) {
+                        d[j] = separation<DIM>(pb[j], pj, u);
+                        d2[j] = distance2<DIM>(d[j], pb[j].code);
+                        in[j] = d2[j] < lo;
+                        band = band || (!in[j] && d2[j] < hi);
+                    }
+                    if (band) {
+#pragma unroll 1
+                        for (int j = 0; j < kVlBatch; j++) {
+                            const float x = j == 0 ? d2[0] : (j == 1 ? d2[1] : (j == 2 ? d2[2] : d2[3]));
+                            const uint32_t e = j == 0 ? en[0] : (j == 1 ? en[1] : (j == 2 ? en[2] : en[3]));
+                            if (!(x < lo) && x < hi && exact_pair<DIM>(P, S, G.id[e], G.id[k])) {
+                                if (j == 0) in[0] = true;
+                                if (j == 1) in[1] = true;
+                                if (j == 2) in[2] = true;
+                                if (j == 3) in[3] = true;
+                            }
+                        }
+                    }
                     float part = 0.0f;
 #pragma unroll
                     for (int j = 0; j < kVlBatch; j++) {
-                        uint32_t cx, cy, cz;
-                        vl_offset<DIM>(en[j], cx, cy, cz);
-                        const float dx = pb[j].x + fmaf((float)cx, M.cell, bx);
-                        const float dy = pb[j].y + fmaf((float)cy, M.cell, by);
-                        const float dz = DIM == 3 ? pb[j].z + fmaf((float)cz, M.cell, bz) : 0.0f;
-                        const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-                        bool in = en[j] != kVlNone && __float_as_int(pb[j].w) != P.type_non_existent &&
-                                  d2 < M.cut2_hi;
-                        if (in && !(d2 < M.cut2_lo)) in = within_cutoff<DIM>(P, S, G, en[j] & IDX, k, d2);
-                        const float4 vdi = CONT && in ? G.VD4[en[j] & IDX] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        const float t = density_term<DIM, SKF, CONT>(M, skf, f, dx, dy, dz, d2, vdi, vdj, delta);
-                        part += in ? t : 0.0f;
-                        if (in) nslab[slab_at<L>(P.n, sub, cnt)] = en[j];
-                        cnt += in;
+                        const float4 vdi = CONT && in[j] ? G.VD4[en[j]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        const float t = density_term<DIM, SKF, CONT>(P, d[j], d2[j], vdi, vdj);
+                        part += in[j] ? t : 0.0f;
+                        if (in[j]) ring[(cnt & 7u) * blockDim.x] = en[j];
+                        cnt += in[j];
                     }
-                    acc.add(M.mass * part);
+                    if (cnt - stored >= 4) store4();
+                    acc.add(part);
                     w = wn;
-                }
-                word = cnt;
-            } else if (sub == 0) {
-                constexpr int NC = DIM == 3 ? 27 : 9;
-                const Stencil<DIM> st(P, G.key[k]);
-#pragma unroll 1
-                for (int c = 0; c < NC; c++) {
-                    uint32_t cell;
-                    int sx, sy, sz;
-                    if (!st.cell(c, cell, sx, sy, sz)) continue;
-                    const uint32_t s = G.cell_start[cell];
-                    if (s == kEmpty) continue;
-                    const uint32_t e = G.cell_end[cell];
-                    const float shx = (float)sx * M.cell - pj.x;
-                    const float shy = (float)sy * M.cell - pj.y;
-                    const float shz = DIM == 3 ? (float)sz * M.cell - pj.z : 0.0f;
-                    float part = 0.0f;
-                    for (uint32_t i = s; i < e; i++) {
-                        if (i == k) continue;
-                        const float4 pi = G.P4[i];
-                        if (__float_as_int(pi.w) == P.type_non_existent) continue;
-                        const float dx = pi.x + shx, dy = pi.y + shy, dz = DIM == 3 ? pi.z + shz : 0.0f;
-                        const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-                        if (!within_cutoff<DIM>(P, S, G, i, k, d2)) continue;
-                        // this step's neighbour list too (the grid is this step's: the stencil
-                        // offsets are within one cell)
-                        if (cnt < (uint32_t)CAP)
-                            nslab[slab_at<1>(P.n, 0, cnt)] = i | vl_code<DIM>(sx, sy, sz);
-                        cnt++;
-                        const float4 vdi = CONT ? G.VD4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        part += density_term<DIM, SKF, CONT>(M, skf, f, dx, dy, dz, d2, vdi, vdj, delta);
-                    }
-                    acc.add(M.mass * part);
-                }
-                word = packed_counts<L>(min(cnt, (uint32_t)CAP));
             }
+            if (cnt > stored) store4();  // (the words past cnt are not read)
+            word = cnt;
+        } else if (sub == 0) {
+            // the stencil search (the grid is this step's)
+            uint32_t* const list = G.nlist + (size_t)k * 4;
+            constexpr int NC = DIM == 3 ? 27 : 9;
+            const Stencil<DIM> st(P, G.key[k]);
+#pragma unroll 1
+            for (int c = 0; c < NC; c++) {
+                uint32_t cell;
+                int sx, sy, sz;
+                if (!st.cell(c, cell, sx, sy, sz)) continue;
+                const uint32_t s = G.cell_start[cell];
+                if (s == kEmpty) continue;
+                const uint32_t e = G.cell_end[cell];
+                float part = 0.0f;
+                for (uint32_t i = s; i < e; i++) {
+                    if (i == k) continue;
+                    const Pos pi = G.pos[i];
+                    if (!searched_pair<DIM>(P, S, G, i, k, pi, pj)) continue;
+                    if (cnt < (uint32_t)CAP) list[(size_t)(cnt >> 2) * 4 * P.n + (cnt & 3u)] = i;
+                    cnt++;
+                    const float4 vdi = CONT ? G.VD4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const float3 d = separation<DIM>(pi, pj, u);
+                    part += density_term<DIM, SKF, CONT>(P, d, distance2<DIM>(d, 0.0f), vdi, vdj);
+                }
+                acc.add(part);
+            }
+            word = packed_counts<L>(min(cnt, (uint32_t)CAP));
         }
     }
     if (L > 1) {
@@ -359,27 +411,24 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
         pn[sub][lane] = cnt;
         __syncthreads();
         if (sub != 0) return;
-        if (active) {
-            // (an over-full list was searched by this warp alone, its counts packed)
-            const bool listed = G.vcount[k] != kListOver;
 #pragma unroll
-            for (int u = 1; u < L; u++) {
-                acc.add(ps[u][lane]);
-                acc.c += pc[u][lane];
-                cnt += pn[u][lane];
-                if (listed) word |= pn[u][lane] << ((uint32_t)u * kCountBits<L>);
-            }
+        for (int u = 1; u < L; u++) {  // (a searched particle's other warps counted nothing)
+            acc.add(ps[u][lane]);
+            acc.c += pc[u][lane];
+            cnt += pn[u][lane];
+            word += pn[u][lane] << ((uint32_t)u * kCountBits<L>);
         }
     }
     if (active) {
         const MixedF& M = P.mf;
         const uint32_t id = G.id[k];
-        G.ncount[k] = L == 1 ? min(cnt, (uint32_t)CAP) : word;
+        G.ncount[k] = word;
         if (cnt > P.max_nb - 1) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
         if (!CONT) {
             // rho - rho0 = sum - (rho0 - m W(0)): the two are within a factor of two,
             // so the float difference is exact; the Kahan and rounding residuals follow
-            const float d = ((acc.s - M.rho0_minus_w0_hi) - acc.c) - M.rho0_minus_w0_lo;
+            const F2 sum = scaled(acc, term_factor<SKF, CONT>(P.rf));
+            const float d = ((sum.hi - M.rho0_minus_w0_hi) + sum.lo) - M.rho0_minus_w0_lo;
             const float rho = M.rho0 + d;
             const float pr = eos_pf(M, d);
             const float2 prr = make_float2(pr, pr * __frcp_rn(rho * rho));
@@ -398,199 +447,56 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
             if (DIM == 2) G.V4[k].z = P.intf_form == 1 ? prr.x : prr.y;
             G.PR[k] = prr;
             S.p[id] = pr;
-            S.drho[id] = acc.value();
+            S.drho[id] = value(scaled(acc, term_factor<SKF, CONT>(P.rf)));
         }
     }
     warp_sum_add(&scal->pairs, cnt);
 }
 
-#if RRSPH_DENSITY_CELL_TILES
-// The cell-tile variant of the 2D summation density pass (compile-time switch
-// RRSPH_DENSITY_CELL_TILES=1; the candidate-list pass above is the default).
-// Each warp (32 consecutive particles in the build's cell order, a 2x2 block
-// of cells or two) stages the particles of its cells' neighbourhood, the
-// bounding box of its build cells widened by two cells each way, from the
-// cell table into shared memory; each lane then tests every particle of the
-// build cells in its particle's window (the 3x3 to 4x4 cells k_vl_build
-// searched) against the reference's cutoff, with the same float test, guard
-// band and double re-test, and writes this step's neighbour list for the
-// force pass as the list variant does. A warp whose box or particle count
-// exceeds the stage reads the cell table and the particles from global memory
-// instead. The cell table read here is the one of the last list build: with
-// this variant the key pass leaves it in place (DevParams::keep_cells) and
-// each rebuild clears it wholesale.
-constexpr int kTileWarps = 4;         // warps per block
-constexpr int kTileBoxCells = 64;     // cells of a staged box
-constexpr int kTileCap = 384;         // particles of a staged box
-struct TileStage {
-    float4 p[kTileCap];
-    uint32_t start[kTileBoxCells];    // first stage index of a box cell
-    uint32_t slot0[kTileBoxCells];    // its first sorted index
-    uint32_t count[kTileBoxCells];
-};
-
-template <bool STAGED>
-__device__ __forceinline__ void tile_density_cells(const DevParams& P, const State& S, const Sorted& G,
-                                                   const TileStage& T, uint32_t k, uint32_t cx, uint32_t cy,
-                                                   uint32_t bx0, uint32_t by0, uint32_t bw, float4 pj,
-                                                   Kahan& acc, uint32_t& cnt, uint4& nb, uint4* nout) {
+// One neighbour's coefficient of the separation in the acceleration, for the
+// common method set (pressure form 2, Monaghan viscosity, cubic kernel, no
+// artificial pressure or XSPH), over the factor ReuseF::a:
+// s (p_i/rho_i^2 + p_j/rho_j^2 + Pi), one quotient for the two of the viscosity.
+// lj: a boundary neighbour of a fluid particle under Lennard-Jones. MU: keep the
+// largest |mu|.
+template <int DIM, bool MU>
+__device__ __forceinline__ float pair_coef(const DevParams& P, float3 d, float d2, const float4& vj, const float4& vi,
+                                           float pf, bool lj, float& arvmu) {
     const MixedF& M = P.mf;
-    const float f = M.kf[1];
-    const float2 bo = S.boff[G.id[k]];
-    int x0, x1, y0, y1;
-    vl_window<2>(bo.x, cx, M.cell, P.vl_skin_edge, x0, x1);
-    vl_window<2>(bo.y, cy, M.cell, P.vl_skin_edge, y0, y1);
-#pragma unroll 1
-    for (int dx = x0; dx <= x1; dx++) {
-#pragma unroll 1
-        for (int dy = y0; dy <= y1; dy++) {
-            uint32_t s, c, base;
-            if (STAGED) {
-                const uint32_t b = (cx + dx - bx0) + (cy + dy - by0) * bw;
-                c = T.count[b];
-                s = T.slot0[b];
-                base = T.start[b];
-            } else {
-                const uint32_t cell = split2_32(cx + dx) | (split2_32(cy + dy) << 1);
-                if (cell >= P.max_cells) continue;
-                s = G.cell_start[cell];
-                if (s == kEmpty) continue;
-                c = G.cell_end[cell] - s;
-                base = s;
-            }
-            const float shx = (float)dx * M.cell - pj.x;
-            const float shy = (float)dy * M.cell - pj.y;
-            const uint32_t code = vl_code<2>(dx, dy, 0);
-            float part = 0.0f;
-            for (uint32_t t = 0; t < c; t++) {
-                const uint32_t i = s + t;
-                const float4 pi = STAGED ? T.p[base + t] : G.P4[base + t];
-                const float ddx = pi.x + shx, ddy = pi.y + shy;
-                const float d2 = ddx * ddx + ddy * ddy;
-                bool in = i != k && __float_as_int(pi.w) != P.type_non_existent && d2 < M.cut2_hi;
-                if (in && !(d2 < M.cut2_lo)) in = within_cutoff<2>(P, S, G, i, k, d2);
-                if (in) {
-                    const float inv_dist = rsqrtf(d2);
-                    part += cubic_wf_sel(f, d2 * inv_dist * M.inv_h);
-                    const uint32_t slot = cnt & 3u, en = i | code;
-                    nb.x = slot == 0 ? en : nb.x;
-                    nb.y = slot == 1 ? en : nb.y;
-                    nb.z = slot == 2 ? en : nb.z;
-                    nb.w = slot == 3 ? en : nb.w;
-                    if (slot == 3 && cnt < (uint32_t)kVerletCap2) nout[(size_t)(cnt >> 2) * P.n] = nb;
-                    cnt++;
-                }
-            }
-            acc.add(M.mass * part);
-        }
+    const ReuseF& U = P.rf;
+    const float rs = inv_distance(d2);
+    const float s = cubic_s(U, d2 * rs * M.inv_h, rs);
+    float vr = (vi.x - vj.x) * d.x + (vi.y - vj.y) * d.y;
+    if (DIM == 3) vr += (vi.z - vj.z) * d.z;
+    // approaching pairs only (vr < 0), evaluated by every lane and clamped
+    const float rhos = vi.w + vj.w;
+    const float w = fminf(vr, 0.0f) * rcp_approx((d2 + M.etq_h2) * rhos);
+    if (MU || U.bulk != 0.0f) {
+        const float mu = M.h * w * rhos;
+        if (MU) arvmu = fmaxf(arvmu, -mu);
+        pf = fmaf(U.bulk * mu, w, pf);
     }
+    float m = s * fmaf(U.visc, w, pf);
+    if (lj && d2 < U.lj_r2 && d2 > 0.0f) {
+        const float rn = M.lj_rr0 * rs;
+        const float rn2 = rn * rn, rn4 = rn2 * rn2, rn8 = rn4 * rn4;
+        m -= U.lj_D * (rn8 * rn4 - rn4) * (rs * rs);
+    }
+    return m;
 }
 
-__global__ void __launch_bounds__(kTileWarps * 32) k_density_tiles(DevParams P, State S, Sorted G,
-                                                                   StepScalars* __restrict__ scal,
-                                                                   uint32_t* __restrict__ flags) {
-    asm volatile("griddepcontrol.launch_dependents;");
-    __shared__ TileStage stage[kTileWarps];
-    TileStage& T = stage[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = k < P.n;
-    // the warp's build cells and their bounding box, two cells wider each way
-    uint32_t cx = 0, cy = 0;
-    if (active) {
-        const uint32_t key = G.key[k];
-        cx = second_bits(key);
-        cy = second_bits(key >> 1);
-    }
-    const uint32_t xmin = __reduce_min_sync(0xFFFFFFFFu, active ? cx : 0xFFFFFFFFu);
-    const uint32_t xmax = __reduce_max_sync(0xFFFFFFFFu, active ? cx : 0u);
-    const uint32_t ymin = __reduce_min_sync(0xFFFFFFFFu, active ? cy : 0xFFFFFFFFu);
-    const uint32_t ymax = __reduce_max_sync(0xFFFFFFFFu, active ? cy : 0u);
-    if (xmin == 0xFFFFFFFFu) return;  // no particle in this warp
-    const uint32_t bx0 = xmin >= 2 ? xmin - 2 : 0, by0 = ymin >= 2 ? ymin - 2 : 0;
-    const uint32_t bx1 = xmax + 2 <= kMaxCellCoord2 ? xmax + 2 : kMaxCellCoord2;
-    const uint32_t by1 = ymax + 2 <= kMaxCellCoord2 ? ymax + 2 : kMaxCellCoord2;
-    const uint32_t bw = bx1 - bx0 + 1, nbox = bw * (by1 - by0 + 1);
-    bool staged = nbox <= (uint32_t)kTileBoxCells;
-    if (staged) {
-        // per box cell: its range in the sorted order, and an exclusive prefix
-        // of the counts over the box (two rounds of 32 cells)
-        uint32_t total = 0;
-        for (uint32_t b0 = 0; b0 < nbox; b0 += 32) {
-            const uint32_t b = b0 + lane;
-            uint32_t s = 0, c = 0;
-            if (b < nbox) {
-                const uint32_t cell = split2_32(bx0 + b % bw) | (split2_32(by0 + b / bw) << 1);
-                if (cell < P.max_cells) {
-                    s = G.cell_start[cell];
-                    if (s != kEmpty) c = G.cell_end[cell] - s;
-                    else s = 0;
-                }
-            }
-            uint32_t incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= (uint32_t)o) incl += v;
-            }
-            if (b < nbox) {
-                T.start[b] = total + incl - c;
-                T.slot0[b] = s;
-                T.count[b] = c;
-            }
-            total += __shfl_sync(0xFFFFFFFFu, incl, 31);
-        }
-        staged = total <= (uint32_t)kTileCap;
-        __syncwarp();
-        if (staged) {
-            for (uint32_t b = lane; b < nbox; b += 32) {
-                const uint32_t s = T.slot0[b], c = T.count[b], d = T.start[b];
-                for (uint32_t t = 0; t < c; t++) T.p[d + t] = G.P4[s + t];
-            }
-        }
-        __syncwarp();
-    }
-    uint32_t cnt = 0;
-    if (active) {
-        const MixedF& M = P.mf;
-        const uint32_t id = G.id[k];
-        const float4 pj = G.P4[k];
-        Kahan acc{0.0f, 0.0f};
-        uint4* const nout = reinterpret_cast<uint4*>(G.nlist) + k;  // group g at nout[g * n]
-        uint4 nb = make_uint4(kVlNone, kVlNone, kVlNone, kVlNone);
-        if (__float_as_int(pj.w) != P.type_non_existent) {
-            if (staged) tile_density_cells<true>(P, S, G, T, k, cx, cy, bx0, by0, bw, pj, acc, cnt, nb, nout);
-            else tile_density_cells<false>(P, S, G, T, k, cx, cy, bx0, by0, bw, pj, acc, cnt, nb, nout);
-            if ((cnt & 3u) && cnt < (uint32_t)kVerletCap2) nout[(size_t)(cnt >> 2) * P.n] = nb;
-        }
-        G.ncount[k] = cnt < (uint32_t)kVerletCap2 ? cnt : (uint32_t)kVerletCap2;
-        if (cnt > P.max_nb - 1) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
-        const float d = ((acc.s - M.rho0_minus_w0_hi) - acc.c) - M.rho0_minus_w0_lo;
-        const float rho = M.rho0 + d;
-        const float pr = eos_pf(M, d);
-        const float2 prr = make_float2(pr, pr * __frcp_rn(rho * rho));
-        reinterpret_cast<float2*>(G.V4 + k)[1] = make_float2(P.intf_form == 1 ? prr.x : prr.y, rho);
-        G.PR[k] = prr;
-        S.rho[id] = P.rho0 + f2d(d);
-        S.p[id] = f2d(pr);
-    }
-    warp_sum_add(&scal->pairs, cnt);
-}
-#endif
-
-// update_acceleration over this step's neighbours: the list the density pass
-// wrote (or the stencil search for an overflowed list). In 2D a neighbour's
-// pressure comes with its velocity and density (V4.z); in 3D from PR. STD: the
-// common method set of ForceAcc::pair_std (2D) / pair_std3 (3D), fixed at
-// compile time. At most
-// 64 registers (4 blocks of 256 threads per SM): the gather hides its L1/L2
-// latency with warps.
+// update_acceleration over this step's neighbours: the list the density pass wrote
+// (or the stencil search, where a searched particle may have
+// more neighbours than a list holds: WV == 0). In 2D a neighbour's pressure comes
+// with its velocity and density (V4.z); in 3D from PR. STD: the common method set
+// (pair_coef), fixed at compile time. At most 64 registers (4 blocks of 256
+// threads per SM): the gather hides its L1/L2 latency with warps.
 // WV != 0: the whole step follows in the same thread (whole_particle with
 // variant WV, thread 0 advancing the scalars into next): it reads nothing that
-// another thread's whole step writes, because this step's copies (P4, V4, VD4)
-// are not the ones the key pass writes (P4n, V4n, VD4n), and the list of every
-// particle is complete (the density pass wrote the neighbours of overflowed
-// lists too, which needs at most Vl<DIM>::cap neighbours per particle).
+// another thread's whole step writes, because this step's copies (pos, V4, VD4)
+// are not the ones the key pass writes (posn, V4n, VD4n), and the neighbours of
+// every particle are listed (the density pass wrote those of searched particles
+// too, which needs at most Vl<DIM>::cap neighbours per particle).
 __device__ __forceinline__ void fetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 // The rows whole_particle and its key pass read of particle id.
 template <int DIM>
@@ -602,13 +508,12 @@ __device__ __forceinline__ void fetch_whole(const State& S, uint32_t id) {
     if (DIM == 3) {
         fetch_l1(S.rz + id);
         fetch_l1(S.vz + id);
-        fetch_l1(S.boff4 + id);
+        fetch_l1(S.bfix4 + id);
     } else {
-        fetch_l1(S.boff + id);
+        fetch_l1(S.bfix2 + id);
     }
     fetch_l1(S.itype + id);
     fetch_l1(S.key_of + id);
-    fetch_l1(S.bcxy + id);
     fetch_l1(S.slot + id);
 }
 template <int DIM, int SKF, bool STD, int WV, int L>
@@ -616,7 +521,8 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
                                                                     StepScalars* __restrict__ scal,
                                                                     StepScalars* __restrict__ next,
                                                                     uint32_t* __restrict__ flags) {
-    constexpr uint32_t IDX = Vl<DIM>::index;
+    constexpr int B = kVlForceBatch<DIM, STD>;
+    constexpr bool MU = WV == 0 || (WV & kVarRare) != 0;
     const uint32_t lane = threadIdx.x & 31u, sub = L > 1 ? threadIdx.x >> 5 : 0u;
     uint32_t k = L > 1 ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = k < P.n;
@@ -629,14 +535,14 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
     if (WV != 0 && L > 1 && sub == 0) fetch_whole<DIM>(S, G.id[k]);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (L > 1 || active) {
-        const MixedF& M = P.mf;
+        const ReuseF& U = P.rf;
         const uint32_t id = G.id[k];
-        const float4 pj4 = G.P4[k];
-        const int32_t tj = __float_as_int(pj4.w);
+        const Pos pj = G.pos[k];
+        const bool fluid = pj.fluid();
         ForceAcc<DIM, SKF> F{P, G, G.V4[k], G.PR[k], 0.0f, false, false, false, false, false, 0, 0,
                              0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         F.rhoj = F.vj.w;
-        F.ext = P.repulsive && tj > 0;
+        F.ext = P.repulsive && fluid;
         F.intf = true;
         F.visc = P.art_visc;
         F.avel = P.avg_vel;
@@ -645,68 +551,65 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
         F.av_skf = SKF ? SKF : P.av_skf;
         Kahan ax{0, 0}, ay{0, 0}, az{0, 0};
         Kahan avx{0, 0}, avy{0, 0}, avz{0, 0};
-        if (tj != P.type_non_existent) {
-            const uint32_t vc = G.vcount[k];
-            if (WV != 0 || vc != kListOver) {
-                // this step's neighbours, four list words per load (the lanes of a
-                // warp load neighbouring uint4s), their data two at a time
+        // the general pair
+        auto general = [&](const float4& vi, float2 pri, const Pos& pi, float3 d, float d2) {
+            F.cax = F.cay = F.caz = F.cvx = F.cvy = F.cvz = 0.0f;
+            F.pair_with(vi, pri, d.x, d.y, d.z, d2, pi.boundary() ? -1 : (pi.fluid() ? 1 : 0));
+            ax.add(F.cax);
+            ay.add(F.cay);
+            if (DIM == 3) az.add(F.caz);
+            if (F.avel) {
+                avx.add(F.cvx);
+                avy.add(F.cvy);
+                if (DIM == 3) avz.add(F.cvz);
+            }
+        };
+        auto one = [&](const float4& vi, float2 pr3, const Pos& pi) {
+            const float3 d = separation<DIM>(pi, pj, U.u);
+            const float d2 = distance2<DIM>(d, 0.0f);
+            if (STD) {
+                const float m = pair_coef<DIM, MU>(P, d, d2, F.vj, vi, (DIM == 3 ? pr3.y : vi.z) + F.prj.y,
+                                                   F.ext && pi.boundary(), F.arvmu);
+                // each pair's terms are added with compensation
+                ax.add(d.x * m);
+                ay.add(d.y * m);
+                if (DIM == 3) az.add(d.z * m);
+            } else if (DIM == 3) {
+                general(vi, pr3, pi, d, d2);
+            } else {  // p (form 1) or p/rho^2, as the density pass wrote it
+                const float z = vi.z;
+                general(vi, F.form1 ? make_float2(z, z * __frcp_rn(vi.w * vi.w)) : make_float2(z, z), pi, d, d2);
+            }
+        };
+        if (!pj.absent()) {
+            if (WV != 0 || G.vcount[k] != kListOver) {
+                // four list words per load (the lanes of a warp load neighbouring uint4s), the
+                // data of B of them together
                 const uint32_t nc = sub_count<L>(G.ncount[k], sub);
-                const uint4* nslab = reinterpret_cast<const uint4*>(G.nlist) + k;  // group g at nslab[g * n]
-                const float bx = -2.0f * M.cell - pj4.x, by = -2.0f * M.cell - pj4.y, bz = -2.0f * M.cell - pj4.z;
+                const uint4* const slab = reinterpret_cast<const uint4*>(G.nlist) + (size_t)sub * P.n + k;
+                // (streaming, as in the density pass; the next words ahead of this group's data)
+                uint4 ahead = make_uint4(0u, 0u, 0u, 0u);
+                if (nc) ahead = __ldcs(slab);
                 for (uint32_t e0 = 0; e0 < nc; e0 += 4) {
-                    // streaming, as in the density pass
-                    const uint4 w = __ldcs(nslab + (size_t)(L == 1 ? e0 >> 2 : sub + L * (e0 >> 2)) * P.n);
-                    const uint32_t eg[4] = {w.x, w.y, w.z, w.w};
+                    const uint4 w = ahead;
+                    if (e0 + 4 < nc) ahead = __ldcs(slab + (size_t)(L * ((e0 >> 2) + 1)) * P.n);
+                    const uint32_t en[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                    for (int h = 0; h < 4; h += kVlForceBatch<DIM, STD>) {
-                        uint32_t en[kVlForceBatch<DIM, STD>];
-                        float4 pb[kVlForceBatch<DIM, STD>], vb[kVlForceBatch<DIM, STD>];
-                        float2 rb[kVlForceBatch<DIM, STD>];
+                    for (int h = 0; h < 4; h += B) {
+                        Pos pb[B];
+                        float4 vb[B];
+                        float2 rb[B];
 #pragma unroll
-                        for (int j = 0; j < kVlForceBatch<DIM, STD>; j++) en[j] = e0 + h + j < nc ? eg[h + j] : kVlNone;
-#pragma unroll
-                        for (int j = 0; j < kVlForceBatch<DIM, STD>; j++) {
-                            if (en[j] == kVlNone) continue;
-                            const uint32_t i = en[j] & IDX;
-                            pb[j] = G.P4[i];
-                            vb[j] = G.V4[i];
-                            if (DIM == 3) rb[j] = G.PR[i];
+                        for (int j = 0; j < B; j++) {
+                            if (e0 + h + j >= nc) continue;
+                            pb[j] = G.pos[en[h + j]];
+                            vb[j] = G.V4[en[h + j]];
+                            if (DIM == 3) rb[j] = G.PR[en[h + j]];
                         }
-                        // each pair's terms are added with compensation (no per-cell
-                        // partial sums, whose flushes would split the warp)
 #pragma unroll
-                        for (int j = 0; j < kVlForceBatch<DIM, STD>; j++) {
-                            if (en[j] == kVlNone) continue;
-                            uint32_t cx, cy, cz;
-                            vl_offset<DIM>(en[j], cx, cy, cz);
-                            const float dx = pb[j].x + fmaf((float)cx, M.cell, bx);
-                            const float dy = pb[j].y + fmaf((float)cy, M.cell, by);
-                            const float dz = DIM == 3 ? pb[j].z + fmaf((float)cz, M.cell, bz) : 0.0f;
-                            const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-                            F.cax = F.cay = F.caz = F.cvx = F.cvy = F.cvz = 0.0f;
-                            if (DIM == 2 && STD) {
-                                F.pair_std(vb[j], dx, dy, d2, __float_as_int(pb[j].w));
-                            } else if (DIM == 3 && STD) {
-                                F.pair_std3(vb[j], rb[j], dx, dy, dz, d2, __float_as_int(pb[j].w));
-                            } else {
-                                float2 pri;
-                                if (DIM == 3) {
-                                    pri = rb[j];
-                                } else {  // p (form 1) or p/rho^2, as the density pass wrote it
-                                    const float z = vb[j].z;
-                                    pri = F.form1 ? make_float2(z, z * __frcp_rn(vb[j].w * vb[j].w))
-                                                  : make_float2(z, z);
-                                }
-                                F.pair_with(vb[j], pri, dx, dy, dz, d2, __float_as_int(pb[j].w));
-                            }
-                            ax.add(F.cax);
-                            ay.add(F.cay);
-                            if (DIM == 3) az.add(F.caz);
-                            if (!STD && F.avel) {
-                                avx.add(F.cvx);
-                                avy.add(F.cvy);
-                                if (DIM == 3) avz.add(F.cvz);
-                            }
+                        for (int j = 0; j < B; j++) {
+                            if (e0 + h + j >= nc) continue;
+                            one(vb[j], DIM == 3 ? rb[j] : make_float2(0.0f, 0.0f), pb[j]);
                         }
                     }
                 }
@@ -721,27 +624,12 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
                     const uint32_t s = G.cell_start[cell];
                     if (s == kEmpty) continue;
                     const uint32_t e = G.cell_end[cell];
-                    const float shx = (float)sx * M.cell - pj4.x;
-                    const float shy = (float)sy * M.cell - pj4.y;
-                    const float shz = DIM == 3 ? (float)sz * M.cell - pj4.z : 0.0f;
-                    F.cax = F.cay = F.caz = F.cvx = F.cvy = F.cvz = 0.0f;
+#pragma unroll 1
                     for (uint32_t i = s; i < e; i++) {
                         if (i == k) continue;
-                        const float4 pi4 = G.P4[i];
-                        const int32_t ti = __float_as_int(pi4.w);
-                        if (ti == P.type_non_existent) continue;
-                        const float dx = pi4.x + shx, dy = pi4.y + shy, dz = DIM == 3 ? pi4.z + shz : 0.0f;
-                        const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-                        if (!within_cutoff<DIM>(P, S, G, i, k, d2)) continue;
-                        F.pair(i, dx, dy, dz, d2, ti);
-                    }
-                    ax.add(F.cax);
-                    ay.add(F.cay);
-                    if (DIM == 3) az.add(F.caz);
-                    if (F.avel) {
-                        avx.add(F.cvx);
-                        avy.add(F.cvy);
-                        if (DIM == 3) avz.add(F.cvz);
+                        const Pos pi = G.pos[i];
+                        if (!searched_pair<DIM>(P, S, G, i, k, pi, pj)) continue;
+                        one(G.V4[i], G.PR[i], pi);
                     }
                 }
             }
@@ -778,8 +666,9 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
             }
         }
         if (L == 1 || active) {
-            const double axd = ax.value(), ayd = ay.value() - P.g;  // gravity along y (ExtForce.h), 2D and 3D
-            const double azd = DIM == 3 ? az.value() : 0.0;
+            const F2 f = STD ? U.a : F2{1.0f, 0.0f};
+            const double axd = value(scaled(ax, f)), ayd = value(scaled(ay, f)) - P.g;  // gravity along y (ExtForce.h), 2D and 3D
+            const double azd = DIM == 3 ? value(scaled(az, f)) : 0.0;
             S.ax[id] = axd;
             S.ay[id] = ayd;
             if (DIM == 3) S.az[id] = azd;
@@ -808,14 +697,16 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
 void launch_verlet_decide(cudaGraphConditionalHandle h, const uint32_t* rebuild, cudaStream_t st) {
     k_vl_decide<<<1, 1, 0, st>>>(h, rebuild);
 }
-void launch_verlet_reset(uint32_t* rebuild, uint32_t* gone, unsigned long long* builds, cudaStream_t st) {
-    k_vl_reset<<<1, 1, 0, st>>>(rebuild, gone, builds);
+void launch_verlet_reset(uint32_t* rebuild, uint32_t* gone, uint32_t* far, unsigned long long* builds,
+                         cudaStream_t st) {
+    k_vl_reset<<<1, 1, 0, st>>>(rebuild, gone, far, builds);
 }
 void launch_verlet_upload_check(uint32_t* rebuild, const uint32_t* gone, cudaStream_t st) {
     k_vl_upload_check<<<1, 1, 0, st>>>(rebuild, gone);
 }
 template <int DIM>
 void launch_verlet_build(const DevParams& P, const State& S, const Sorted& G, cudaStream_t st) {
+    if (P.reuse == kReuseCell) return launch_verlet_build_cell(P, S, G, st);
     constexpr int kBuildThreads = 128;
     k_vl_build<DIM><<<(P.n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, st>>>(P, S, G);
 }
@@ -830,21 +721,15 @@ int verlet_split(int dim, uint32_t n) { return n <= (dim == 3 ? 128000u : 36000u
 template <int DIM>
 void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal, uint32_t* flags,
                            cudaStream_t st, int threads) {
+    if (P.reuse == kReuseCell) return launch_density_cell(P, S, G, scal, flags, st);
     const bool cont = P.density_treatment != 0;
     const unsigned extra = has_pistons(P, S) ? 1 : 0;
-#if RRSPH_DENSITY_CELL_TILES
-    if (DIM == 2 && !cont && P.all_cubic) {
-        constexpr int tt = kTileWarps * 32;
-        k_density_tiles<<<(P.n + tt - 1) / tt, tt, 0, st>>>(P, S, G, scal, flags);
-        return;
-    }
-#endif
 #define RRSPH_DV(SKF, CONT)                                                                                           \
     do {                                                                                                              \
-        if (P.vl_split == 4)                                                                                          \
-            k_density_verlet<DIM, SKF, CONT, 4><<<(P.n + 31) / 32 + extra, 128, 0, st>>>(P, S, G, scal, flags);       \
+        if (DIM == 3 && P.vl_split == 4)                                                                              \
+            k_density_verlet<DIM, SKF, CONT, DIM == 3 ? 4 : 1><<<(P.n + 31) / 32 + extra, 128, 128 * 32, st>>>(P, S, G, scal, flags);       \
         else                                                                                                          \
-            k_density_verlet<DIM, SKF, CONT, 1><<<(P.n + threads - 1) / threads, threads, 0, st>>>(P, S, G, scal, flags); \
+            k_density_verlet<DIM, SKF, CONT, 1><<<(P.n + threads - 1) / threads, threads, threads * 32, st>>>(P, S, G, scal, flags); \
     } while (0)
     if (P.all_cubic) {
         if (cont) RRSPH_DV(1, true);
@@ -855,23 +740,6 @@ void launch_density_verlet(const DevParams& P, const State& S, const Sorted& G, 
     }
 #undef RRSPH_DV
 }
-// A launch that may start while the stream's previous kernel finishes
-// (programmatic dependent launch); the kernel waits for it with
-// griddepcontrol.wait before it reads what that kernel wrote.
-template <typename... Params, typename... Args>
-void launch_after(void (*kernel)(Params...), unsigned blocks, int threads, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int DIM>
 void launch_forces_verlet(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal,
                           StepScalars* scal_next, uint32_t* flags, cudaStream_t st, int threads, int whole) {
@@ -879,12 +747,13 @@ void launch_forces_verlet(const DevParams& P, const State& S, const Sorted& G, S
     const int wv = whole ? (kVarMixed | (P.density_treatment != 0 ? kVarCont : 0) |
                             (P.avg_vel || P.dt_method == 2 ? kVarRare : 0))
                          : 0;
+    if (P.reuse == kReuseCell) return launch_forces_cell(P, S, G, scal, scal_next, flags, st, std_terms, wv);
 // the force gather follows the density gather with a programmatic dependency:
 // its blocks launch as the density gather's last blocks run, then wait for it
 #define RRSPH_FV(SKF, STD, WV)                                                                                       \
     do {                                                                                                             \
-        if (P.vl_split == 4)                                                                                         \
-            launch_after(k_forces_verlet<DIM, SKF, STD, WV, 4>, (P.n + 31) / 32, 128, st, P, S, G, scal, scal_next, flags); \
+        if (DIM == 3 && P.vl_split == 4)                                                                             \
+            launch_after(k_forces_verlet<DIM, SKF, STD, WV, DIM == 3 ? 4 : 1>, (P.n + 31) / 32, 128, st, P, S, G, scal, scal_next, flags); \
         else                                                                                                         \
             launch_after(k_forces_verlet<DIM, SKF, STD, WV, 1>, (P.n + threads - 1) / threads, threads, st, P, S, G, \
                          scal, scal_next, flags);                                                                    \
@@ -908,35 +777,28 @@ void launch_forces_verlet(const DevParams& P, const State& S, const Sorted& G, S
 
 namespace {
 
-// sub_count with the split as a value.
-__device__ __forceinline__ uint32_t split_count(uint32_t word, uint32_t sub, uint32_t split) {
-    const uint32_t bits = 32u / split;
-    return split == 1 ? word : (word >> (sub * bits)) & ((1u << bits) - 1u);
-}
-
-// The neighbour list the last density pass of the reuse step wrote (nlist,
-// ncount: build slots with cell codes, in list order), as particle ids: row
-// G.id[k] of `list` gets the ids of slot k's entries.
-template <int DIM>
+// The neighbour list the last density pass of the reuse step wrote, as particle
+// ids: row G.id[k] of `list` gets the ids of slot k's.
+template <int DIM, int L>
 __global__ void k_nlist_export(DevParams P, Sorted G, uint32_t* __restrict__ counts, uint32_t* __restrict__ list,
                                uint32_t max_per, uint32_t* __restrict__ flags) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.n) return;
-    const uint32_t id = G.id[k], split = (uint32_t)P.vl_split, word = G.ncount[k];
+    const uint32_t id = G.id[k];
+    const uint32_t index = P.reuse == kReuseCell ? kCellEntryIndex : 0xFFFFFFFFu;
     uint32_t c = 0;
-    for (uint32_t u = 0; u < split; u++) c += split_count(word, u, split);
+    for (uint32_t u = 0; u < (uint32_t)L; u++) {
+        const uint32_t m = sub_count<L>(G.ncount[k], u);
+        for (uint32_t e = 0; e < m; e++, c++)
+            if (c < max_per)
+                list[(size_t)id * max_per + c] =
+                    G.id[G.nlist[((size_t)(u + L * (e >> 2)) * P.n + k) * 4 + (e & 3u)] & index];
+    }
     counts[id] = c;
-    // a searched (over-full) particle stores at most the list capacity: a full
-    // row may have lost entries, which this copy cannot show
+    // a searched particle stores at most the list capacity: a full row may have
+    // lost entries, which this copy cannot show
     const bool clipped = c == (uint32_t)Vl<DIM>::cap && G.vcount[k] == kListOver;
     if (c > max_per || clipped) atomicOr(flags, RRSPH_FLAG_NEIGHBOUR_OVERFLOW);
-    const uint32_t* const nslab = G.nlist + (size_t)k * 4;
-    uint32_t e = 0;
-    for (uint32_t u = 0; u < split; u++) {
-        const uint32_t m = split_count(word, u, split);
-        for (uint32_t j = 0; j < m && e < max_per; j++, e++)
-            list[(size_t)id * max_per + e] = G.id[nslab[(size_t)(u + split * (j >> 2)) * 4 * P.n + (j & 3u)] & Vl<DIM>::index];
-    }
 }
 
 }  // namespace
@@ -945,7 +807,8 @@ template <int DIM>
 void launch_nlist_export(const DevParams& P, const Sorted& G, uint32_t* counts, uint32_t* list, uint32_t max_per,
                          uint32_t* flags, cudaStream_t st) {
     const unsigned blocks = (P.n + 255) / 256;
-    k_nlist_export<DIM><<<blocks, 256, 0, st>>>(P, G, counts, list, max_per, flags);
+    if (P.vl_split == 4) k_nlist_export<DIM, 4><<<blocks, 256, 0, st>>>(P, G, counts, list, max_per, flags);
+    else k_nlist_export<DIM, 1><<<blocks, 256, 0, st>>>(P, G, counts, list, max_per, flags);
 }
 
 namespace {

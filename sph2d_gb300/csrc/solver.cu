@@ -199,6 +199,24 @@ int fill_dev_params(const rrsph_params& p, rrsph::DevParams& P) {
     M.ap_inv_wdelta = (float)(1.0 / P.ap_wdelta);
     M.avel_coef2 = (float)(2.0 * P.avg_vel_coef);
     M.dhc = (float)P.delta_sph_dhc;
+    rrsph::ReuseF& U = P.rf;
+    {
+        auto split = [](double v) {
+            const float hi = (float)v;
+            return rrsph::F2{hi, (float)(v - (double)hi)};
+        };
+        const float near = M.inv_h * M.inv_h * M.kf[1];
+        const double a = 0.5 * M.mass * near;
+        U.u = M.cell / (float)(1 << rrsph::kFixBits);  // exact
+        U.w = split((double)M.mass * M.kf[1]);
+        U.a = split(a);
+        U.m = split(M.mass);
+        U.far = (float)((double)M.inv_h * M.kf[1] / near);
+        U.visc = P.art_visc ? -2.0f * M.av_alpha_c * M.h : 0.0f;
+        U.bulk = P.art_visc ? 2.0f * M.av_beta * M.h : 0.0f;
+        U.lj_D = (float)(P.lj_D / a);
+        U.lj_r2 = M.lj_rr0 * M.lj_rr0;
+    }
     rrsph::PairConst& C = P.pc;
     C.inv_h = P.inv_h;
     C.h = P.h;
@@ -254,8 +272,7 @@ void set_verlet_params(rrsph_solver* s) {
     s->P.vl_skin_edge = (float)(skin * 1.01);
     // reset + sort (3, or 3 per 8-bit pass) + reorder + build (a step that reuses the
     // lists launches nothing for them: the key pass wrote its cell-order copies)
-    s->vl_extra_launches = 3ull + (s->G.scattered ? 3ull : 3ull * (unsigned long long)((s->sort_bits + 7) / 8)) +
-                           (s->P.keep_cells && !s->G.scattered ? 1ull : 0ull);
+    s->vl_extra_launches = 3ull + (s->G.scattered ? 3ull : 3ull * (unsigned long long)((s->sort_bits + 7) / 8));
 }
 
 int check_handle(rrsph_solver* s, const char* fn) {
@@ -316,12 +333,13 @@ void enqueue_forces(rrsph_solver* s, uint32_t terms, rrsph::StepScalars* scal, i
 // the lists has its cell-order copies from the key pass). The rebuilt grid
 // stays in (keys_a, ids_a) while the lists are reused: the key pass of every
 // step rewrites keys_in.
-// Neighbour reuse: the step of parity `read` reads P4 / V4 [read]; the key
+// Neighbour reuse: the step of parity `read` reads positions / V4 [read]; the key
 // pass writes its copies into [write].
 void set_verlet_copies(rrsph_solver* s, int read, int write) {
     s->G.P4 = s->p4buf[read];
+    s->G.pos = reinterpret_cast<rrsph::Pos*>(s->p4buf[read]);
     s->G.V4 = s->v4buf[read];
-    s->G.P4n = s->p4buf[write];
+    s->G.posn = reinterpret_cast<rrsph::Pos*>(s->p4buf[write]);
     s->G.V4n = s->v4buf[write];
     if (s->G.VD4n) {
         s->G.VD4 = s->vd4buf[read];
@@ -329,37 +347,17 @@ void set_verlet_copies(rrsph_solver* s, int read, int write) {
     }
 }
 
-// Whether the cell-tile density pass runs (compile-time variant: 2D summation
-// density with the cubic kernel), which reads the last build's cell table.
-bool tiles_active(const rrsph_solver* s) {
-    return RRSPH_DENSITY_CELL_TILES && s->verlet && s->dim == 2 && s->P.density_treatment == 0 && s->P.all_cubic;
-}
-// The key pass keeps or clears cell-table entries as the density pass needs
-// (the counting sort rewrites the whole table: kept); on a change the table is
-// cleared wholesale (no entry of another grid stays).
-int set_keep_cells(rrsph_solver* s) {
-    const int keep = s->G.scattered || tiles_active(s) ? 1 : 0;
-    if (keep != s->P.keep_cells) {
-        s->P.keep_cells = keep;
-        RRSPH_CUDA_TRY(cudaMemsetAsync(s->G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream));
-    }
-    return RRSPH_OK;
-}
-
 void enqueue_verlet_rebuild(rrsph_solver* s, cudaStream_t st) {
-    rrsph::launch_verlet_reset(s->S.vl_rebuild, s->S.vl_gone, s->vl_builds, st);
-    if (s->P.keep_cells && !s->G.scattered) {  // the previous build's table stayed in place: clear it for the reorder
-        rrsph::launch_clear_cells(s->G.cell_start, s->P.max_cells, st);
-        s->launches++;
-    }
+    rrsph::launch_verlet_reset(s->S.vl_rebuild, s->S.vl_gone, s->S.vl_far, s->vl_builds, st);
     sort_grid(s, st);
     const bool cont = s->P.density_treatment != 0;
     rrsph::GatherSrc fsrc{s->S.vpx, s->S.vpy, s->S.vpz, cont ? s->S.rho_pred : s->S.rho, nullptr, 1};
     if (s->dim == 3) {
-        rrsph::launch_reorder<3>(s->P, s->S, s->G, fsrc, rrsph::kReorderMixed, st);
+        rrsph::launch_reorder<3>(s->P, s->S, s->G, fsrc, rrsph::kReorderReuse, st);
         rrsph::launch_verlet_build<3>(s->P, s->S, s->G, st);
     } else {
-        rrsph::launch_reorder<2>(s->P, s->S, s->G, fsrc, rrsph::kReorderMixed, st);
+        rrsph::launch_reorder<2>(s->P, s->S, s->G, fsrc,
+                                 s->P.reuse == rrsph::kReuseCell ? rrsph::kReorderMixed : rrsph::kReorderReuse, st);
         rrsph::launch_verlet_build<2>(s->P, s->S, s->G, st);
     }
     s->launches += 3;
@@ -612,25 +610,29 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
         if (d3) { A(S.coff4, n); A(S.vpf4, n); } else { A(S.coff2, n); A(S.vpf2, n); }
         if (n < rrsph::verlet_max_particles(s->dim)) {  // neighbour reuse
             const size_t cap = (size_t)rrsph::verlet_cap(s->dim);
-            A(S.cxy, n); A(S.bcxy, n); A(S.slot, n); A(S.vl_rebuild, 2); A(s->vl_builds, 1);
+            A(S.slot, n); A(S.vl_rebuild, 4); A(s->vl_builds, 1);
             if (d3) {
-                A(S.boff4, n);
-            } else {
-                A(S.boff, n);
+                A(S.fix4, n); A(S.bfix4, n);
+            } else if (rrsph::verlet_split(2, (uint32_t)n) == 1) {
+                A(S.fix2, n); A(S.bfix2, n);
+            } else {  // kReuseCell
+                A(S.bcxy, n); A(S.boff, n);
             }
             S.vl_gone = S.vl_rebuild + 1;
+            S.vl_far = S.vl_rebuild + 2;
             A(G.vlist, cap * n); A(G.vcount, n); A(G.nlist, cap * n); A(G.ncount, n);
         }
-        A(G.P4, n); A(G.V4, n); A(G.PR, n);
+        A(G.P4, n + 1); A(G.V4, n); A(G.PR, n);  // (reuse: row n of an absent particle)
         if (cont) A(G.VD4, n);
         s->p4buf[0] = s->p4buf[1] = G.P4;
         s->v4buf[0] = s->v4buf[1] = G.V4;
         s->vd4buf[0] = s->vd4buf[1] = G.VD4;
         if (G.vlist) {
-            A(s->p4buf[1], n); A(s->v4buf[1], n);
+            A(s->p4buf[1], n + 1); A(s->v4buf[1], n);
             if (cont) A(s->vd4buf[1], n);
         }
-        G.P4n = s->p4buf[1];
+        G.pos = reinterpret_cast<rrsph::Pos*>(s->p4buf[0]);
+        G.posn = reinterpret_cast<rrsph::Pos*>(s->p4buf[1]);
         G.V4n = s->v4buf[1];
         G.VD4n = cont ? s->vd4buf[1] : nullptr;
         if (!d3) A(G.nbmask, 10 * n);
@@ -649,27 +651,35 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
             size_t bytes;
             const char* name;
         } zero[] = {{S.vl_rebuild, 0xFF, sizeof(uint32_t), "rebuild flag"},
-                    {S.vl_gone, 0, sizeof(uint32_t), "build flags"},
+                    {S.vl_gone, 0, 3 * sizeof(uint32_t), "build flags"},
                     {s->vl_builds, 0, sizeof(unsigned long long), "build count"},
                     {G.vcount, 0, n * sizeof(uint32_t), "candidate counts"},
                     {G.ncount, 0, n * sizeof(uint32_t), "neighbour counts"},
-                    {S.bcxy, 0, n * sizeof(uint32_t), "build cells"},
                     {S.slot, 0, n * sizeof(uint32_t), "build slots"},
-                    {d3 ? (void*)S.boff4 : (void*)S.boff, 0, n * (d3 ? sizeof(float4) : sizeof(float2)), "build offsets"},
+                    {d3 ? (void*)S.bfix4 : (S.bfix2 ? (void*)S.bfix2 : (void*)S.boff), 0,
+                     n * (d3 ? sizeof(int4) : sizeof(int2)), "build positions"},
+                    {S.bcxy, 0, S.bcxy ? n * sizeof(uint32_t) : 0, "build cells"},
                     {G.keys_a, 0, n * sizeof(uint32_t), "grid keys"},
                     {G.ids_a, 0, n * sizeof(uint32_t), "grid ids"}};
         for (const auto& z : zero) {
+            if (!z.bytes) continue;
             const cudaError_t e = cudaMemsetAsync(z.ptr, z.value, z.bytes, s->stream);
             if (e != cudaSuccess)
                 return fail(set_error(RRSPH_ERR_CUDA, std::string("rrsph_create: memset of the ") + z.name +
                                                           " failed: " + cudaGetErrorString(e)));
         }
+        // the row the lists are padded with: an absent particle
+        static const rrsph::Pos kAbsent{0, 0, 0, INFINITY};
+        for (float4* buf : s->p4buf)
+            if (cudaMemcpyAsync(buf + n, &kAbsent, sizeof(kAbsent), cudaMemcpyHostToDevice, s->stream) != cudaSuccess)
+                return fail(set_error(RRSPH_ERR_CUDA, "rrsph_create: the absent particle's row"));
         s->verlet = true;
+        s->P.reuse = S.boff ? rrsph::kReuseCell : rrsph::kReuseFixed;
         s->verlet_skin = s->dim == 3 ? kDefaultSkin3 : kDefaultSkin2;
     }
-    s->P.keep_cells = G.scattered || tiles_active(s) ? 1 : 0;  // the table is cleared wholesale below
+    s->P.keep_cells = G.scattered ? 1 : 0;
     if (s->verlet) {
-        s->P.vl_split = tiles_active(s) ? 1 : rrsph::verlet_split(s->dim, (uint32_t)n);
+        s->P.vl_split = rrsph::verlet_split(s->dim, (uint32_t)n);
         set_verlet_params(s);
     }
     if (cudaMallocHost(&s->h_scal, sizeof(rrsph::StepScalars)) != cudaSuccess ||
@@ -1171,8 +1181,6 @@ template <int DIM>
 void enqueue_component_grid(rrsph_solver* s, bool with_p) {
     s->keys_ready = false;  // this grid's keys were made without the predictor
     s->nlist_valid = false;  // and it replaces the grid the last step's list refers to
-    if (s->P.keep_cells && !s->G.scattered)  // the last build's table is still in place
-        cudaMemsetAsync(s->G.cell_start, 0xFF, (size_t)s->P.max_cells * sizeof(uint32_t), s->stream);
     if (s->S.vl_rebuild) cudaMemsetAsync(s->S.vl_rebuild, 0xFF, sizeof(uint32_t), s->stream);
     rrsph::GatherSrc fsrc{s->S.vx, s->S.vy, s->S.vz, s->S.rho, with_p ? s->S.p : nullptr, 0};
     enqueue_grid<DIM>(s, 0, s->scal, fsrc);
@@ -1407,9 +1415,9 @@ extern "C" int rrsph_set_neighbour_reuse(rrsph_solver* s, int enable, double ski
     if (skin_over_h == 0) skin_over_h = s->verlet_skin;  // keep the current skin
     drop_graphs(s);
     s->verlet = enable != 0;
+    s->P.reuse = !enable ? 0 : (s->S.boff ? rrsph::kReuseCell : rrsph::kReuseFixed);
     s->nlist_valid = false;
     if (enable) s->verlet_skin = skin_over_h;
-    if ((rc = set_keep_cells(s)) != 0) return rc;
     if (enable) set_verlet_params(s);
     if (s->S.vl_rebuild) RRSPH_CUDA_TRY(cudaMemsetAsync(s->S.vl_rebuild, 0xFF, sizeof(uint32_t), s->stream));
     s->keys_ready = false;

@@ -39,16 +39,19 @@ __device__ __forceinline__ bool in_geometry(const DevParams& P, double x, double
 enum : int { kVarCont = 1, kVarRare = 2, kVarMixed = 4 };  // continuity, XSPH or dynamic dt, FP32-mixed
 // M: 0 = FP64 step, 1 = FP32-mixed step, 2 = decided at run time from the state's buffers.
 
-// Neighbour reuse, in the key pass of particle i: the next step's cell-order
-// copies at the particle's slot of the last build, with (px, py, pz) its offset
-// from the edge of its build cell (a step that rebuilds overwrites them in its
-// new order). With continuity density V4.w is rho_predict and VD4 = (v,
-// rho - rho0), as the reorder writes them.
+// A particle that moved more than half the skin since the build asks for a
+// rebuild (one atomic per warp).
+__device__ __forceinline__ void reuse_check(const State& S, bool moved) {
+    const unsigned am = __activemask();
+    const unsigned who = __ballot_sync(am, moved);
+    if (who && (threadIdx.x & 31) == (unsigned)(__ffs(am) - 1)) atomicOr(S.vl_rebuild, 1u);
+}
+
+// Neighbour reuse, in the key pass of particle i: the velocity (and with
+// continuity density VD4) copies of the next step at slot k.
 template <int DIM>
-__device__ __forceinline__ void reuse_copies(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
-                                             float px, float py, float pz) {
-    const uint32_t k = S.slot[i];
-    G.P4n[k] = make_float4(px, py, pz, __int_as_float(S.itype[i]));
+__device__ __forceinline__ void velocity_copies(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
+                                                uint32_t k) {
     float4 v;
     if (DIM == 3) {
         v = S.vpf4[i];
@@ -63,24 +66,63 @@ __device__ __forceinline__ void reuse_copies(const DevParams& P, const State& S,
     }
     G.V4n[k] = v;
 }
-// A particle that moved more than half the skin since the build asks for a
-// rebuild (one atomic per warp).
-__device__ __forceinline__ void reuse_check(const State& S, bool moved) {
-    const unsigned am = __activemask();
-    const unsigned who = __ballot_sync(am, moved);
-    if (who && (threadIdx.x & 31) == (unsigned)(__ffs(am) - 1)) atomicOr(S.vl_rebuild, 1u);
+// kReuseCell: the same copies and test with the position as the offset (ox, oy)
+// from the edge of its cell (cx, cy).
+__device__ __forceinline__ void reuse_cell_pass(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
+                                                uint32_t cx, uint32_t cy, float ox, float oy) {
+    const uint32_t b = S.bcxy[i];
+    const float2 bo = S.boff[i];
+    // offset from the edge of the cell the particle had at the build
+    const float px = ox + (float)((int)cx - (int)(b & 0xFFFFu)) * P.mf.cell;
+    const float py = oy + (float)((int)cy - (int)(b >> 16)) * P.mf.cell;
+    const uint32_t k = S.slot[i];
+    reinterpret_cast<float4*>(G.posn)[k] = make_float4(px, py, 0.0f, __int_as_float(S.itype[i]));
+    velocity_copies<2>(P, S, G, i, k);
+    const float dx = px - bo.x, dy = py - bo.y;
+    reuse_check(S, !(dx * dx + dy * dy <= P.vl_half_skin2));
+}
+
+// Neighbour reuse, in the key pass of particle i at fixed-point position (x, y,
+// z): the next step's cell-order copies at the particle's slot of the last build (a
+// step that rebuilds overwrites them in its new order), the position for the next
+// build, and the test whether the particle has moved too far since the last. With
+// continuity density V4.w is rho_predict and VD4 = (v, rho - rho0), as the reorder
+// writes them. A particle outside the grid is searched on a fresh grid each step.
+template <int DIM>
+__device__ __forceinline__ void reuse_pass(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
+                                           uint32_t x, uint32_t y, uint32_t z, bool far) {
+    const uint32_t k = S.slot[i];
+    G.posn[k] = Pos{(int)x, (int)y, (int)z, Pos::code_of(S.itype[i], P.type_non_existent, far)};
+    velocity_copies<DIM>(P, S, G, i, k);
+    float d2;
+    if (DIM == 3) {
+        const int4 b = S.bfix4[i];
+        S.fix4[i] = make_int4((int)x, (int)y, (int)z, 0);
+        const float dx = (float)(int)(x - (uint32_t)b.x) * P.rf.u, dy = (float)(int)(y - (uint32_t)b.y) * P.rf.u,
+                    dz = (float)(int)(z - (uint32_t)b.z) * P.rf.u;
+        d2 = dx * dx + dy * dy + dz * dz;
+    } else {
+        const int2 b = S.bfix2[i];
+        S.fix2[i] = make_int2((int)x, (int)y);
+        const float dx = (float)(int)(x - (uint32_t)b.x) * P.rf.u, dy = (float)(int)(y - (uint32_t)b.y) * P.rf.u;
+        d2 = dx * dx + dy * dy;
+    }
+    if (far) *S.vl_far = 1u;
+    reuse_check(S, far || d2 > P.vl_half_skin2);
 }
 
 template <int DIM, int M>
 __device__ __forceinline__ void key_pass(const DevParams& P, const State& S, const Sorted& G, uint32_t i, double x,
                                          double y, double z, uint32_t* __restrict__ flags) {
-    const CellSplit sx = cell_split(x, P.xmin, P.cell, P.inv_cell, P.mf.cell);
-    const CellSplit sy = cell_split(y, P.ymin, P.cell, P.inv_cell, P.mf.cell);
+    constexpr uint32_t cmax = DIM == 3 ? 0x3FFu : 0xFFFFu;
+    constexpr bool FIX = M != 0;
+    const CellSplit sx = cell_split<FIX>(x, P.xmin, P.cell, P.inv_cell, P.mf.cell, cmax);
+    const CellSplit sy = cell_split<FIX>(y, P.ymin, P.cell, P.inv_cell, P.mf.cell, cmax);
     bool outside = sx.below || sy.below;
     uint64_t key;
-    CellSplit sz{0, 0.0f, false};
+    CellSplit sz{};
     if (DIM == 3) {
-        sz = cell_split(z, P.zmin, P.cell, P.inv_cell, P.mf.cell);
+        sz = cell_split<FIX>(z, P.zmin, P.cell, P.inv_cell, P.mf.cell, cmax);
         outside = outside || sz.below;
         key = split3(sx.c) | (split3(sy.c) << 1) | (split3(sz.c) << 2);
     } else {
@@ -96,6 +138,9 @@ __device__ __forceinline__ void key_pass(const DevParams& P, const State& S, con
     S.key_of[i] = (uint32_t)key;
     G.keys_in[i] = (uint32_t)key;
     G.ids_in[i] = i;
+    if (M != 0 && P.reuse == kReuseFixed)
+        reuse_pass<DIM>(P, S, G, i, sx.fix, sy.fix, sz.fix, sx.far || sy.far || (DIM == 3 && sz.far));
+    if (M == 1 && P.reuse == kReuseFixed) return;  // the loop's next grid is the reuse step's
     if (M == 0 && !(DIM == 3 ? (void*)S.coff4 : (void*)S.coff2)) return;
     // offsets from the edge of the cell the key names: the Morton code keeps 16
     // bits per axis in 2D and 10 in 3D (GridUtils.h:50-64, 92-104). A cell
@@ -106,36 +151,13 @@ __device__ __forceinline__ void key_pass(const DevParams& P, const State& S, con
         const float ox = sx.off + (float)(uint32_t)(sx.c & ~0xFFFFull) * P.mf.cell;
         const float oy = sy.off + (float)(uint32_t)(sy.c & ~0xFFFFull) * P.mf.cell;
         S.coff2[i] = make_float2(ox, oy);
-        if (S.cxy) {  // neighbour reuse: the current cell, and the displacement since the list build
-            const uint32_t cx = (uint32_t)(sx.c & 0xFFFFu), cy = (uint32_t)(sy.c & 0xFFFFu);
-            S.cxy[i] = cx | (cy << 16);
-            const uint32_t b = S.bcxy[i];
-            const float2 bo = S.boff[i];
-            // offset from the edge of the cell the particle had at the build
-            const float px = ox + (float)((int)cx - (int)(b & 0xFFFFu)) * P.mf.cell;
-            const float py = oy + (float)((int)cy - (int)(b >> 16)) * P.mf.cell;
-            reuse_copies<DIM>(P, S, G, i, px, py, 0.0f);
-            const float dx = px - bo.x, dy = py - bo.y;
-            reuse_check(S, !(dx * dx + dy * dy <= P.vl_half_skin2));
-        }
+        if (M != 0 && P.reuse == kReuseCell)
+            reuse_cell_pass(P, S, G, i, (uint32_t)(sx.c & 0xFFFFu), (uint32_t)(sy.c & 0xFFFFu), ox, oy);
     } else if (DIM == 3 && (M == 1 || S.coff4)) {
         const float ox = sx.off + (float)(uint32_t)(sx.c & ~0x3FFull) * P.mf.cell;
         const float oy = sy.off + (float)(uint32_t)(sy.c & ~0x3FFull) * P.mf.cell;
         const float oz = sz.off + (float)(uint32_t)(sz.c & ~0x3FFull) * P.mf.cell;
         S.coff4[i] = make_float4(ox, oy, oz, 0.0f);
-        if (S.cxy) {
-            const uint32_t cx = (uint32_t)(sx.c & 0x3FFu), cy = (uint32_t)(sy.c & 0x3FFu),
-                           cz = (uint32_t)(sz.c & 0x3FFu);
-            S.cxy[i] = cx | (cy << 10) | (cz << 20);
-            const uint32_t b = S.bcxy[i];
-            const float4 bo = S.boff4[i];
-            const float px = ox + (float)((int)cx - (int)(b & 0x3FFu)) * P.mf.cell;
-            const float py = oy + (float)((int)cy - (int)((b >> 10) & 0x3FFu)) * P.mf.cell;
-            const float pz = oz + (float)((int)cz - (int)(b >> 20)) * P.mf.cell;
-            reuse_copies<DIM>(P, S, G, i, px, py, pz);
-            const float dx = px - bo.x, dy = py - bo.y, dz = pz - bo.z;
-            reuse_check(S, !(dx * dx + dy * dy + dz * dz <= P.vl_half_skin2));
-        }
     }
 }
 
