@@ -15,7 +15,9 @@
 // symmetry of each pair's contribution: with Λ = λa_j − λa_i the pair adds
 // ℓ = (Λ·e) S − (Λ_LJ·e) fl to Σ_j λa_j·a_j, the same scalar seen from j or
 // from i, so every particle gathers ∂ℓ/∂(its own r, v*, rho, p) over its
-// neighbours and no pair result is scattered (no atomics). The density part is
+// neighbours and no pair result is added into another's (no atomics): with the
+// stored-pair FP64 step each pair's derivatives are evaluated once and stored for
+// both sides (they are equal or opposite), else each side evaluates them. The density part is
 // ℓ_rho = (λrho_j + λrho_i) m W(|e|), gathered the same way. The neighbour
 // pairs of step n are the forward step's own: its sorted grid (keys, ids) and
 // the neighbour masks its density pass recorded are kept for every step of the
@@ -34,6 +36,7 @@
 #include "../host/error.hpp"
 #include "kernels.cuh"
 #include "neighbour.cuh"
+#include "pairs64.cuh"
 #include "sort.cuh"
 #include "solver_impl.cuh"
 
@@ -62,6 +65,8 @@ struct AdjBuf {
     double* lrho;         // total λrho (cell order)
     double* pr2;          // p / rho^2 (cell order)
     double* gvx;          // dL/d(piston vx) per piston particle (id order)
+    double2* la;          // stored pairs: λa of step n (cell order)
+    double* rec;          // stored pairs: [cap][n] records of six derivatives
 };
 
 namespace {
@@ -347,6 +352,252 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_density(DevParams P, Sorted
     A.out_ry[id] += gry;
 }
 
+// ------------------------------------------- each pair once (pairs64.cuh) --
+// k_adj_reorder for the stored pairs: the same, into the rows and float offsets
+// (as k_reorder's) that the neighbour masks and the pair passes read.
+__global__ void k_adj_pair_reorder(DevParams P, Sorted G, SnapView sn, const double* __restrict__ rho_n, AdjBuf A,
+                                   double dt, double v_dt, int piston) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.n) return;
+    const uint32_t key = G.key[k];
+    const uint32_t id = G.id[k];
+    if (k == 0 || G.key[k - 1] != key) G.cell_start[key] = k;
+    if (k == P.n - 1 || G.key[k + 1] != key) G.cell_end[key] = k + 1;
+    const int32_t t = sn.itype[id];
+    const double rho = rho_n[id], x = sn.rx[id], y = sn.ry[id];
+    const double p = eos_p(P, rho);
+    const CellSplit cx = cell_split<false>(x, P.xmin, P.cell, P.inv_cell, P.mf.cell);
+    const CellSplit cy = cell_split<false>(y, P.ymin, P.cell, P.inv_cell, P.mf.cell);
+    float4 o = make_float4(cx.off + (float)(uint32_t)(cx.c & ~0xFFFFull) * P.mf.cell,
+                           cy.off + (float)(uint32_t)(cy.c & ~0xFFFFull) * P.mf.cell, 0.0f, 0.0f);
+    const float half = 0.5f * P.mf.cell;
+    if (!(fmaxf(fabsf(o.x - half), fabsf(o.y - half)) <= half * 1.001f)) o.x = __int_as_float(0x7FC00000);
+    if (t == P.type_non_existent) o.x = __int_as_float(0x7F800000);
+    G.P4[k] = o;
+    G.itype[k] = t;
+    reinterpret_cast<double2*>(G.pr)[k] = make_double2(x, y);
+    reinterpret_cast<double2*>(G.pv)[k] = make_double2(sn.vx[id] + sn.ax[id] * dt * 0.5, sn.vy[id] + sn.ay[id] * dt * 0.5);
+    reinterpret_cast<double2*>(G.pq)[k] = make_double2(rho, p / (rho * rho));
+    double lrx = A.in_rx[id], lry = A.in_ry[id], lvx = A.in_vx[id], lvy = A.in_vy[id];
+    double lax = A.in_ax[id], lay = A.in_ay[id];
+    if (t > 0) {  // v' = v + a v_dt, r' = r + v' dt
+        const double mx = lvx + dt * lrx, my = lvy + dt * lry;
+        lvx = mx;
+        lvy = my;
+        lax += v_dt * mx;
+        lay += v_dt * my;
+    }
+    if (piston && id >= P.nwm_start && id < P.nwm_end) {  // r.x += vx dt, v.x = vx
+        A.gvx[id] = lrx * dt + lvx;
+        lvx = 0.0;
+    }
+    A.out_rx[id] = lrx;
+    A.out_ry[id] = lry;
+    A.out_vx[id] = lvx;
+    A.out_vy[id] = lvy;
+    A.la[k] = make_double2(lax, lay);
+}
+
+// A pair's derivatives as k gathers them (e = r_i - r_k, s2 = |e|^2): of its own
+// r and v*, the pressure terms' Σ m sc Λ·e and the viscosity's share of ∂/∂rho.
+// i's are the same with the first four opposite. msc: m sc.
+struct AdjTerms {
+    double rx, ry, vx, vy, p, rho, msc;
+};
+template <bool NEAR>
+__device__ __forceinline__ AdjTerms adj_terms(const DevParams& P, const Sorted& G, const AdjBuf& A, uint32_t k,
+                                              uint32_t i, D3 e, double s2) {
+    const PairConst& C = P.pc;
+    AdjTerms T{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const double y1 = inv_root_40(s2);
+    if (__double2hiint(y1) == 0x7FF00000) return T;  // coincident: every derivative is along e = 0
+    const double r = s2 * y1, hy = half_of(y1);
+    const double dist = fma(fma(-r, r, s2), hy, r);
+    const double y = fma(y1, fma(-r, hy, 0.5), y1);
+    const double q = dist * C.inv_h;
+    double sc, sc1;  // m sc, m (dsc/ddist)/dist
+    if (NEAR) {
+        sc = fma(C.s1q, q, C.s1);
+        sc1 = C.s1q * C.inv_h * y;
+    } else {
+        const double t = 2.0 - q;
+        const bool in = __double2hiint(t) >= 0;
+        sc = in ? (C.s2 * y) * (t * t) : 0.0;
+        sc1 = in ? -(C.s2 * t) * ((y * y) * fma(t, y, 2.0 * C.inv_h)) : 0.0;
+    }
+    T.msc = sc;
+    const double2 lk = A.la[k], li = A.la[i];
+    const double2 vk = reinterpret_cast<const double2*>(G.pv)[k], vi = reinterpret_cast<const double2*>(G.pv)[i];
+    const double2 qk = reinterpret_cast<const double2*>(G.pq)[k], qi = reinterpret_cast<const double2*>(G.pq)[i];
+    const double lx = lk.x - li.x, ly = lk.y - li.y;
+    const double le = fma(lx, e.x, ly * e.y);
+    const double PF = qi.y + qk.y;
+    const double dvx = vk.x - vi.x, dvy = vk.y - vi.y;
+    const double vr = -fma(dvx, e.x, dvy * e.y);
+    T.p = sc * le;
+    if (C.visc && __double2hiint(vr) < 0) {
+        const double sp = s2 + C.etq_h2, rs = qi.x + qk.x, x = sp * rs;
+        const double inv0 = inverse_40(x), inv = fma(inv0, fma(-x, inv0, 1.0), inv0);
+        const double hd = C.h * (inv * rs), inv_rbar = 2.0 * (inv * sp);
+        const double ac = P.av_alpha * P.c_av, bmu = P.av_beta * (hd * vr);
+        const double Pi = (bmu - ac) * (hd * vr) * inv_rbar;
+        const double dv = -sc * ((2.0 * bmu - ac) * inv_rbar) * hd;   // coefficient of dv in ∂S/∂e
+        const double S = sc * (PF + Pi);
+        const double a = le * fma(sc1, PF + Pi, 2.0 * dv * vr * (inv * rs)), b = le * dv;
+        T.rx = -fma(lx, S, fma(a, e.x, b * dvx));
+        T.ry = -fma(ly, S, fma(a, e.y, b * dvy));
+        T.vx = b * e.x;
+        T.vy = b * e.y;
+        T.rho = -(T.p * 0.5) * (Pi * inv_rbar);
+    } else {
+        const double S = sc * PF, a = le * (sc1 * PF);
+        T.rx = -fma(lx, S, a * e.x);
+        T.ry = -fma(ly, S, a * e.y);
+    }
+    const int32_t tk = G.itype[k], ti = G.itype[i];
+    if (lj_pair(P, tk, ti) && dist < C.lj_rr0) {
+        const double Lx = tk > 0 ? lk.x : -li.x, Ly = tk > 0 ? lk.y : -li.y;
+        const double rn = C.lj_rr0 * y;
+        const double rn2 = rn * rn, rn4 = rn2 * rn2, rn12 = rn4 * rn4 * rn4;
+        const double inv_s = y * y;
+        const double fl = C.lj_D * (rn12 - rn4) * inv_s;
+        const double fls = C.lj_D * (-7.0 * rn12 + 3.0 * rn4) * inv_s * inv_s;
+        const double LE = Lx * e.x + Ly * e.y;
+        T.rx += Lx * fl + 2.0 * LE * fls * e.x;
+        T.ry += Ly * fl + 2.0 * LE * fls * e.y;
+    }
+    return T;
+}
+__device__ __forceinline__ AdjTerms adj_terms_any(const DevParams& P, const Sorted& G, const AdjBuf& A, uint32_t k,
+                                                  uint32_t i, D3 e, double s2) {
+    return s2 < P.h * P.h ? adj_terms<true>(P, G, A, k, i, e, s2) : adj_terms<false>(P, G, A, k, i, e, s2);
+}
+
+// Adjoint of update_acceleration, each pair once: six derivatives into both
+// columns, m sc kept by the owner. About 45 FP64 operations a pair, 25 more for an
+// approaching one, against some 150 for each side in k_adj_forces (42k particles:
+// 260 us).
+__global__ void __launch_bounds__(128) k_adj_pair_forces(DevParams P, Sorted G, AdjBuf A) {
+    __shared__ uint2 stacks[4 * 2 * kStack];
+    const uint32_t cap = P.pc.cap;
+    const size_t n = P.n;
+    walk_pairs<2, true, true>(P, G, stacks, [&](const uint2 w, bool active, auto near) {
+        if (!active) return;
+        const Pair q = pair_of(w, warp_first());
+        const uint32_t ri = rank_of<2>(P, G, q.i, q.c, q.bit);
+        const D3 a = row<2>(G.pr, q.k), b = row<2>(G.pr, q.i);
+        const D3 e{b.x - a.x, b.y - a.y, 0.0};
+        const AdjTerms T = adj_terms<decltype(near)::value>(P, G, A, q.k, q.i, e, dot<2>(e, e));
+        if (q.rank < cap) {
+            double2* const o = reinterpret_cast<double2*>(A.rec + (q.rank * n + q.k) * 6);
+            o[0] = make_double2(T.rx, T.ry);
+            o[1] = make_double2(T.vx, T.vy);
+            o[2] = make_double2(T.p, T.rho);
+        }
+        if (ri < cap) {
+            double2* const o = reinterpret_cast<double2*>(A.rec + (ri * n + q.i) * 6);
+            o[0] = make_double2(flip(T.rx), flip(T.ry));
+            o[1] = make_double2(flip(T.vx), flip(T.vy));
+            o[2] = make_double2(T.p, T.rho);
+        }
+        if (q.order < cap) {
+            G.ps[q.order * n + q.k] = T.msc;
+            G.prank[q.order * n + q.k] = (uint8_t)min(ri, 255u);
+        }
+    });
+}
+
+// The sums of those, and with them what k_adj_forces does per particle: v* = v +
+// a_prev dt/2 passes λv* to λv and λa_prev, λrho collects the EOS chain rule.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_pair_sum(DevParams P, Sorted G, AdjBuf A, double dt) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.n) return;
+    const size_t n = P.n;
+    uint32_t over, slots;
+    const bool more = stored_slots<2>(P, G, k, over, slots);
+    double rx = 0.0, ry = 0.0, vx = 0.0, vy = 0.0, gp = 0.0, grho = 0.0;
+#pragma unroll 2
+    for (uint32_t s = 0; s < slots; s++) {
+        const double2* const o = reinterpret_cast<const double2*>(A.rec + (s * n + k) * 6);
+        const double2 r = o[0], v = o[1], t = o[2];
+        rx += r.x;
+        ry += r.y;
+        vx += v.x;
+        vy += v.y;
+        gp += t.x;
+        grho += t.y;
+    }
+    if (more && G.itype[k] != P.type_non_existent) {
+        unstored_neighbours<2>(P, G, k, over, slots, [&](uint32_t i, D3 e, double s2) {
+            const AdjTerms T = adj_terms_any(P, G, A, k, i, e, s2);
+            rx += T.rx;
+            ry += T.ry;
+            vx += T.vx;
+            vy += T.vy;
+            gp += T.p;
+            grho += T.rho;
+        });
+    }
+    const double2 q = reinterpret_cast<const double2*>(G.pq)[k];
+    const uint32_t id = G.id[k];
+    A.out_rx[id] += rx;
+    A.out_ry[id] += ry;
+    A.out_vx[id] += vx;
+    A.out_vy[id] += vy;
+    A.out_ax[id] = vx * dt * 0.5;
+    A.out_ay[id] = vy * dt * 0.5;
+    // ∂PF/∂rho = -2 (p/rho^2) / rho, ∂PF/∂p = 1 / rho^2: the particle's own
+    grho += gp * (-2.0 * q.y / q.x);
+    A.lrho[k] = grho + eos_dp(P, q.x) * (gp / (q.x * q.x));
+}
+
+// Adjoint of density_sum, each pair once: (λrho_k + λrho_i) m sc e.
+__global__ void __launch_bounds__(128) k_adj_pair_density(DevParams P, Sorted G, AdjBuf A) {
+    __shared__ uint2 stacks[4 * kStack];
+    const uint32_t cap = P.pc.cap;
+    const size_t n = P.n;
+    walk_pairs<2, false, true>(P, G, stacks, [&](const uint2 w, bool active, auto) {
+        if (!active) return;
+        const Pair q = pair_of(w, warp_first());
+        const D3 a = row<2>(G.pr, q.k), b = row<2>(G.pr, q.i);
+        const D3 e{b.x - a.x, b.y - a.y, 0.0};
+        const bool stored = q.order < cap;
+        const size_t ao = q.order * n + q.k;
+        const double sc = stored ? G.ps[ao] : cubic_any(P.pc, dot<2>(e, e)).s;
+        const uint32_t ri = stored ? G.prank[ao] : rank_of<2>(P, G, q.i, q.c, q.bit);
+        const double cf = (A.lrho[q.k] + A.lrho[q.i]) * sc;
+        const double2 g = make_double2(cf * e.x, cf * e.y);
+        double2* const rec = reinterpret_cast<double2*>(G.pf);
+        if (q.rank < cap) rec[q.rank * n + q.k] = make_double2(flip(g.x), flip(g.y));
+        if (ri < cap) rec[ri * n + q.i] = g;
+    });
+}
+__global__ void __launch_bounds__(kAdjThreads) k_adj_pair_density_sum(DevParams P, Sorted G, AdjBuf A) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.n) return;
+    uint32_t over, slots;
+    const bool more = stored_slots<2>(P, G, k, over, slots);
+    double rx = 0.0, ry = 0.0;
+    const double2* const rec = reinterpret_cast<const double2*>(G.pf) + k;
+#pragma unroll 4
+    for (uint32_t s = 0; s < slots; s++) {
+        const double2 g = rec[(size_t)s * P.n];
+        rx += g.x;
+        ry += g.y;
+    }
+    if (more && G.itype[k] != P.type_non_existent) {
+        const double lk = A.lrho[k];
+        unstored_neighbours<2>(P, G, k, over, slots, [&](uint32_t i, D3 e, double s2) {
+            const double cf = (lk + A.lrho[i]) * cubic_any(P.pc, s2).s;
+            rx -= cf * e.x;
+            ry -= cf * e.y;
+        });
+    }
+    const uint32_t id = G.id[k];
+    A.out_rx[id] += rx;
+    A.out_ry[id] += ry;
+}
+
 // Σ dL/d(piston vx) over the piston particles, in a fixed order.
 __global__ void k_adj_piston_sum(const double* __restrict__ gvx, uint32_t start, uint32_t end,
                                  double* __restrict__ out) {
@@ -386,6 +637,8 @@ struct AdjointRun {
     uint32_t *seg_key = nullptr, *seg_id = nullptr, *seg_mask = nullptr;
     double* lam[2][6] = {};
     double *la_x = nullptr, *la_y = nullptr, *lrho = nullptr, *pr2 = nullptr, *gvx = nullptr;
+    double2* la = nullptr;  // stored pairs (else the directed gathers on seg_mask)
+    double* rec = nullptr;
     double* g_steps = nullptr;
     double *end_rho = nullptr, *end_p = nullptr;  // density and pressure at the end of the forward run
     unsigned long long* gauge_best = nullptr;
@@ -427,6 +680,24 @@ int adj_alloc(AdjointRun* run, T** ptr, size_t count) {
     run->allocs.push_back(p);
     *ptr = static_cast<T*>(p);
     return RRSPH_OK;
+}
+
+// The stored pairs' records where the forward step stores pairs and there is room
+// for them, else the masks of a segment's steps.
+int adj_alloc_pairs(rrsph_solver* s, AdjointRun* run) {
+    const size_t n = s->P.n;
+    void *la = nullptr, *rec = nullptr;
+    if (s->pairs64 && cudaMalloc(&la, n * sizeof(double2)) == cudaSuccess) {
+        run->allocs.push_back(la);
+        if (cudaMalloc(&rec, (size_t)s->P.pc.cap * n * 6 * sizeof(double)) == cudaSuccess) {
+            run->allocs.push_back(rec);
+            run->la = static_cast<double2*>(la);
+            run->rec = static_cast<double*>(rec);
+            return RRSPH_OK;
+        }
+    }
+    cudaGetLastError();
+    return adj_alloc(run, &run->seg_mask, run->K * 10 * n);
 }
 
 int alloc_snap(AdjointRun* run, rrsph::Snap& sn, size_t slots, size_t n) {
@@ -530,21 +801,33 @@ void enqueue_reverse_step(rrsph_solver* s, AdjointRun* run, uint64_t m, size_t j
     rrsph::Sorted G = s->G;
     G.key = run->seg_key + j * n;
     G.id = run->seg_id + j * n;
-    G.nbmask = run->seg_mask + j * 10 * n;
+    if (!run->rec) G.nbmask = run->seg_mask + j * 10 * n;
     rrsph::launch_clear_cells(G.cell_start, s->P.max_cells, st);
     const int nxt = cur ^ 1;
     rrsph::AdjBuf A{run->lam[cur][0], run->lam[cur][1], run->lam[cur][2], run->lam[cur][3], run->lam[cur][4],
                     run->lam[cur][5], run->lam[nxt][0], run->lam[nxt][1], run->lam[nxt][2], run->lam[nxt][3],
-                    run->lam[nxt][4], run->lam[nxt][5], run->la_x, run->la_y, run->lrho, run->pr2, run->gvx};
+                    run->lam[nxt][4], run->lam[nxt][5], run->la_x, run->la_y, run->lrho, run->pr2, run->gvx,
+                    run->la, run->rec};
     const double t = run->times[m];
     const int piston = piston_active(s, t) ? 1 : 0;
     const double v_dt = (run->step0 + m) ? run->dt : run->dt * 0.5;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     const unsigned gblocks = (unsigned)((n + rrsph::kAdjThreads - 1) / rrsph::kAdjThreads);
-    rrsph::k_adj_reorder<<<blocks, 256, 0, st>>>(s->P, G, sv, run->seg_rho + j * n, A, run->dt, v_dt, piston);
-    rrsph::k_adj_forces<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A, run->dt);
-    rrsph::k_adj_density<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A);
-    s->launches += 4;
+    if (run->rec) {
+        const dim3 pblocks((unsigned)((n + 127) / 128), rrsph::pair_slices((uint32_t)n));
+        rrsph::k_adj_pair_reorder<<<blocks, 256, 0, st>>>(s->P, G, sv, run->seg_rho + j * n, A, run->dt, v_dt, piston);
+        rrsph::launch_pair_masks<2>(s->P, s->S, G, s->scal, st);
+        rrsph::k_adj_pair_forces<<<pblocks, 128, 0, st>>>(s->P, G, A);
+        rrsph::k_adj_pair_sum<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A, run->dt);
+        rrsph::k_adj_pair_density<<<pblocks, 128, 0, st>>>(s->P, G, A);
+        rrsph::k_adj_pair_density_sum<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A);
+        s->launches += 7;
+    } else {
+        rrsph::k_adj_reorder<<<blocks, 256, 0, st>>>(s->P, G, sv, run->seg_rho + j * n, A, run->dt, v_dt, piston);
+        rrsph::k_adj_forces<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A, run->dt);
+        rrsph::k_adj_density<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A);
+        s->launches += 4;
+    }
     if (piston) {
         rrsph::k_adj_piston_sum<<<1, 256, 0, st>>>(run->gvx, s->P.nwm_start, s->P.nwm_end, run->g_steps + m);
         s->launches++;
@@ -603,7 +886,7 @@ extern "C" int rrsph_adjoint_forward(rrsph_solver* s, const rrsph_adjoint_config
     if ((rc = alloc_snap(run, run->ck, run->nck, n)) != 0 || (rc = alloc_snap(run, run->seg, run->K, n)) != 0 ||
         (rc = adj_alloc(run, &run->ck_scal, run->nck)) != 0 || (rc = adj_alloc(run, &run->seg_rho, run->K * n)) != 0 ||
         (rc = adj_alloc(run, &run->seg_key, run->K * n)) != 0 || (rc = adj_alloc(run, &run->seg_id, run->K * n)) != 0 ||
-        (rc = adj_alloc(run, &run->seg_mask, run->K * 10 * n)) != 0)
+        (rc = adj_alloc_pairs(s, run)) != 0)
         return rc;
     for (auto& set : run->lam)
         for (auto& p : set)
@@ -705,8 +988,9 @@ extern "C" int rrsph_adjoint_reverse(rrsph_solver* s, const double* dgauges, dou
                                     cudaMemcpyDeviceToDevice, st));
             ADJ_TRY(cudaMemcpyAsync(run->seg_id + (m - m0) * n, s->G.id, n * sizeof(uint32_t),
                                     cudaMemcpyDeviceToDevice, st));
-            ADJ_TRY(cudaMemcpyAsync(run->seg_mask + (m - m0) * 10 * n, s->G.nbmask, 10 * n * sizeof(uint32_t),
-                                    cudaMemcpyDeviceToDevice, st));
+            if (run->seg_mask)
+                ADJ_TRY(cudaMemcpyAsync(run->seg_mask + (m - m0) * 10 * n, s->G.nbmask, 10 * n * sizeof(uint32_t),
+                                        cudaMemcpyDeviceToDevice, st));
         }
         for (uint64_t m = m1; m-- > m0;) {
             enqueue_reverse_step(s, run, m, m - m0, cur);
