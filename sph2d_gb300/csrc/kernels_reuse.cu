@@ -61,11 +61,17 @@ __device__ __forceinline__ uint32_t packed_counts(uint32_t c) {
     return word;
 }
 
-// Separation of two positions in metres, exact before the conversion.
+// Separation of two positions in fixed-point units, exact before the conversion ...
+template <int DIM>
+__device__ __forceinline__ float3 difference(const Pos& i, const Pos& j) {
+    auto diff = [](int a, int b) { return (float)(int)((uint32_t)a - (uint32_t)b); };
+    return make_float3(diff(i.x, j.x), diff(i.y, j.y), DIM == 3 ? diff(i.z, j.z) : 0.0f);
+}
+// ... and in metres.
 template <int DIM>
 __device__ __forceinline__ float3 separation(const Pos& i, const Pos& j, float u) {
-    auto diff = [](int a, int b) { return (float)(int)((uint32_t)a - (uint32_t)b); };
-    return make_float3(diff(i.x, j.x) * u, diff(i.y, j.y) * u, DIM == 3 ? diff(i.z, j.z) * u : 0.0f);
+    const float3 d = difference<DIM>(i, j);
+    return make_float3(d.x * u, d.y * u, DIM == 3 ? d.z * u : 0.0f);
 }
 // Squared distance, + the neighbour's code: nothing for a live particle, infinite
 // or NaN (never below a cutoff) for one that is absent or not listed.
@@ -162,8 +168,16 @@ __device__ __forceinline__ float gap_to_cell(int d, float p, float cell) {
 // (the lanes of a warp store neighbouring uint4s), in cell order x outer, the last
 // group padded with the row of an absent particle (index n). A particle outside
 // the grid gets no list: it is searched, as is one with too many candidates.
+//
+// A thread first lists the cells of its window, then goes through their particles
+// in one loop: a warp's lanes then wait for the lane with the most particles, not
+// in every cell for the lane whose cell holds most (half of the lanes were idle).
+// The entries pass through a ring in shared memory, as in the density pass: no
+// branch per candidate. BUILDFIG
+constexpr int kVlBuildThreads = 128;
+constexpr int kVlRow = 5;  // cells along an axis of the window, at most
 template <int DIM>
-__global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, State S, Sorted G) {
+__global__ void __launch_bounds__(kVlBuildThreads) k_vl_build(DevParams P, State S, Sorted G) {
     constexpr int CAP = Vl<DIM>::cap;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.n) return;
@@ -184,8 +198,18 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, Sta
     }
     S.slot[id] = k;
     uint4* const slab = reinterpret_cast<uint4*>(G.vlist) + k;  // group g at slab[g * n]
-    uint4 buf = make_uint4(P.n, P.n, P.n, P.n);
-    uint32_t nl = 0;
+    // this thread's columns: the non-empty cells of a row of its window, as ranges of
+    // sorted indices, and a ring of eight list entries waiting to be stored
+    __shared__ uint2 ranges[kVlRow][kVlBuildThreads];
+    __shared__ uint32_t ring[8][kVlBuildThreads];
+    const uint32_t t = threadIdx.x;
+    uint32_t nl = 0, stored = 0;
+    auto store4 = [&]() {
+        const uint32_t q = stored & 4u;
+        if (stored < (uint32_t)CAP)
+            slab[(size_t)(stored >> 2) * P.n] = make_uint4(ring[q][t], ring[q + 1][t], ring[q + 2][t], ring[q + 3][t]);
+        stored += 4;
+    };
     if (pj.absent()) atomicOr(S.vl_gone, 1u);
     // offset from the lower edges of the key's cell
     const float px = (float)(int)((uint32_t)pj.x - (cx << kFixBits)) * U.u;
@@ -200,55 +224,83 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_vl_build(DevParams P, Sta
         vl_window<DIM>(px, cx, cell, edge, x0, x1);
         vl_window<DIM>(py, cy, cell, edge, y0, y1);
         if (DIM == 3) vl_window<DIM>(pz, cz, cell, edge, z0, z1);
-#pragma unroll 1
-        for (int dx = x0; dx <= x1; dx++) {
-#pragma unroll 1
-            for (int dy = y0; dy <= y1; dy++) {
-#pragma unroll 1
-                for (int dz = z0; dz <= z1; dz++) {
-                    // a cell none of whose points lies within the list cutoff of the
-                    // particle holds no candidate: the distance from the particle
-                    // to the cell's nearest side, per axis (the window's corner and
-                    // far diagonal cells mostly)
-                    const float gx = gap_to_cell(dx, px, cell), gy = gap_to_cell(dy, py, cell);
-                    const float gz = DIM == 3 ? gap_to_cell(dz, pz, cell) : 0.0f;
-                    if (gx * gx + gy * gy + gz * gz >= P.vl_cut2) continue;
-                    const uint32_t c = DIM == 3 ? split3_32(cx + dx) | (split3_32(cy + dy) << 1) |
-                                                      (split3_32(cz + dz) << 2)
-                                                : split2_32(cx + dx) | (split2_32(cy + dy) << 1);
-                    if (c >= P.max_cells) continue;
-                    const uint32_t s = G.cell_start[c];
-                    if (s == kEmpty) continue;
-                    const uint32_t e = G.cell_end[c];
-                    // the cell's particles four at a time: their loads issue together (an
-                    // index past the cell's end loads its last particle and is skipped)
-                    for (uint32_t i0 = s; i0 < e; i0 += kVlBatch) {
-                        Pos q[kVlBatch];
-#pragma unroll
-                        for (int u = 0; u < kVlBatch; u++) q[u] = G.pos[min(i0 + u, e - 1u)];
-#pragma unroll
-                        for (int u = 0; u < kVlBatch; u++) {
-                            const uint32_t i = i0 + u;
-                            if (i >= e || i == k) continue;
-                            if (distance2<DIM>(separation<DIM>(q[u], pj, U.u), q[u].code) < P.vl_cut2) {
-                                if (nl < (uint32_t)CAP) {
-                                    // shifted in: the group's entries in order once its fourth arrives
-                                    buf = make_uint4(buf.y, buf.z, buf.w, i);
-                                    if ((nl & 3u) == 3u) slab[(size_t)(nl >> 2) * P.n] = buf;
-                                }
-                                nl++;
-                            }
-                        }
-                    }
+        const float cut = P.vl_cut2 / (U.u * U.u);
+        uint32_t nr = 0;
+        // notes the particles of cell c, if a point of it lies within the list cutoff
+        // of the particle: the distances to its nearest sides, per axis, squared and
+        // summed (the window's corner and far diagonal cells mostly hold no candidate)
+        auto note = [&](uint32_t c, float gap2) {
+            if (gap2 >= P.vl_cut2 || c >= P.max_cells) return;
+            const uint32_t s = G.cell_start[c];
+            if (s != kEmpty) ranges[nr++][t] = make_uint2(s, G.cell_end[c]);
+        };
+        // the noted particles four at a time, their loads together (the rows past a
+        // cell's end are another cell's, or the spare ones past the last: skipped)
+        auto candidates = [&]() {
+            uint32_t r = 0, i0 = 0, e = 0;
+            while (true) {
+                if (i0 >= e) {
+                    if (r == nr) break;
+                    const uint2 se = ranges[r++][t];
+                    i0 = se.x;
+                    e = se.y;
                 }
+                const Pos* const row = G.pos + i0;
+                Pos q[kVlBatch];
+#pragma unroll
+                for (int u = 0; u < kVlBatch; u++) q[u] = row[u];
+#pragma unroll
+                for (int u = 0; u < kVlBatch; u++) {
+                    const uint32_t i = i0 + u;
+                    const bool in = distance2<DIM>(difference<DIM>(q[u], pj), q[u].code) < cut && i < e && i != k;
+                    if (in) ring[nl & 7u][t] = i;
+                    nl += in;
+                }
+                if (nl - stored >= 4) store4();
+                i0 += kVlBatch;
+            }
+            nr = 0;
+        };
+        auto square = [](float x) { return x * x; };
+        if (DIM == 3) {
+            const uint32_t mz0 = split3_32(cz + z0);
+#pragma unroll 1
+            for (int dx = x0; dx <= x1; dx++) {
+                const uint32_t mx = split3_32(cx + dx);
+                const float gx = square(gap_to_cell(dx, px, cell));
+#pragma unroll 1
+                for (int dy = y0; dy <= y1; dy++) {
+                    const float gxy = gx + square(gap_to_cell(dy, py, cell));
+                    if (gxy >= P.vl_cut2) continue;
+                    const uint32_t mxy = mx | (split3_32(cy + dy) << 1);
+                    uint32_t mz = mz0;
+#pragma unroll 1
+                    for (int dz = z0; dz <= z1; dz++) {
+                        note(mxy | (mz << 2), gxy + square(gap_to_cell(dz, pz, cell)));
+                        mz = ((mz | 0xF6DB6DB6u) + 1u) & 0x09249249u;  // of the next z
+                    }
+                    candidates();
+                }
+            }
+        } else {
+            const uint32_t my0 = split2_32(cy + y0);
+#pragma unroll 1
+            for (int dx = x0; dx <= x1; dx++) {
+                const uint32_t mx = split2_32(cx + dx);
+                const float gx = square(gap_to_cell(dx, px, cell));
+                uint32_t my = my0;
+#pragma unroll 1
+                for (int dy = y0; dy <= y1; dy++) {
+                    note(mx | (my << 1), gx + square(gap_to_cell(dy, py, cell)));
+                    my = ((my | 0xAAAAAAAAu) + 1u) & 0x55555555u;  // of the next y
+                }
+                candidates();
             }
         }
     }
-    if (nl < (uint32_t)CAP && (nl & 3u)) {  // the padded last group: its m entries to the front
-        const uint32_t m = nl & 3u;
-        buf = m == 1u ? make_uint4(buf.w, P.n, P.n, P.n)
-                      : (m == 2u ? make_uint4(buf.z, buf.w, P.n, P.n) : make_uint4(buf.y, buf.z, buf.w, P.n));
-        slab[(size_t)(nl >> 2) * P.n] = buf;
+    if (nl > stored) {  // the last group, padded
+        for (uint32_t u = nl; u < stored + 4; u++) ring[u & 7u][t] = P.n;
+        store4();
     }
     const bool search = outside || nl > (uint32_t)CAP;
     G.vcount[k] = search ? kListOver : nl;
@@ -707,8 +759,7 @@ void launch_verlet_upload_check(uint32_t* rebuild, const uint32_t* gone, cudaStr
 template <int DIM>
 void launch_verlet_build(const DevParams& P, const State& S, const Sorted& G, cudaStream_t st) {
     if (P.reuse == kReuseCell) return launch_verlet_build_cell(P, S, G, st);
-    constexpr int kBuildThreads = 128;
-    k_vl_build<DIM><<<(P.n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, st>>>(P, S, G);
+    k_vl_build<DIM><<<(P.n + kVlBuildThreads - 1) / kVlBuildThreads, kVlBuildThreads, 0, st>>>(P, S, G);
 }
 // Warps per 32 particles of the two gathers (DevParams::vl_split, fixed when a
 // solver is created): four where a thread per particle leaves the SMs a few warps

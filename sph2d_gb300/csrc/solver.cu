@@ -622,13 +622,13 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
             S.vl_far = S.vl_rebuild + 2;
             A(G.vlist, cap * n); A(G.vcount, n); A(G.nlist, cap * n); A(G.ncount, n);
         }
-        A(G.P4, n + 1); A(G.V4, n); A(G.PR, n);  // (reuse: row n of an absent particle)
+        A(G.P4, n + 4); A(G.V4, n); A(G.PR, n);  // (reuse: row n of an absent particle; batches of four read on)
         if (cont) A(G.VD4, n);
         s->p4buf[0] = s->p4buf[1] = G.P4;
         s->v4buf[0] = s->v4buf[1] = G.V4;
         s->vd4buf[0] = s->vd4buf[1] = G.VD4;
         if (G.vlist) {
-            A(s->p4buf[1], n + 1); A(s->v4buf[1], n);
+            A(s->p4buf[1], n + 4); A(s->v4buf[1], n);
             if (cont) A(s->vd4buf[1], n);
         }
         G.pos = reinterpret_cast<rrsph::Pos*>(s->p4buf[0]);

@@ -87,3 +87,18 @@ def test_particles_outside_the_grid_and_absent_ones(gpu_available, dim):
             c.r[first + j, 0] = p.x_mingeom - (cells + 0.3 * j) * cell
             c.v[first + j] = 0.0
     _same(p, c, steps=2)
+
+
+@pytest.mark.parametrize("dim,nx,ny", [(2, 12, 9), (2, 300, 150), (3, 8, 6)])
+@pytest.mark.parametrize("every", [1, 2, 3])
+def test_crowded_cells(gpu_available, dim, nx, ny, every):
+    """A patch of the fluid drawn together: cells with several batches of candidates,
+    lists that are full to the last group, and particles with more than a list holds."""
+    c = _scene(dim, 1, nx, ny)
+    c.v[:] = 0.0
+    m = 60 * every if dim == 2 else 130 * every
+    m = min(m, c.particle["nfluid"]) if dim == 2 else min(m, c.particle["nfluid"] // 2)
+    centre = c.r[:m].mean(axis=0)
+    c.r[:m:2] = centre + (c.r[:m:2] - centre) * 0.35
+    c.model["consistency_check"] = False
+    _same(c.params(), c, steps=2)
