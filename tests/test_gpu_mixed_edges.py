@@ -90,15 +90,15 @@ def test_particles_outside_the_grid_and_absent_ones(gpu_available, dim):
 
 
 @pytest.mark.parametrize("dim,nx,ny", [(2, 12, 9), (2, 300, 150), (3, 8, 6)])
-@pytest.mark.parametrize("every", [1, 2, 3])
-def test_crowded_cells(gpu_available, dim, nx, ny, every):
-    """A patch of the fluid drawn together: cells with several batches of candidates,
-    lists that are full to the last group, and particles with more than a list holds."""
+@pytest.mark.parametrize("factor", [0.5, 0.6])
+def test_crowded_cells(gpu_available, dim, nx, ny, factor):
+    """Every other particle of a patch drawn together: cells with several batches of
+    candidates, lists full to the last group and (0.5 in 2D) particles with more
+    candidates than a list holds, but no more neighbours than the model allows."""
     c = _scene(dim, 1, nx, ny)
     c.v[:] = 0.0
-    m = 60 * every if dim == 2 else 130 * every
-    m = min(m, c.particle["nfluid"]) if dim == 2 else min(m, c.particle["nfluid"] // 2)
-    centre = c.r[:m].mean(axis=0)
-    c.r[:m:2] = centre + (c.r[:m:2] - centre) * 0.35
-    c.model["consistency_check"] = False
+    k = min(100 if dim == 2 else 300, c.particle["nfluid"])
+    centre = c.r[:k].mean(axis=0)
+    patch = np.argsort(np.abs(c.r - centre).max(axis=1), kind="stable")[:k][::2]
+    c.r[patch] = centre + (c.r[patch] - centre) * factor
     _same(c.params(), c, steps=2)
