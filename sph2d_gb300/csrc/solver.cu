@@ -1036,6 +1036,11 @@ extern "C" int rrsph_step(rrsph_solver* s, uint64_t nsteps, double* time_io) {
 }
 
 namespace {
+// Particles above which p and rho come back while the force gather runs. us per
+// rrsph_step_host of one mixed 2D step, with / without: 2.5k 74.7 / 71.3, 10.9k
+// 95.3 / 86.1, 33k 146.2 / 123.7, 74k 191.9 / 187.8, 133k 225.6 / 231.1, 265k
+// 302.5 / 322.0; FP64: 33k 124.1 / 119.7, 133k 266.8 / 274.4.
+constexpr size_t kEarlyCopies = 100000;
 // rrsph_step_host (upload first) and rrsph_step_download (the state on the
 // device); the arguments are checked by the callers.
 int steps_and_download(rrsph_solver* s, uint64_t nsteps, double* time_io, double* r, uint32_t stride, double* v,
@@ -1045,8 +1050,9 @@ int steps_and_download(rrsph_solver* s, uint64_t nsteps, double* time_io, double
     const size_t n = s->P.n;
     // with graph replay the last step marks the end of its density pass: p, and
     // rho with summation density (the whole step leaves it), come back on a
-    // copy stream while the force gather runs
-    const bool mark = s->graphs && !s->timing;
+    // copy stream while the force gather runs. Few particles: the second stream
+    // and its events cost more than the copies take (kEarlyCopies).
+    const bool mark = s->graphs && !s->timing && n > kEarlyCopies;
     if (mark && !s->dl_stream) {
         if (cudaStreamCreateWithFlags(&s->dl_stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->ev_density, cudaEventDisableTiming) != cudaSuccess ||
