@@ -87,63 +87,48 @@ __global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_mas
                 const float3 sh = stencil_shift<DIM>(c);
                 const float shx = sh.x * F.cell - pj.x, shy = sh.y * F.cell - pj.y;
                 const float shz = DIM == 3 ? sh.z * F.cell - pj.z : 0.0f;
-                auto dist2 = [&](const float4& pi) {
-                    const float dx = pi.x + shx, dy = pi.y + shy, dz = DIM == 3 ? pi.z + shz : 0.0f;
-                    return DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-                };
-                auto exact = [&](uint32_t i, uint32_t bit, uint32_t& in, uint32_t& close) {
-                    const D3 a = row<DIM>(G.pr, i), b = row<DIM>(G.pr, k);
-                    const double r2 = exact_dist2<DIM>(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y),
-                                                       DIM == 3 ? __dsub_rn(a.z, b.z) : 0.0);
-                    if (r2 < P.cut2 && G.itype[i] != P.type_non_existent) {
-                        in |= bit;
-                        if (r2 < P.h * P.h) close |= bit;
-                    }
-                };
-                if (DIM == 2) {
-                    uint32_t in = 0, close = 0, bit = 1;
-#pragma unroll 4
-                    for (uint32_t i = s; i < e; i++, bit <<= 1) {
-                        const float d2 = dist2(G.P4[i]);
-                        if (d2 < F.cut2_lo) in |= bit;
-                        if (d2 < h2) close |= bit;
-                        if (!(d2 < F.cut2_lo) && !(d2 >= F.cut2_hi)) exact(i, bit, in, close);
-                    }
-                    mask = in;
-                    near = close;
-                } else {
-                    // twice as many in a cell: a word of bits at a time, the loads of four
-                    // together (an index past the cell's end loads its last particle; its bit
-                    // is dropped). 385k particles 436 -> 314 us; in 2D 409k 55 -> 62
+                // a word of bits at a time, the loads of a batch together (an index past the
+                // cell's end loads its last particle; its bit is dropped); in 2D, with half
+                // as many in a cell, batches of two: 59 us on the 409k flume, of four 62; in
+                // 3D of four: 314 us on 385k, one candidate at a time into 64-bit words 436
+                constexpr uint32_t B = DIM == 3 ? 4 : 2;
 #pragma unroll 1
-                    for (uint32_t s0 = s; s0 < e; s0 += 32) {
-                        const uint32_t len = min(e - s0, 32u);
-                        uint32_t in = 0, below = 0, close = 0;  // below the guard band, or its end; at up to one h
+                for (uint32_t s0 = s; s0 < e; s0 += 32) {
+                    const uint32_t len = min(e - s0, 32u);
+                    uint32_t in = 0, below = 0, close = 0;  // below the guard band, or its end; at up to one h
 #pragma unroll 1
-                        for (uint32_t j = 0; j < len; j += 4) {
-                            float4 q[4];
+                    for (uint32_t j = 0; j < len; j += B) {
+                        float4 q[B];
 #pragma unroll
-                            for (uint32_t u = 0; u < 4; u++) q[u] = G.P4[min(s0 + j + u, e - 1u)];
-                            uint32_t a = 0, b = 0, o = 0;
+                        for (uint32_t u = 0; u < B; u++) q[u] = G.P4[min(s0 + j + u, e - 1u)];
+                        uint32_t a = 0, b = 0, o = 0;
 #pragma unroll
-                            for (uint32_t u = 0; u < 4; u++) {
-                                const float d2 = dist2(q[u]);
-                                if (d2 < F.cut2_lo) a |= 1u << u;
-                                if (!(d2 >= F.cut2_hi)) b |= 1u << u;
-                                if (d2 < h2) o |= 1u << u;
-                            }
-                            in |= a << j;
-                            below |= b << j;
-                            close |= o << j;
+                        for (uint32_t u = 0; u < B; u++) {
+                            const float dx = q[u].x + shx, dy = q[u].y + shy, dz = DIM == 3 ? q[u].z + shz : 0.0f;
+                            const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
+                            if (d2 < F.cut2_lo) a |= 1u << u;
+                            if (!(d2 >= F.cut2_hi)) b |= 1u << u;
+                            if (d2 < h2) o |= 1u << u;
                         }
-                        const uint32_t valid = 0xFFFFFFFFu >> (32u - len);
-                        in &= valid;
-                        close &= valid;
-                        for (uint32_t band = below & valid & ~in; band; band &= band - 1)
-                            exact(s0 + __ffs(band) - 1, band & -band, in, close);
-                        mask |= (T)in << ((s0 - s) & (M::bits - 1));
-                        near |= (T)close << ((s0 - s) & (M::bits - 1));
+                        in |= a << j;
+                        below |= b << j;
+                        close |= o << j;
                     }
+                    const uint32_t valid = 0xFFFFFFFFu >> (32u - len);
+                    in &= valid;
+                    close &= valid;
+                    for (uint32_t band = below & valid & ~in; band; band &= band - 1) {
+                        const uint32_t bit = __ffs(band) - 1, i = s0 + bit;
+                        const D3 a = row<DIM>(G.pr, i), b = row<DIM>(G.pr, k);
+                        const double r2 = exact_dist2<DIM>(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y),
+                                                           DIM == 3 ? __dsub_rn(a.z, b.z) : 0.0);
+                        if (r2 < P.cut2 && G.itype[i] != P.type_non_existent) {
+                            in |= 1u << bit;
+                            if (r2 < P.h * P.h) close |= 1u << bit;
+                        }
+                    }
+                    mask |= (T)in << ((s0 - s) & (M::bits - 1));
+                    near |= (T)close << ((s0 - s) & (M::bits - 1));
                 }
                 if (c == M::nc / 2) mask &= ~((T)1 << (k - s));  // not itself
             }
