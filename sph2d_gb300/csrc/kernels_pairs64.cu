@@ -18,9 +18,11 @@
 //   k_pair_sum     accelerations (and drho) from the stored ones
 //
 // Against the directed gathers (kernels_fp64.cu; both sides of a pair, IEEE
-// forms, 22 of 32 lanes): the 409k flume's density and forces 1.93 -> 0.48 ms
-// (step 1.91 -> 0.515), 385k particles in 3D 8.25 -> 2.2 ms a step, the 6k dam
-// break 189 -> 56 us. The FP64 pipe is 74-80 % busy in the pair passes.
+// forms, 22 of 32 lanes): the 409k flume's density and forces 1.93 -> 0.46 ms
+// (masks 59 us, terms 131, density 33, forces 174, sum 40), 385k particles in 3D
+// 8.25 -> 2.0 ms a step (masks 314 us, terms 1287, sum 272), the 6k dam break 189
+// -> 46 us (its sort, 30 us of the 189, then 15). The FP64 pipe is 74-80 % busy in
+// the pair passes.
 //
 // A pair of particles k < i is evaluated by k's warp. Neighbour number s of a
 // particle (its rank in the search's order: cells in stencil order, ids

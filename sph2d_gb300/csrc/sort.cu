@@ -145,6 +145,11 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t* __rest
 }
 
 // ------------------------------------------- counting sort over the cells --
+//
+// Three launches where the radix sort takes three per eight key bits, and the
+// table with them: bound by launch latency on small sets, by the sweep of the
+// table (flume: 2.1M cells) on large ones. us with the radix sort and reorder of
+// the table, and so: 409k flume 55 / 23, 6k dam break 28 / 15.
 
 // A place in its cell for every particle (in the order the atomics arrive), and
 // the particles per tile of cells: neighbouring ids mostly share a tile, so a
