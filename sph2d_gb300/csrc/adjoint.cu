@@ -404,18 +404,16 @@ __global__ void k_adj_pair_reorder(DevParams P, Sorted G, SnapView sn, const dou
 struct AdjTerms {
     double rx, ry, vx, vy, p, rho, msc;
 };
+// Inverse distance, distance, m sc and m (dsc/ddist)/dist; false: coincident.
 template <bool NEAR>
-__device__ __forceinline__ AdjTerms adj_terms(const DevParams& P, const Sorted& G, const AdjBuf& A, uint32_t k,
-                                              uint32_t i, D3 e, double s2) {
-    const PairConst& C = P.pc;
-    AdjTerms T{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+__device__ __forceinline__ bool adj_kernel(const PairConst& C, double s2, double& y, double& dist, double& sc,
+                                           double& sc1) {
     const double y1 = inv_root_40(s2);
-    if (__double2hiint(y1) == 0x7FF00000) return T;  // coincident: every derivative is along e = 0
+    if (__double2hiint(y1) == 0x7FF00000) return false;
     const double r = s2 * y1, hy = half_of(y1);
-    const double dist = fma(fma(-r, r, s2), hy, r);
-    const double y = fma(y1, fma(-r, hy, 0.5), y1);
+    dist = fma(fma(-r, r, s2), hy, r);
+    y = fma(y1, fma(-r, hy, 0.5), y1);
     const double q = dist * C.inv_h;
-    double sc, sc1;  // m sc, m (dsc/ddist)/dist
     if (NEAR) {
         sc = fma(C.s1q, q, C.s1);
         sc1 = C.s1q * C.inv_h * y;
@@ -425,47 +423,71 @@ __device__ __forceinline__ AdjTerms adj_terms(const DevParams& P, const Sorted& 
         sc = in ? (C.s2 * y) * (t * t) : 0.0;
         sc1 = in ? -(C.s2 * t) * ((y * y) * fma(t, y, 2.0 * C.inv_h)) : 0.0;
     }
-    T.msc = sc;
+    return true;
+}
+struct AdjRows {
+    double2 lk, li;  // Λ's two sides, l = Λ
+    double lx, ly, dvx, dvy, pf, rs;
+};
+__device__ __forceinline__ AdjRows adj_rows(const Sorted& G, const AdjBuf& A, uint32_t k, uint32_t i) {
     const double2 lk = A.la[k], li = A.la[i];
     const double2 vk = reinterpret_cast<const double2*>(G.pv)[k], vi = reinterpret_cast<const double2*>(G.pv)[i];
     const double2 qk = reinterpret_cast<const double2*>(G.pq)[k], qi = reinterpret_cast<const double2*>(G.pq)[i];
-    const double lx = lk.x - li.x, ly = lk.y - li.y;
-    const double le = fma(lx, e.x, ly * e.y);
-    const double PF = qi.y + qk.y;
-    const double dvx = vk.x - vi.x, dvy = vk.y - vi.y;
-    const double vr = -fma(dvx, e.x, dvy * e.y);
+    return {lk, li, lk.x - li.x, lk.y - li.y, vk.x - vi.x, vk.y - vi.y, qi.y + qk.y, qi.x + qk.x};
+}
+// The terms of an approaching pair (viscosity), and of one without; T.p is set.
+// Pi = (beta mu - alpha c) mu / rbar with mu = h vr / (s2 + etq_h2) and 1 / rbar =
+// 2 u; the doublings are in the constants.
+__device__ __forceinline__ void adj_approaching(const DevParams& P, const AdjRows& R, D3 e, double s2, double sc,
+                                                double sc1, double le, double vr, AdjTerms& T) {
+    const PairConst& C = P.pc;
+    const double ac2 = 2.0 * P.av_alpha * P.c_av, beta2 = 2.0 * P.av_beta, beta4 = 4.0 * P.av_beta;
+    const double two_inv_h = 2.0 * C.inv_h;
+    const double sp = s2 + C.etq_h2, x = sp * R.rs;
+    const double inv0 = inverse_40(x), inv = fma(inv0, fma(-x, inv0, 1.0), inv0);
+    const double hd = C.h * (inv * R.rs), u = inv * sp, mu = hd * vr;
+    const double Pi = fma(beta2, mu, -ac2) * mu * u;
+    const double dv = -sc * (fma(beta4, mu, -ac2) * u) * hd;   // coefficient of dv in ∂S/∂e
+    const double pf = R.pf + Pi, S = sc * pf;
+    const double a = le * fma(sc1, pf, dv * mu * two_inv_h), b = le * dv;
+    T.rx = -fma(R.lx, S, fma(a, e.x, b * R.dvx));
+    T.ry = -fma(R.ly, S, fma(a, e.y, b * R.dvy));
+    T.vx = b * e.x;
+    T.vy = b * e.y;
+    T.rho = -T.p * (Pi * u);
+}
+__device__ __forceinline__ void adj_receding(const AdjRows& R, D3 e, double sc, double sc1, double le, AdjTerms& T) {
+    const double S = sc * R.pf, a = le * (sc1 * R.pf);
+    T.rx = -fma(R.lx, S, a * e.x);
+    T.ry = -fma(R.ly, S, a * e.y);
+}
+// The Lennard-Jones part of a wall pair closer than its range.
+__device__ __forceinline__ void adj_wall(const PairConst& C, const AdjRows& R, int32_t tk, D3 e, double y, AdjTerms& T) {
+    const double Lx = tk > 0 ? R.lk.x : -R.li.x, Ly = tk > 0 ? R.lk.y : -R.li.y;
+    const double rn = C.lj_rr0 * y;
+    const double rn2 = rn * rn, rn4 = rn2 * rn2, rn12 = rn4 * rn4 * rn4;
+    const double inv_s = y * y;
+    const double fl = C.lj_D * (rn12 - rn4) * inv_s;
+    const double fls = C.lj_D * (-7.0 * rn12 + 3.0 * rn4) * inv_s * inv_s;
+    const double LE = Lx * e.x + Ly * e.y;
+    T.rx += Lx * fl + 2.0 * LE * fls * e.x;
+    T.ry += Ly * fl + 2.0 * LE * fls * e.y;
+}
+template <bool NEAR>
+__device__ __forceinline__ AdjTerms adj_terms(const DevParams& P, const Sorted& G, const AdjBuf& A, uint32_t k,
+                                              uint32_t i, D3 e, double s2) {
+    const PairConst& C = P.pc;
+    AdjTerms T{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double y, dist, sc, sc1;
+    if (!adj_kernel<NEAR>(C, s2, y, dist, sc, sc1)) return T;  // coincident: every derivative is along e = 0
+    const AdjRows R = adj_rows(G, A, k, i);
+    const double le = fma(R.lx, e.x, R.ly * e.y), vr = -fma(R.dvx, e.x, R.dvy * e.y);
+    T.msc = sc;
     T.p = sc * le;
-    if (C.visc && __double2hiint(vr) < 0) {
-        const double sp = s2 + C.etq_h2, rs = qi.x + qk.x, x = sp * rs;
-        const double inv0 = inverse_40(x), inv = fma(inv0, fma(-x, inv0, 1.0), inv0);
-        const double hd = C.h * (inv * rs), inv_rbar = 2.0 * (inv * sp);
-        const double ac = P.av_alpha * P.c_av, bmu = P.av_beta * (hd * vr);
-        const double Pi = (bmu - ac) * (hd * vr) * inv_rbar;
-        const double dv = -sc * ((2.0 * bmu - ac) * inv_rbar) * hd;   // coefficient of dv in ∂S/∂e
-        const double S = sc * (PF + Pi);
-        const double a = le * fma(sc1, PF + Pi, 2.0 * dv * vr * (inv * rs)), b = le * dv;
-        T.rx = -fma(lx, S, fma(a, e.x, b * dvx));
-        T.ry = -fma(ly, S, fma(a, e.y, b * dvy));
-        T.vx = b * e.x;
-        T.vy = b * e.y;
-        T.rho = -(T.p * 0.5) * (Pi * inv_rbar);
-    } else {
-        const double S = sc * PF, a = le * (sc1 * PF);
-        T.rx = -fma(lx, S, a * e.x);
-        T.ry = -fma(ly, S, a * e.y);
-    }
+    if (C.visc && __double2hiint(vr) < 0) adj_approaching(P, R, e, s2, sc, sc1, le, vr, T);
+    else adj_receding(R, e, sc, sc1, le, T);
     const int32_t tk = G.itype[k], ti = G.itype[i];
-    if (lj_pair(P, tk, ti) && dist < C.lj_rr0) {
-        const double Lx = tk > 0 ? lk.x : -li.x, Ly = tk > 0 ? lk.y : -li.y;
-        const double rn = C.lj_rr0 * y;
-        const double rn2 = rn * rn, rn4 = rn2 * rn2, rn12 = rn4 * rn4 * rn4;
-        const double inv_s = y * y;
-        const double fl = C.lj_D * (rn12 - rn4) * inv_s;
-        const double fls = C.lj_D * (-7.0 * rn12 + 3.0 * rn4) * inv_s * inv_s;
-        const double LE = Lx * e.x + Ly * e.y;
-        T.rx += Lx * fl + 2.0 * LE * fls * e.x;
-        T.ry += Ly * fl + 2.0 * LE * fls * e.y;
-    }
+    if (lj_pair(P, tk, ti) && dist < C.lj_rr0) adj_wall(C, R, tk, e, y, T);
     return T;
 }
 __device__ __forceinline__ AdjTerms adj_terms_any(const DevParams& P, const Sorted& G, const AdjBuf& A, uint32_t k,
@@ -474,20 +496,26 @@ __device__ __forceinline__ AdjTerms adj_terms_any(const DevParams& P, const Sort
 }
 
 // Adjoint of update_acceleration, each pair once: six derivatives into both
-// columns, m sc kept by the owner. About 45 FP64 operations a pair, 25 more for an
-// approaching one, against some 150 for each side in k_adj_forces: 42k particles
-// 102 us, the sums 26 (k_adj_forces 260). Bound by the FP64 pipe.
+// columns, m sc kept by the owner. Bound by the FP64 pipe: some 30 operations for
+// every pair and 45 more for an approaching one, against some 150 for each side
+// in k_adj_forces. As in the forward step's forces, the approaching pairs go on
+// to a second stack of the warp, so that receding ones do not pay for them: 205k
+// particles 355 -> 279 us, 42k (their stacks drain half full) 50 reverse steps 16.5
+// -> 15.7 ms; k_adj_forces took 260 us a step on 42k.
+struct AdjApproach {  // a warp's second stack
+    uint2 w[kStack];
+    double ex[kStack], ey[kStack], vr[kStack], sc[kStack], sc1[kStack], le[kStack];
+};
 __global__ void __launch_bounds__(128) k_adj_pair_forces(DevParams P, Sorted G, AdjBuf A) {
     __shared__ uint2 stacks[4 * 2 * kStack];
-    const uint32_t cap = P.pc.cap;
+    __shared__ AdjApproach second_stacks[4];
+    AdjApproach& B = second_stacks[threadIdx.x >> 5];
+    const PairConst& C = P.pc;
+    const uint32_t cap = C.cap, lane = threadIdx.x & 31u;
     const size_t n = P.n;
-    walk_pairs<2, true, true>(P, G, stacks, [&](const uint2 w, bool active, auto near) {
-        if (!active) return;
-        const Pair q = pair_of(w, warp_first());
+    uint32_t held = 0;
+    auto put = [&](const Pair& q, const AdjTerms& T) {
         const uint32_t ri = rank_of<2>(P, G, q.i, q.c, q.bit);
-        const D3 a = row<2>(G.pr, q.k), b = row<2>(G.pr, q.i);
-        const D3 e{b.x - a.x, b.y - a.y, 0.0};
-        const AdjTerms T = adj_terms<decltype(near)::value>(P, G, A, q.k, q.i, e, dot<2>(e, e));
         if (q.rank < cap) {
             double2* const o = reinterpret_cast<double2*>(A.rec + (q.rank * n + q.k) * 6);
             o[0] = make_double2(T.rx, T.ry);
@@ -504,7 +532,63 @@ __global__ void __launch_bounds__(128) k_adj_pair_forces(DevParams P, Sorted G, 
             G.ps[q.order * n + q.k] = T.msc;
             G.prank[q.order * n + q.k] = (uint8_t)min(ri, 255u);
         }
+    };
+    auto second = [&](uint32_t at) {
+        const Pair q = pair_of(B.w[at], warp_first());
+        const D3 e{B.ex[at], B.ey[at], 0.0};
+        const double sc = B.sc[at], le = B.le[at];
+        AdjTerms T{0.0, 0.0, 0.0, 0.0, sc * le, 0.0, sc};
+        adj_approaching(P, adj_rows(G, A, q.k, q.i), e, dot<2>(e, e), sc, B.sc1[at], le, B.vr[at], T);
+        put(q, T);
+    };
+    walk_pairs<2, true, true>(P, G, stacks, [&](const uint2 w, bool active, auto near) {
+        bool go_on = false;
+        D3 e{0.0, 0.0, 0.0};
+        double vr = 0.0, sc = 0.0, sc1 = 0.0, le = 0.0;
+        if (active) {
+            const Pair q = pair_of(w, warp_first());
+            const D3 a = row<2>(G.pr, q.k), b = row<2>(G.pr, q.i);
+            e = {b.x - a.x, b.y - a.y, 0.0};
+            AdjTerms T{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            double y, dist;
+            if (adj_kernel<decltype(near)::value>(C, dot<2>(e, e), y, dist, sc, sc1)) {  // (as adj_terms)
+                const AdjRows R = adj_rows(G, A, q.k, q.i);
+                le = fma(R.lx, e.x, R.ly * e.y);
+                vr = -fma(R.dvx, e.x, R.dvy * e.y);
+                T.msc = sc;
+                T.p = sc * le;
+                const int32_t tk = G.itype[q.k], ti = G.itype[q.i];
+                const bool wall = lj_pair(P, tk, ti) && dist < C.lj_rr0;
+                const bool approaching = C.visc && __double2hiint(vr) < 0;
+                go_on = approaching && !wall;
+                if (!go_on) {
+                    if (approaching) adj_approaching(P, R, e, dot<2>(e, e), sc, sc1, le, vr, T);
+                    else adj_receding(R, e, sc, sc1, le, T);
+                    if (wall) adj_wall(C, R, tk, e, y, T);
+                }
+            }
+            if (!go_on) put(q, T);
+        }
+        const uint32_t who = __ballot_sync(0xFFFFFFFFu, go_on);
+        if (go_on) {
+            const uint32_t at = held + __popc(who & ((1u << lane) - 1u));
+            B.w[at] = w;
+            B.ex[at] = e.x;
+            B.ey[at] = e.y;
+            B.vr[at] = vr;
+            B.sc[at] = sc;
+            B.sc1[at] = sc1;
+            B.le[at] = le;
+        }
+        held += __popc(who);
+        __syncwarp();
+        if (held >= 32) {
+            held -= 32;
+            second(held + lane);
+            __syncwarp();
+        }
     });
+    if (lane < held) second(lane);
 }
 
 // The sums of those, and with them what k_adj_forces does per particle: v* = v +
