@@ -265,6 +265,13 @@ enum : int { kReuseFixed = 1, kReuseCell = 2 };
 constexpr uint32_t kCellEntryIndex = (1u << 27) - 1u;
 constexpr uint32_t kListOver = 0xFFFFFFFFu;
 constexpr int kGatherThreads = 128;     // default block size of the pair gathers
+// ... of the 3D reuse gathers: bound by L1, which the warps of a block share
+// (1.06M particles, us a step: 64 753, 128 717, 256 688)
+constexpr int kReuseThreads3 = 256;
+// ... of the stored-pair passes, whose warps meet nowhere: single warps, so that a
+// block ends with its longest one (us a step at 32 / 64 / 128: 43k delta-SPH 93.1 /
+// 96.9 / 98.7, 409k flume 476 / 479 / 480, 385k 3D 1988 / 1988 / 1993)
+constexpr int kPairThreads = 32;
 constexpr int kMaxGatherThreads = 256;
 
 }  // namespace rrsph

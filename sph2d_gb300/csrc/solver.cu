@@ -256,6 +256,11 @@ int key_bits(uint64_t max_cells) {
     return b < 1 ? 1 : b;
 }
 
+// The block size of the density (0) or force (1) gather.
+int block_size(const rrsph_solver* s, int gather, int own) {
+    return s->gather_threads[gather] ? s->gather_threads[gather] : own;
+}
+
 void drop_graphs(rrsph_solver* s) {
     cudaStreamSynchronize(s->stream);
     rrsph_impl::destroy_step_graphs(s);
@@ -310,7 +315,7 @@ void enqueue_grid(rrsph_solver* s, int predict, rrsph::StepScalars* scal, rrsph:
 
 template <int DIM>
 void enqueue_density(rrsph_solver* s, rrsph::StepScalars* scal) {
-    const int th = s->gather_threads[0];
+    const int th = block_size(s, 0, rrsph::kGatherThreads);
     if (s->precision == RRSPH_PRECISION_MIXED) rrsph::launch_density_mixed<DIM>(s->P, s->S, s->G, scal, s->flags, s->stream, th);
     else rrsph::launch_density_fp64<DIM>(s->P, s->S, s->G, scal, s->flags, s->stream, th);
     s->launches++;
@@ -318,7 +323,7 @@ void enqueue_density(rrsph_solver* s, rrsph::StepScalars* scal) {
 
 template <int DIM>
 void enqueue_forces(rrsph_solver* s, uint32_t terms, rrsph::StepScalars* scal, int write_mu, int use_masks = 0) {
-    const int th = s->gather_threads[1];
+    const int th = block_size(s, 1, rrsph::kGatherThreads);
     if (s->precision == RRSPH_PRECISION_MIXED)
         rrsph::launch_forces_mixed<DIM>(s->P, s->S, s->G, terms, scal, s->flags, write_mu, use_masks, s->stream, th);
     else rrsph::launch_forces_fp64<DIM>(s->P, s->S, s->G, terms, scal, s->flags, write_mu, s->stream, th, use_masks);
@@ -417,16 +422,16 @@ int enqueue_step_verlet(rrsph_solver* s, int par, cudaEvent_t* events, bool with
         cudaEventRecord(events[3], st);
     }
     const bool d3 = s->dim == 3;
-    if (d3) rrsph::launch_density_verlet<3>(s->P, s->S, s->G, cur, s->flags, st, s->gather_threads[0]);
-    else rrsph::launch_density_verlet<2>(s->P, s->S, s->G, cur, s->flags, st, s->gather_threads[0]);
+    if (d3) rrsph::launch_density_verlet<3>(s->P, s->S, s->G, cur, s->flags, st, block_size(s, 0, rrsph::kReuseThreads3));
+    else rrsph::launch_density_verlet<2>(s->P, s->S, s->G, cur, s->flags, st, block_size(s, 0, rrsph::kGatherThreads));
     if (s->mark_density) RRSPH_CUDA_TRY(cudaEventRecordWithFlags(s->ev_density, st, cudaEventRecordExternal));
     if (events) cudaEventRecord(events[4], st);
     // the whole step runs inside the force gather unless dt waits for the step's
     // maxima or a particle may have more neighbours than a list holds
     const bool fuse = !(s->P.dt_method == 2 && s->P.dt_reduce) &&
                       s->P.max_nb <= (uint32_t)rrsph::verlet_cap(s->dim) + 1u;
-    if (d3) rrsph::launch_forces_verlet<3>(s->P, s->S, s->G, cur, nxt, s->flags, st, s->gather_threads[1], fuse ? 1 : 0);
-    else rrsph::launch_forces_verlet<2>(s->P, s->S, s->G, cur, nxt, s->flags, st, s->gather_threads[1], fuse ? 1 : 0);
+    if (d3) rrsph::launch_forces_verlet<3>(s->P, s->S, s->G, cur, nxt, s->flags, st, block_size(s, 1, rrsph::kReuseThreads3), fuse ? 1 : 0);
+    else rrsph::launch_forces_verlet<2>(s->P, s->S, s->G, cur, nxt, s->flags, st, block_size(s, 1, rrsph::kGatherThreads), fuse ? 1 : 0);
     if (events) cudaEventRecord(events[5], st);
     if (!fuse) {
         const bool pistons = s->P.vl_split > 1;  // the split density gather's
@@ -474,7 +479,7 @@ void enqueue_step(rrsph_solver* s, int par, cudaEvent_t* events, bool with_keys)
     if (events) cudaEventRecord(events[3], s->stream);
     if (s->pairs64) {
         rrsph::launch_pair_masks<DIM>(s->P, s->S, s->G, cur, s->stream);
-        rrsph::launch_pair_terms<DIM>(s->P, s->G, s->stream, s->gather_threads[0]);
+        rrsph::launch_pair_terms<DIM>(s->P, s->G, s->stream, block_size(s, 0, rrsph::kPairThreads));
         if (!cont) rrsph::launch_pair_density<DIM>(s->P, s->S, s->G, cur, s->flags, s->stream);
         s->launches += cont ? 2 : 3;
     } else {
@@ -483,7 +488,7 @@ void enqueue_step(rrsph_solver* s, int par, cudaEvent_t* events, bool with_keys)
     if (s->mark_density) cudaEventRecordWithFlags(s->ev_density, s->stream, cudaEventRecordExternal);
     if (events) cudaEventRecord(events[4], s->stream);
     if (s->pairs64) {
-        if (!cont) rrsph::launch_pair_forces<DIM>(s->P, s->G, s->stream, s->gather_threads[1]);
+        if (!cont) rrsph::launch_pair_forces<DIM>(s->P, s->G, s->stream, block_size(s, 1, rrsph::kPairThreads));
         rrsph::launch_pair_sum<DIM>(s->P, s->S, s->G, cur, s->flags, s->stream);
         s->launches += cont ? 1 : 2;
     } else {

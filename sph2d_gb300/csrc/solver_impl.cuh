@@ -74,7 +74,7 @@ struct rrsph_solver {
     double phase_ms[kPhases] = {};
     uint64_t timed_steps = 0;
     rrsph_impl::AdjointRun* adj = nullptr;
-    int gather_threads[2] = {rrsph::kGatherThreads, rrsph::kGatherThreads};  // density, forces block sizes
+    int gather_threads[2] = {0, 0};  // block sizes of the density and force gathers, 0: the kernels' own
     bool pairs64 = false;  // the loop's FP64 step evaluates each pair once (kernels_pairs64.cu)
     // neighbour reuse of the FP32-mixed step
     bool verlet = false;

@@ -123,3 +123,21 @@ def test_coincident_absent_and_outside_particles(gpu_available, dim, treatment):
             c.r[first + j] = c.r[20]
             c.r[first + j, 0] = p.x_mingeom - (cells + 0.21 * j) * cell
     _check(p, c, treatment)
+
+
+@pytest.mark.parametrize("dim,treatment", [(2, 0), (2, 1), (3, 1)])
+def test_block_sizes_give_the_same_bits(gpu_available, dim, treatment):
+    from sph2d_gb300 import Solver
+
+    c = _scene(dim, treatment, 1.3, 23, 11)
+    out = []
+    for threads in (None, 64, 128, 256):
+        with Solver(c.params(), "fp64") as s:
+            if threads:
+                s.set_gather_threads(threads, threads)
+            s.upload(c.r, c.v, c.rho, c.itype)
+            s.step(3)
+            out.append(s.download())
+    for o in out[1:]:
+        for k in ("r", "v", "rho", "p"):
+            assert np.array_equal(o[k], out[0][k]), k
