@@ -501,14 +501,14 @@ __device__ __forceinline__ AdjTerms adj_terms_any(const DevParams& P, const Sort
 // in k_adj_forces. As in the forward step's forces, the approaching pairs go on
 // to a second stack of the warp, so that receding ones do not pay for them: 205k
 // particles 355 -> 279 us, 42k (their stacks drain half full) 50 reverse steps 16.5
-// -> 15.7 ms; k_adj_forces took 260 us a step on 42k.
+// -> 15.7 ms, and 15.2 in blocks of one warp; k_adj_forces took 260 us a step on 42k.
 struct AdjApproach {  // a warp's second stack
     uint2 w[kStack];
     double ex[kStack], ey[kStack], vr[kStack], sc[kStack], sc1[kStack], le[kStack];
 };
-__global__ void __launch_bounds__(128) k_adj_pair_forces(DevParams P, Sorted G, AdjBuf A) {
-    __shared__ uint2 stacks[4 * 2 * kStack];
-    __shared__ AdjApproach second_stacks[4];
+__global__ void __launch_bounds__(kPairThreads) k_adj_pair_forces(DevParams P, Sorted G, AdjBuf A) {
+    __shared__ uint2 stacks[kPairThreads / 32 * 2 * kStack];
+    __shared__ AdjApproach second_stacks[kPairThreads / 32];
     AdjApproach& B = second_stacks[threadIdx.x >> 5];
     const PairConst& C = P.pc;
     const uint32_t cap = C.cap, lane = threadIdx.x & 31u;
@@ -636,8 +636,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_pair_sum(DevParams P, Sorte
 }
 
 // Adjoint of density_sum, each pair once: (λrho_k + λrho_i) m sc e.
-__global__ void __launch_bounds__(128) k_adj_pair_density(DevParams P, Sorted G, AdjBuf A) {
-    __shared__ uint2 stacks[4 * kStack];
+__global__ void __launch_bounds__(kPairThreads) k_adj_pair_density(DevParams P, Sorted G, AdjBuf A) {
+    __shared__ uint2 stacks[kPairThreads / 32 * kStack];
     const uint32_t cap = P.pc.cap;
     const size_t n = P.n;
     walk_pairs<2, false, true>(P, G, stacks, [&](const uint2 w, bool active, auto) {
@@ -898,12 +898,12 @@ void enqueue_reverse_step(rrsph_solver* s, AdjointRun* run, uint64_t m, size_t j
     const unsigned blocks = (unsigned)((n + 255) / 256);
     const unsigned gblocks = (unsigned)((n + rrsph::kAdjThreads - 1) / rrsph::kAdjThreads);
     if (run->rec) {
-        const dim3 pblocks((unsigned)((n + 127) / 128), rrsph::pair_slices((uint32_t)n));
+        const dim3 pblocks((unsigned)((n + rrsph::kPairThreads - 1) / rrsph::kPairThreads), rrsph::pair_slices((uint32_t)n));
         rrsph::k_adj_pair_reorder<<<blocks, 256, 0, st>>>(s->P, G, sv, run->seg_rho + j * n, A, run->dt, v_dt, piston);
         rrsph::launch_pair_masks<2>(s->P, s->S, G, s->scal, st);
-        rrsph::k_adj_pair_forces<<<pblocks, 128, 0, st>>>(s->P, G, A);
+        rrsph::k_adj_pair_forces<<<pblocks, rrsph::kPairThreads, 0, st>>>(s->P, G, A);
         rrsph::k_adj_pair_sum<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A, run->dt);
-        rrsph::k_adj_pair_density<<<pblocks, 128, 0, st>>>(s->P, G, A);
+        rrsph::k_adj_pair_density<<<pblocks, rrsph::kPairThreads, 0, st>>>(s->P, G, A);
         rrsph::k_adj_pair_density_sum<<<gblocks, rrsph::kAdjThreads, 0, st>>>(s->P, G, A);
         s->launches += 7;
     } else {
