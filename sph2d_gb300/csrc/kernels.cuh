@@ -32,8 +32,8 @@ struct State {
     int2* fix2;                // 2D: fixed-point position (Pos)
     int4* fix4;                // 3D: the same (x, y, z)
     int2* bfix2;               // 2D: the same at the last list build
-    int4* bfix4;               // 3D
-    uint32_t* bcxy;            // kReuseCell: cell coordinates at the last list build, x | y << 16
+    int4* bfix4;               // 3D; .w: its cell coordinates, x | y << 10 | z << 20
+    uint32_t* bcxy;            // 2D: cell coordinates at the last list build, x | y << 16
     float2* boff;              // kReuseCell: offset from that cell's edges at the last list build
     uint32_t* slot;            // cell-order index at the last list build
     uint32_t* vl_far;          // non-zero: some particle is outside the grid (CellSplit::far); [1]: at the last rebuild

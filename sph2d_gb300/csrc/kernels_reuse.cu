@@ -190,11 +190,12 @@ __global__ void __launch_bounds__(kVlBuildThreads) k_vl_build(DevParams P, State
         cx = third_bits(key);
         cy = third_bits(key >> 1);
         cz = third_bits(key >> 2);
-        S.bfix4[id] = make_int4(pj.x, pj.y, pj.z, 0);
+        S.bfix4[id] = make_int4(pj.x, pj.y, pj.z, (int)(cx | cy << 10 | cz << 20));
     } else {
         cx = second_bits(key);
         cy = second_bits(key >> 1);
         S.bfix2[id] = make_int2(pj.x, pj.y);
+        S.bcxy[id] = cx | cy << 16;
     }
     S.slot[id] = k;
     uint4* const slab = reinterpret_cast<uint4*>(G.vlist) + k;  // group g at slab[g * n]
@@ -563,6 +564,7 @@ __device__ __forceinline__ void fetch_whole(const State& S, uint32_t id) {
         fetch_l1(S.bfix4 + id);
     } else {
         fetch_l1(S.bfix2 + id);
+        fetch_l1(S.bcxy + id);
     }
     fetch_l1(S.itype + id);
     fetch_l1(S.key_of + id);

@@ -619,7 +619,7 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
             if (d3) {
                 A(S.fix4, n); A(S.bfix4, n);
             } else if (rrsph::verlet_split(2, (uint32_t)n) == 1) {
-                A(S.fix2, n); A(S.bfix2, n);
+                A(S.fix2, n); A(S.bfix2, n); A(S.bcxy, n);
             } else {  // kReuseCell
                 A(S.bcxy, n); A(S.boff, n);
             }

@@ -83,14 +83,20 @@ __device__ __forceinline__ void reuse_cell_pass(const DevParams& P, const State&
 }
 
 // Neighbour reuse, in the key pass of particle i at fixed-point position (x, y,
-// z): the next step's cell-order copies at the particle's slot of the last build (a
-// step that rebuilds overwrites them in its new order), the position for the next
-// build, and the test whether the particle has moved too far since the last. With
-// continuity density V4.w is rho_predict and VD4 = (v, rho - rho0), as the reorder
-// writes them. A particle outside the grid is searched on a fresh grid each step.
+// z) in cell (cx, cy, cz): the next step's cell-order copies at the particle's slot of
+// the last build (a step that rebuilds overwrites them in its new order), the position
+// for the next build, and the test whether the particle has moved too far since the
+// last: its separation in fixed point, which repeats every 32 cells, and its cell,
+// which an upload may have changed by any number of them. With continuity density V4.w
+// is rho_predict and VD4 = (v, rho - rho0), as the reorder writes them. A particle
+// outside the grid is searched on a fresh grid each step.
 template <int DIM>
 __device__ __forceinline__ void reuse_pass(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
-                                           uint32_t x, uint32_t y, uint32_t z, bool far) {
+                                           uint32_t x, uint32_t y, uint32_t z, uint32_t cx, uint32_t cy, uint32_t cz,
+                                           bool far) {
+    // within 16 cells of the cell at the build, where the separation is the only one
+    auto near_cell = [](uint32_t c, uint32_t at_build) { return c - at_build + 16u <= 32u; };
+    bool near;
     const uint32_t k = S.slot[i];
     G.posn[k] = Pos{(int)x, (int)y, (int)z, Pos::code_of(S.itype[i], P.type_non_existent, far)};
     velocity_copies<DIM>(P, S, G, i, k);
@@ -101,14 +107,18 @@ __device__ __forceinline__ void reuse_pass(const DevParams& P, const State& S, c
         const float dx = (float)(int)(x - (uint32_t)b.x) * P.rf.u, dy = (float)(int)(y - (uint32_t)b.y) * P.rf.u,
                     dz = (float)(int)(z - (uint32_t)b.z) * P.rf.u;
         d2 = dx * dx + dy * dy + dz * dz;
+        near = near_cell(cx, (uint32_t)b.w & 0x3FFu) && near_cell(cy, (uint32_t)b.w >> 10 & 0x3FFu) &&
+               near_cell(cz, (uint32_t)b.w >> 20);
     } else {
         const int2 b = S.bfix2[i];
         S.fix2[i] = make_int2((int)x, (int)y);
+        const uint32_t bc = S.bcxy[i];
         const float dx = (float)(int)(x - (uint32_t)b.x) * P.rf.u, dy = (float)(int)(y - (uint32_t)b.y) * P.rf.u;
         d2 = dx * dx + dy * dy;
+        near = near_cell(cx, bc & 0xFFFFu) && near_cell(cy, bc >> 16);
     }
     if (far) *S.vl_far = 1u;
-    reuse_check(S, far || d2 > P.vl_half_skin2);
+    reuse_check(S, far || !near || d2 > P.vl_half_skin2);
 }
 
 template <int DIM, int M>
@@ -139,7 +149,8 @@ __device__ __forceinline__ void key_pass(const DevParams& P, const State& S, con
     G.keys_in[i] = (uint32_t)key;
     G.ids_in[i] = i;
     if (M != 0 && P.reuse == kReuseFixed)
-        reuse_pass<DIM>(P, S, G, i, sx.fix, sy.fix, sz.fix, sx.far || sy.far || (DIM == 3 && sz.far));
+        reuse_pass<DIM>(P, S, G, i, sx.fix, sy.fix, sz.fix, (uint32_t)sx.c & cmax, (uint32_t)sy.c & cmax,
+                        (uint32_t)sz.c & cmax, sx.far || sy.far || (DIM == 3 && sz.far));
     if (M == 1 && P.reuse == kReuseFixed) return;  // the loop's next grid is the reuse step's
     if (M == 0 && !(DIM == 3 ? (void*)S.coff4 : (void*)S.coff2)) return;
     // offsets from the edge of the cell the key names: the Morton code keeps 16
