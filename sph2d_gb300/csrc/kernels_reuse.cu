@@ -88,15 +88,23 @@ __device__ __noinline__ bool exact_pair(const DevParams& P, const State& S, uint
     return exact_dist2<DIM>(dx, dy, dz) < P.cut2;
 }
 // The stencil search's test of particle i (sorted) against k: an absent one never,
-// one outside the grid in double.
+// in double one outside the grid and those of a cell that the stencil meets by
+// wrapping (the 3D key of coordinate 1024 is that of 0, 1024 cells away, where fixed
+// point repeats).
 template <int DIM>
 __device__ __forceinline__ bool searched_pair(const DevParams& P, const State& S, const Sorted& G, uint32_t i,
-                                              uint32_t k, const Pos& pi, const Pos& pk) {
+                                              uint32_t k, const Pos& pi, const Pos& pk, bool wraps) {
     if (pi.absent()) return false;
-    if (pi.unlisted() || pk.unlisted()) return exact_pair<DIM>(P, S, G.id[i], G.id[k]);
+    if (wraps || pi.unlisted() || pk.unlisted()) return exact_pair<DIM>(P, S, G.id[i], G.id[k]);
     const float d2 = distance2<DIM>(separation<DIM>(pi, pk, P.rf.u), pi.code);
     if (d2 < P.mf.cut2_lo) return true;
     return d2 < P.mf.cut2_hi && exact_pair<DIM>(P, S, G.id[i], G.id[k]);
+}
+
+// Whether a stencil cell with these offsets is met by wrapping.
+template <int DIM>
+__device__ __forceinline__ bool wrapped(int sx, int sy, int sz) {
+    return DIM == 3 && (sx < -1 || sy < -1 || sz < -1);
 }
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -440,11 +448,12 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_verlet(DevParams 
                 const uint32_t s = G.cell_start[cell];
                 if (s == kEmpty) continue;
                 const uint32_t e = G.cell_end[cell];
+                const bool wraps = wrapped<DIM>(sx, sy, sz);
                 float part = 0.0f;
                 for (uint32_t i = s; i < e; i++) {
                     if (i == k) continue;
                     const Pos pi = G.pos[i];
-                    if (!searched_pair<DIM>(P, S, G, i, k, pi, pj)) continue;
+                    if (!searched_pair<DIM>(P, S, G, i, k, pi, pj, wraps)) continue;
                     if (cnt < (uint32_t)CAP) list[(size_t)(cnt >> 2) * 4 * P.n + (cnt & 3u)] = i;
                     cnt++;
                     const float4 vdi = CONT ? G.VD4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -678,11 +687,12 @@ __global__ void __launch_bounds__(L > 1 ? 32 * L : kMaxGatherThreads, 4) k_force
                     const uint32_t s = G.cell_start[cell];
                     if (s == kEmpty) continue;
                     const uint32_t e = G.cell_end[cell];
+                    const bool wraps = wrapped<DIM>(sx, sy, sz);
 #pragma unroll 1
                     for (uint32_t i = s; i < e; i++) {
                         if (i == k) continue;
                         const Pos pi = G.pos[i];
-                        if (!searched_pair<DIM>(P, S, G, i, k, pi, pj)) continue;
+                        if (!searched_pair<DIM>(P, S, G, i, k, pi, pj, wraps)) continue;
                         one(G.V4[i], G.PR[i], pi);
                     }
                 }

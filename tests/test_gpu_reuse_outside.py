@@ -1,0 +1,67 @@
+"""The FP32-mixed step with neighbour reuse on fixed-point positions where their
+repetition every 32 cells, or the edge of what a key holds, could show: against the
+step without reuse (cell-relative positions), with the bars of the mixed step
+against the FP64 oracle (test_gpu_parity.py)."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(p, r, v, rho, itype, steps, reuse):
+    from sph2d_gb300 import Solver
+
+    pairs, t = [], 0.0
+    with Solver(p, "mixed") as s:
+        s.set_neighbour_reuse(reuse)
+        s.upload(r, v, rho, itype)
+        for _ in range(steps):
+            t = s.step(1, t)
+            pairs.append(s.pair_count()[0])
+        return s.download() | s.download_rates(), pairs
+
+
+def _same(p, c, steps=2):
+    a, pa = _run(p, c.r, c.v, c.rho, c.itype, steps, True)
+    b, pb = _run(p, c.r, c.v, c.rho, c.itype, steps, False)
+    assert pa == pb
+    assert np.array_equal(a["itype"], b["itype"])
+    for k, bar in (("r", 1e-8), ("v", 1e-4), ("rho", 1e-6), ("p", 1e-3)):
+        x, y = a[k], b[k]
+        assert np.array_equal(np.isnan(x), np.isnan(y)), k
+        assert rel_l2(np.nan_to_num(x), np.nan_to_num(y)) < bar, (k, rel_l2(np.nan_to_num(x), np.nan_to_num(y)))
+
+
+def _at_the_last_key(crowd, near, extent, max_neighbours):
+    """`crowd` fluid particles in a half ball at the far side of the last cell along x
+    whose coordinate a 3D key holds (1023), and `near` others in the first cell, on
+    the same y and z: the stencil of cell 1023 ends in cell 0."""
+    from sph2d_gb300 import cases
+
+    c = cases.dam_break_3d(dx=0.1, tank=(0.5, 0.5, 0.5), block=(0.4, 0.5, 0.3))
+    c.model["intf_hsml_coef"] = 1.0
+    c.model["max_neighbours"] = max_neighbours
+    rng = np.random.default_rng(crowd)
+    n = crowd + near
+    geom = {"x_mingeom": 0.0, "x_maxgeom": 1023.9, "y_mingeom": 0.0, "y_maxgeom": 4.0, "z_mingeom": 0.0, "z_maxgeom": 4.0}
+    c.particle.update(geom, delta=0.5, ntotal=n, nfluid=n, nvirt=0)  # cells of 1
+    d = rng.standard_normal((crowd, 3))
+    d *= (extent * rng.uniform(0.0, 1.0, (crowd, 1)) ** (1 / 3)) / np.linalg.norm(d, axis=1, keepdims=True)
+    d[:, 0] = -np.abs(d[:, 0])
+    c.r = np.concatenate([np.array([1023.85, 1.5, 1.5]) + d,
+                          np.array([0.05, 1.0, 1.0]) + rng.uniform(0.0, 0.9, (near, 3)) * np.array([0.3, 1.0, 1.0])])
+    c.v = rng.standard_normal((n, 3)) * 0.01
+    c.rho = np.full(n, 1000.0)
+    c.itype = np.full(n, 2, dtype=np.int32)
+    return c
+
+
+# 299 candidates within cutoff and skin: searched. Within 0.49 all of them are neighbours; within 1.18
+# at most 256 are, and the whole step runs in the force gather
+@pytest.mark.parametrize("crowd,extent,max_neighbours", [(300, 0.49, 1000), (300, 1.18, 257)])
+def test_stencil_of_the_last_key(gpu_available, crowd, extent, max_neighbours):
+    c = _at_the_last_key(crowd, 40, extent, max_neighbours)
+    _same(c.params(), c, steps=1)
