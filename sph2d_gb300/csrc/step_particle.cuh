@@ -98,7 +98,9 @@ __device__ __forceinline__ void reuse_pass(const DevParams& P, const State& S, c
     auto near_cell = [](uint32_t c, uint32_t at_build) { return c - at_build + 16u <= 32u; };
     bool near;
     const uint32_t k = S.slot[i];
-    G.posn[k] = Pos{(int)x, (int)y, (int)z, Pos::code_of(S.itype[i], P.type_non_existent, far)};
+    const int32_t type = S.itype[i];
+    far = far && type != P.type_non_existent;  // an absent one is nobody's neighbour wherever it lies
+    G.posn[k] = Pos{(int)x, (int)y, (int)z, Pos::code_of(type, P.type_non_existent, far)};
     velocity_copies<DIM>(P, S, G, i, k);
     float d2;
     if (DIM == 3) {

@@ -65,3 +65,28 @@ def _at_the_last_key(crowd, near, extent, max_neighbours):
 def test_stencil_of_the_last_key(gpu_available, crowd, extent, max_neighbours):
     c = _at_the_last_key(crowd, 40, extent, max_neighbours)
     _same(c.params(), c, steps=1)
+
+
+@pytest.mark.parametrize("name", ["2d", "3d_split"])
+def test_absent_particles_far_outside_ask_for_no_rebuild(gpu_available, name):
+    """Non-existent particles parked far below the geometry are nobody's neighbours:
+    the lists of the others hold as long as without them."""
+    from test_gpu_moved_uploads import _scene
+
+    from sph2d_gb300 import Solver
+
+    builds = []
+    for parked in (False, True):
+        c = _scene(name)
+        c.model["consistency_check"] = False
+        c.model["consistency_treatment"] = 0
+        p = c.params()
+        c.itype[:40] = 0
+        if parked:
+            c.r[:40, 0] = p.x_mingeom - 100.0 * p.hsml
+            c.r[20:40, 1] = p.y_mingeom - 1e6
+        with Solver(p, "mixed") as s:
+            s.upload(c.r, c.v, c.rho, c.itype)
+            s.step(6)
+            builds.append(s.neighbour_rebuilds())
+    assert builds[0] == builds[1] == 1
