@@ -112,16 +112,16 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// The cubic spline: W / f with q = |r| / h ...
+// The cubic spline, zero beyond q = 2 (cells may be wider): W / f with q = |r| / h ...
 __device__ __forceinline__ float cubic_w(float q) {
-    const float t = 2.0f - q;
+    const float t = fmaxf(2.0f - q, 0.0f);
     const float far = (1.0f / 6.0f) * (t * (t * t));
     const float near = fmaf(q * q, fmaf(0.5f, q, -1.0f), 2.0f / 3.0f);
     return q <= 1.0f ? near : far;
 }
 // ... and s with dW/dr = diff s f / (2 h^2) (rs: 1 / distance).
 __device__ __forceinline__ float cubic_s(const ReuseF& U, float q, float rs) {
-    const float t = 2.0f - q;
+    const float t = fmaxf(2.0f - q, 0.0f);
     const float far = -(rs * U.far) * (t * t);
     const float near = fmaf(3.0f, q, -4.0f);
     return q <= 1.0f ? near : far;

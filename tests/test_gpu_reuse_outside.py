@@ -90,3 +90,20 @@ def test_absent_particles_far_outside_ask_for_no_rebuild(gpu_available, name):
             s.step(6)
             builds.append(s.neighbour_rebuilds())
     assert builds[0] == builds[1] == 1
+
+
+@pytest.mark.parametrize("dim,treatment", [(2, 0), (2, 1), (3, 0), (3, 1)])
+def test_cells_wider_than_the_cubic_kernel(gpu_available, dim, treatment):
+    """cell_scale_k above 2 with cubic kernels: pairs beyond 2h are neighbours (and
+    counted) whose kernel is zero."""
+    from sph2d_gb300 import cases
+
+    if dim == 2:
+        c = cases.dam_break_2d(seed=2, nx=300, ny=150, dx=0.02, tank=(6.6, 3.4), density_treatment=treatment)
+    else:
+        c = cases.dam_break_3d(dx=0.02, tank=(0.5, 0.2, 0.3), block=(0.3, 0.2, 0.2), density_treatment=treatment)
+    c.model["max_neighbours"] = 700
+    c.v = np.random.default_rng(dim).standard_normal(c.v.shape) * 0.3
+    p = c.params()
+    p.cell_scale_k = 2.6
+    _same(p, c)
