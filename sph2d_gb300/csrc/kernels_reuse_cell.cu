@@ -196,7 +196,10 @@ __device__ __forceinline__ float density_term(const MixedF& M, int skf, float f,
                                               float4 vdi, float4 vdj, bool delta) {
     const float inv_dist = rsqrtf(d2);
     const float q = d2 * inv_dist * M.inv_h;
-    if (!CONT) return SKF == 1 ? cubic_wf_sel(f, q) : kernel_wf(skf, f, q);
+    if (!CONT) {
+        const float qw = fmaxf(q, 0.0f);  // (of coincident particles NaN: W(0))
+        return SKF == 1 ? cubic_wf_sel(f, qw) : kernel_wf(skf, f, qw);
+    }
     const float sc = SKF == 1 ? cubic_dwdr_sel(f, q, inv_dist, M.inv_h)
                               : kernel_dwdr_scalef(skf, f, q, inv_dist, M.inv_h);
     float vcc = (vdi.x - vdj.x) * dx + (vdi.y - vdj.y) * dy;

@@ -107,3 +107,30 @@ def test_cells_wider_than_the_cubic_kernel(gpu_available, dim, treatment):
     p = c.params()
     p.cell_scale_k = 2.6
     _same(p, c)
+
+
+@pytest.mark.parametrize("name,reuse", [("2d", True), ("2d_small", True), ("2d_small", False), ("3d_split", True),
+                                         ("3d_split", False)])
+def test_coincident_particles_count_each_other(gpu_available, name, reuse):
+    """Summation density of two particles on one point holds W(0) twice, as in FP64,
+    for any number of particles and with and without reuse."""
+    from test_gpu_moved_uploads import _scene
+
+    from sph2d_gb300 import Solver
+
+    c = _scene(name)
+    c.model["density_treatment"] = 0
+    first = np.arange(3, 1203, 12)  # (many: cell-relative separations of some are exactly zero)
+    c.r[first] = c.r[first + 1]
+    p = c.params()
+    rho = []
+    for precision in ("fp64", "mixed"):
+        with Solver(p, precision) as s:
+            if precision == "mixed":
+                s.set_neighbour_reuse(reuse)
+            s.upload(c.r, c.v, c.rho, c.itype)
+            s.step(1)
+            rho.append(s.download()["rho"])
+    assert rel_l2(rho[1], rho[0]) < 1e-6
+    both = np.concatenate([first, first + 1])
+    assert np.all(np.abs(rho[1][both] / rho[0][both] - 1.0) < 1e-6)
