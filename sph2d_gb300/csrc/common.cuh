@@ -366,7 +366,8 @@ __device__ inline double kernel_dwdr_scale(int skf, double f, double q, double d
 // correctly rounded quotient (Markstein).
 __device__ inline double eos_p(const DevParams& P, double rho) {
     const double x0 = rho * P.inv_rho0;
-    const double x = fma(fma(-x0, P.rho0, rho), P.inv_rho0, x0);
+    double x = fma(fma(-x0, P.rho0, rho), P.inv_rho0, x0);
+    if ((__double2hiint(x0) & 0x7FF00000) == 0x7FF00000) x = x0;  // infinite: the residual is not a number
     const double x2 = x * x;
     const double x4 = x2 * x2;
     return P.B * (x4 * x2 * x - 1.0);

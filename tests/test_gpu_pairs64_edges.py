@@ -1,0 +1,54 @@
+"""The stored-pair FP64 step where the values, not the bookkeeping, are special,
+against the directed gathers behind rrsph_density / rrsph_forces."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(dim, treatment, bulk=0.0):
+    from sph2d_gb300 import cases
+
+    if dim == 2:
+        c = cases.dam_break_2d(seed=3, nx=24, ny=13, dx=0.02, tank=(1.0, 0.6), density_treatment=min(treatment, 1))
+    else:
+        c = cases.dam_break_3d(seed=3, dx=0.02, tank=(0.5, 0.2, 0.3), block=(0.16, 0.2, 0.12),
+                               density_treatment=min(treatment, 1))
+    c.model["max_neighbours"] = 700
+    c.model["artificial_bulk_visc"] = bulk
+    if treatment == 2:
+        c.model["density_treatment"] = 2
+        c.model["density_delta_sph_coef"] = 0.1
+    c.v = np.random.default_rng(1).standard_normal(c.v.shape) * 0.3
+    return c
+
+
+def _both(c, treatment):
+    """(density or rate, pressure, accelerations) of the first step, and of the loop pieces."""
+    from sph2d_gb300 import Solver
+
+    p = c.params()
+    with Solver(p, "fp64") as s:
+        s.upload(c.r, c.v, c.rho, c.itype)
+        s.step_async(1)
+        s.status()  # (waits; a step that throws particles out may raise at sync)
+        st = s.download() | s.download_rates()
+    with Solver(p, "fp64") as s:
+        s.upload(c.r, c.v, c.rho, c.itype)
+        d, pres = s.density()
+        a = s.forces()[0]
+    return (st["rho" if treatment == 0 else "drho"], st["p"], st["a"]), (d, pres, a)
+
+
+@pytest.mark.parametrize("treatment", [1, 2])
+@pytest.mark.parametrize("rho,p", [(np.inf, np.inf), (-np.inf, -np.inf), (np.nan, np.nan)])
+def test_pressure_of_a_density_that_is_no_number(gpu_available, treatment, rho, p):
+    """B ((rho / rho0)^7 - 1) of the first step and of the loop piece."""
+    c = _scene(2, treatment)
+    c.rho[100] = rho
+    for x in _both(c, treatment):
+        assert np.array_equal(x[1][100], p, equal_nan=True)
+        assert np.all(np.isfinite(np.delete(x[1], 100)))
