@@ -484,7 +484,7 @@ __device__ __forceinline__ AdjTerms adj_terms(const DevParams& P, const Sorted& 
     const double le = fma(R.lx, e.x, R.ly * e.y), vr = -fma(R.dvx, e.x, R.dvy * e.y);
     T.msc = sc;
     T.p = sc * le;
-    if (C.visc && __double2hiint(vr) < 0) adj_approaching(P, R, e, s2, sc, sc1, le, vr, T);
+    if (C.visc && negative(vr)) adj_approaching(P, R, e, s2, sc, sc1, le, vr, T);
     else adj_receding(R, e, sc, sc1, le, T);
     const int32_t tk = G.itype[k], ti = G.itype[i];
     if (lj_pair(P, tk, ti) && dist < C.lj_rr0) adj_wall(C, R, tk, e, y, T);
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kPairThreads) k_adj_pair_forces(DevParams P, S
                 T.p = sc * le;
                 const int32_t tk = G.itype[q.k], ti = G.itype[q.i];
                 const bool wall = lj_pair(P, tk, ti) && dist < C.lj_rr0;
-                const bool approaching = C.visc && __double2hiint(vr) < 0;
+                const bool approaching = C.visc && negative(vr);
                 go_on = approaching && !wall;
                 if (!go_on) {
                     if (approaching) adj_approaching(P, R, e, dot<2>(e, e), sc, sc1, le, vr, T);

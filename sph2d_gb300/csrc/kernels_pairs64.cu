@@ -160,15 +160,24 @@ __global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_mas
     }
 }
 
+// The viscous part in the IEEE forms of the directed gathers, for what the seeds do
+// not take (infinite velocities and densities, densities that sum to zero).
+__device__ __noinline__ double visc_ieee(double h, double alpha_c, double beta, double vr, double sep, double rhos) {
+    const double mu = h * vr / sep;
+    return (beta * mu - alpha_c) * mu / (0.5 * rhos);
+}
 // The viscous part of the coefficient (artificial_viscosity_part,
 // ArtificialViscosity.h:29-65) added to pf: Pi_ij for an approaching pair, with
 // one quotient for its two divisions. vr = (v_j - v_i).(r_j - r_i).
-__device__ __forceinline__ double add_visc(const PairConst& C, double pf, double vr, double d2, double rhos) {
-    if (__double2hiint(vr) >= 0) return pf;
-    const double x = (d2 + C.etq_h2) * rhos;
+__device__ __forceinline__ double add_visc(const DevParams& P, double pf, double vr, double d2, double rhos) {
+    if (!negative(vr)) return pf;
+    const PairConst& C = P.pc;
+    const double sep = d2 + C.etq_h2;
+    const double x = sep * rhos;
     const double r = inverse_40(x);
     const double e = fma(-x, r, 1.0);
     const double u = vr * r;
+    if (no_number(u)) return pf + visc_ieee(P.h, P.av_alpha * P.c_av, P.av_beta, vr, sep, rhos);
     const double w = fma(u, e, u);
     double f = C.av_c;  // -2 h alpha c; 2 h (beta mu - alpha c) with a bulk term
     if (C.bulk) f = fma(C.av_beta2h, C.h * rhos * w, f);
@@ -194,7 +203,7 @@ __device__ __forceinline__ void force_coefs(const DevParams& P, const PairConst&
     double pf = prk + pri;
     if (C.visc) {
         const double vr = dot<DIM>({vi.x - vk.x, vi.y - vk.y, DIM == 3 ? vi.z - vk.z : 0.0}, d);
-        pf = add_visc(C, pf, vr, d2, rhok + rhoi);
+        pf = add_visc(P, pf, vr, d2, rhok + rhoi);
     }
     ck = ci = s * pf;
     if (lj_pair(P, tk, ti)) {
@@ -330,7 +339,7 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_pair_forces(DevParams P, 
             ri = rank_of<DIM>(P, G, i, q.c, q.bit);
         }
         double pf = prk + pri;
-        if (C.visc) pf = add_visc(C, pf, vr, d2, rhok + rhoi);
+        if (C.visc) pf = add_visc(P, pf, vr, d2, rhok + rhoi);
         double ck = s * pf, ci = ck;
         const bool lj = lj_pair(P, tk, ti);
         if (lj) {
@@ -355,7 +364,7 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_pair_forces(DevParams P, 
             go_on = q.order >= cap || lj_pair(P, G.itype[k], G.itype[i]);
             if (C.visc) {
                 vr = dot<DIM>({vb.x - va.x, vb.y - va.y, DIM == 3 ? vb.z - va.z : 0.0}, d);
-                go_on = go_on || __double2hiint(vr) < 0;
+                go_on = go_on || negative(vr);
             }
             if (!go_on) {
                 const size_t ao = q.order * n + k;

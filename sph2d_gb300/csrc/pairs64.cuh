@@ -142,6 +142,12 @@ __device__ __forceinline__ double inverse_40(double x) {
     e = fmaf(-ml, z, e);
     return step_mantissa(y, z, fmaf(e, e, e));
 }
+// Infinite or not a number.
+__device__ __forceinline__ bool no_number(double x) { return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000; }
+// Below zero; a NaN of either sign is not (the machine's own has the sign bit set).
+__device__ __forceinline__ bool negative(double x) {
+    return (uint32_t)__double2hiint(x) - 0x80000000u <= 0x7FF00000u;
+}
 // Half of a normal double, by its exponent.
 __device__ __forceinline__ double half_of(double x) {
     return __hiloint2double(__double2hiint(x) - 0x00100000, __double2loint(x));

@@ -52,3 +52,29 @@ def test_pressure_of_a_density_that_is_no_number(gpu_available, treatment, rho, 
     for x in _both(c, treatment):
         assert np.array_equal(x[1][100], p, equal_nan=True)
         assert np.all(np.isfinite(np.delete(x[1], 100)))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("treatment", [0, 1, 2])
+@pytest.mark.parametrize("bulk", [0.0, 0.1])
+@pytest.mark.parametrize("what", ["v=nan", "v=-nan", "v=inf", "v=-inf", "v=1e200", "rho=nan", "rho=inf", "rho=-1000"])
+def test_one_particle_that_is_no_number(gpu_available, dim, treatment, bulk, what):
+    """A velocity or density that is not a number (of either sign: the GPU's own is
+    negative), infinite or huge: the same entries of the neighbours' sums are NaN,
+    +inf, -inf or finite, and the finite ones equal."""
+    name, value = what.split("=")
+    if name == "rho" and treatment == 0:
+        pytest.skip("summation density reads none")
+    c = _scene(dim, treatment, bulk)
+    x = np.copysign(np.nan, -1.0) if value == "-nan" else float(value)
+    if name == "v":
+        c.v[100, 0] = x
+    else:
+        c.rho[100] = x
+    for got, want in zip(*_both(c, treatment)):
+        for kind in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(kind(got), kind(want))
+        ok = np.isfinite(want) & (np.abs(want) < 1e100)
+        assert rel_l2(got[ok], want[ok]) < 1e-11
+        big = np.isfinite(want) & ~ok
+        assert np.all(np.abs(got[big] / want[big] - 1.0) < 1e-11)
