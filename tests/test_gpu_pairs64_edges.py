@@ -78,3 +78,18 @@ def test_one_particle_that_is_no_number(gpu_available, dim, treatment, bulk, wha
         assert rel_l2(got[ok], want[ok]) < 1e-11
         big = np.isfinite(want) & ~ok
         assert np.all(np.abs(got[big] / want[big] - 1.0) < 1e-11)
+
+
+@pytest.mark.parametrize("jitter", [0.0, 1e-8, 1e-7, 3e-7, 1e-6, 1e-5])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_pairs_at_one_h(gpu_available, dim, jitter):
+    """Lattices of spacing h with pairs within 1e-5 of q = 1, where the kernel's two
+    branches meet: they differ by 2 (q - 1)^2 in the gradient, so the branch has to
+    be chosen in double. Bar: some 20 (80) terms good to 4 units of 1.1e-16 each, of
+    alternating sign, against their sum."""
+    c = _scene(dim, 1)
+    c.model["intf_hsml_coef"] = 1.0
+    rng = np.random.default_rng(5)
+    c.r = np.round(c.r / 0.005) * 0.005 + rng.uniform(-jitter * 0.02, jitter * 0.02, c.r.shape)
+    got, want = _both(c, 1)
+    assert rel_l2(got[0], want[0]) < 1.5e-15 and rel_l2(got[2], want[2]) < 1.5e-15
