@@ -743,6 +743,8 @@ void adjoint_release(rrsph_solver* s) {
     s->adj = nullptr;
 }
 
+bool adjoint_uses_pairs(const rrsph_solver* s) { return s->adj && s->adj->rec; }
+
 }  // namespace rrsph_impl
 
 namespace {

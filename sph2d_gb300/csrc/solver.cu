@@ -16,7 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
-#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../host/error.hpp"
@@ -37,45 +37,82 @@ namespace {
                              std::string(#call) + ": " + cudaGetErrorString(err_));                \
     } while (0)
 
+void drop_graphs(rrsph_solver* s);
+
+// The arrays of the stored-pair FP64 step, as (pointer, bytes).
+std::vector<std::pair<void**, size_t>> pair_arrays(rrsph_solver* s) {
+    std::vector<std::pair<void**, size_t>> list;
+    auto& G = s->G;
+    const bool d3 = s->dim == 3, cont = s->P.density_treatment != 0;
+    const size_t n = s->P.n, cap = s->P.pc.cap * n, cells = (d3 ? 27 : 9) * n, w = d3 ? 4 : 2;
+    auto add = [&](auto** ptr, size_t count) { list.emplace_back(reinterpret_cast<void**>(ptr), count * sizeof(**ptr)); };
+    add(&G.pr, w * n);
+    add(&G.pv, w * n);
+    if (!d3) add(&G.pq, 2 * n);
+    if (cont) add(&G.pd, w * n);
+    if (s->P.density_treatment == 2) add(&G.pe, 2 * n);
+    add(&G.pnear, (d3 ? 2 : 1) * cells);
+    add(&G.pbefore, cells);
+    add(&G.pfirst, cells);
+    add(&G.pcount, n);
+    add(&G.pf, (d3 || cont ? 4 : 2) * cap);
+    if (!cont) {
+        add(&G.pw, cap);
+        add(&G.pown, cells);
+        add(&G.ps, cap);
+        add(&G.prank, cap);
+    }
+    return list;
+}
+void free_pairs(rrsph_solver* s) {
+    for (auto& a : pair_arrays(s)) {
+        if (*a.first) cudaFree(*a.first);
+        *a.first = nullptr;
+    }
+    s->pairs64 = false;
+}
+// All of them or none, and only where they fit the optional share of the free
+// memory (optional_memory_fits); without them the directed gathers run.
+void alloc_pairs(rrsph_solver* s) {
+    const auto list = pair_arrays(s);
+    size_t total = 0;
+    for (auto& a : list) total += a.second;
+    s->pairs64 = rrsph_impl::optional_memory_fits(total);
+    for (auto& a : list) {
+        if (s->pairs64 && cudaMalloc(a.first, a.second) != cudaSuccess) {
+            cudaGetLastError();
+            *a.first = nullptr;
+            s->pairs64 = false;
+        }
+    }
+    if (!s->pairs64) free_pairs(s);
+}
+// What the handle needs comes before what it only takes to be faster: where
+// `alloc` finds no memory the stored pairs are given back (unless a recorded
+// adjoint run reads them), and taken again if that was not enough.
+template <class F>
+cudaError_t alloc_with_room(rrsph_solver* s, F&& alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && s->pairs64 && !rrsph_impl::adjoint_uses_pairs(s)) {
+        cudaGetLastError();
+        drop_graphs(s);  // they hold the pointers by value
+        free_pairs(s);
+        e = alloc();
+        if (e != cudaSuccess) alloc_pairs(s);
+    }
+    if (e != cudaSuccess) cudaGetLastError();  // reported by the caller, not by the next call
+    return e;
+}
+
 template <typename T>
 int dev_alloc(rrsph_solver* s, T** ptr, size_t count) {
     *ptr = nullptr;
     if (count == 0) return RRSPH_OK;
     void* p = nullptr;
-    RRSPH_CUDA_TRY(cudaMalloc(&p, count * sizeof(T)));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMalloc(&p, count * sizeof(T)); }));
     s->allocations.push_back(p);
     *ptr = static_cast<T*>(p);
     return RRSPH_OK;
-}
-
-// The arrays of the stored-pair FP64 step, all of them or none.
-bool alloc_pairs(rrsph_solver* s) {
-    auto& G = s->G;
-    const size_t n = s->P.n, cap = s->P.pc.cap, w = s->dim == 3 ? 4 : 2;
-    const bool cont = s->P.density_treatment != 0;
-    const size_t before = s->allocations.size();
-    auto get = [&](auto** ptr, size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, count * sizeof(**ptr)) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        s->allocations.push_back(p);
-        *ptr = static_cast<std::remove_reference_t<decltype(*ptr)>>(p);
-        return true;
-    };
-    const bool ok = get(&G.pr, w * n) && get(&G.pv, w * n) && (s->dim == 3 || get(&G.pq, 2 * n)) &&
-                    (!cont || get(&G.pd, w * n)) && (s->P.density_treatment != 2 || get(&G.pe, 2 * n)) &&
-                    get(&G.pnear, (s->dim == 3 ? 2 * 27 : 9) * n) && get(&G.pbefore, (s->dim == 3 ? 27 : 9) * n) &&
-                    get(&G.pfirst, (s->dim == 3 ? 27 : 9) * n) && get(&G.pcount, n) && (cont || get(&G.pw, cap * n)) &&
-                    get(&G.pf, (s->dim == 3 || cont ? 4 : 2) * cap * n) &&
-                    (cont || (get(&G.pown, (s->dim == 3 ? 27 : 9) * n) && get(&G.ps, cap * n) && get(&G.prank, cap * n)));
-    if (ok) return true;
-    while (s->allocations.size() > before) {
-        cudaFree(s->allocations.back());
-        s->allocations.pop_back();
-    }
-    return false;
 }
 
 // Host copies of the smoothing-kernel factors and W (SmoothingKernel.h).
@@ -545,6 +582,18 @@ int flags_to_status(const rrsph_solver* s, uint32_t f) {
 
 int rrsph_impl::flags_status(const rrsph_solver* s, uint32_t f) { return flags_to_status(s, f); }
 
+bool rrsph_impl::optional_memory_fits(size_t bytes) {
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes <= free_bytes / 4;
+}
+cudaError_t rrsph_impl::malloc_with_room(rrsph_solver* s, void** p, size_t bytes) {
+    return alloc_with_room(s, [&] { return cudaMalloc(p, bytes); });
+}
+
 // ============================================================== C ABI ======
 
 extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver** out) {
@@ -609,8 +658,6 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
         if (d3) A(S.coff4, n); else A(S.coff2, n);
         A(G.P4, n);
         if (cont) { A(G.vdx, n); A(G.vdy, n); if (d3) A(G.vdz, n); A(G.rhod, n); }
-        // 1.2 KB (3D: 5.7 KB) a particle; without room for them the directed gathers run
-        if (pair_method(s->P)) s->pairs64 = alloc_pairs(s);
     } else {
         if (d3) { A(S.coff4, n); A(S.vpf4, n); } else { A(S.coff2, n); A(S.vpf2, n); }
         if (n < rrsph::verlet_max_particles(s->dim)) {  // neighbour reuse
@@ -708,6 +755,8 @@ extern "C" int rrsph_create(const rrsph_params* p, int precision, rrsph_solver**
     }
     if (cudaStreamSynchronize(s->stream) != cudaSuccess)
         return fail(set_error(RRSPH_ERR_CUDA, "rrsph_create: synchronize failed"));
+    // last, 1.7 KB a particle (3D: 5.6 KB, with summation density 8.3 KB)
+    if (!mixed && pair_method(s->P)) alloc_pairs(s);
     *out = s;
     return RRSPH_OK;
 }
@@ -723,6 +772,7 @@ extern "C" void rrsph_destroy(rrsph_solver* s) {
     if (s->dl_stream) cudaStreamDestroy(s->dl_stream);
     for (int i = 0; i <= kPhases; i++)
         if (s->ev[i]) cudaEventDestroy(s->ev[i]);
+    if (s->pairs64) free_pairs(s);
     for (void* a : s->allocations)
         if (a) cudaFree(a);
     if (s->h_scal) cudaFreeHost(s->h_scal);
@@ -1223,7 +1273,7 @@ extern "C" int rrsph_grid_find(rrsph_solver* s, uint32_t* keys, uint32_t* grid, 
     const size_t n = s->P.n;
     uint32_t* d_cs = nullptr;
     if (cells_start) {
-        RRSPH_CUDA_TRY(cudaMallocAsync(&d_cs, ((size_t)s->P.max_cells + 1) * sizeof(uint32_t), st));
+        RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMallocAsync(&d_cs, ((size_t)s->P.max_cells + 1) * sizeof(uint32_t), st); }));
         rrsph::launch_cells_start(s->P, s->G, d_cs, st);
         s->launches++;
         RRSPH_CUDA_TRY(cudaMemcpyAsync(cells_start, d_cs, ((size_t)s->P.max_cells + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -1244,8 +1294,8 @@ extern "C" int rrsph_neighbours(rrsph_solver* s, uint32_t* counts, uint32_t* lis
     RRSPH_CUDA_TRY(cudaMemsetAsync(s->flags, 0, sizeof(uint32_t), st));
     enqueue_component_grid_dim(s, false);
     uint32_t *d_counts = nullptr, *d_list = nullptr;
-    RRSPH_CUDA_TRY(cudaMallocAsync(&d_counts, n * sizeof(uint32_t), st));
-    RRSPH_CUDA_TRY(cudaMallocAsync(&d_list, n * (size_t)max_per * sizeof(uint32_t), st));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMallocAsync(&d_counts, n * sizeof(uint32_t), st); }));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMallocAsync(&d_list, n * (size_t)max_per * sizeof(uint32_t), st); }));
     if (s->dim == 3) rrsph::launch_neighbour_list<3>(s->P, s->G, d_counts, d_list, max_per, s->flags, st);
     else rrsph::launch_neighbour_list<2>(s->P, s->G, d_counts, d_list, max_per, s->flags, st);
     s->launches++;
@@ -1277,8 +1327,8 @@ extern "C" int rrsph_step_neighbours(rrsph_solver* s, uint32_t* counts, uint32_t
     const size_t n = s->P.n;
     RRSPH_CUDA_TRY(cudaMemsetAsync(s->flags, 0, sizeof(uint32_t), st));
     uint32_t *d_counts = nullptr, *d_list = nullptr;
-    RRSPH_CUDA_TRY(cudaMallocAsync(&d_counts, n * sizeof(uint32_t), st));
-    RRSPH_CUDA_TRY(cudaMallocAsync(&d_list, n * (size_t)max_per * sizeof(uint32_t), st));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMallocAsync(&d_counts, n * sizeof(uint32_t), st); }));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMallocAsync(&d_list, n * (size_t)max_per * sizeof(uint32_t), st); }));
     s->G.key = s->G.keys_a;  // the grid of the last rebuild, which the list refers to
     s->G.id = s->G.ids_a;
     if (s->dim == 3) rrsph::launch_nlist_export<3>(s->P, s->G, d_counts, d_list, max_per, s->flags, st);
@@ -1459,7 +1509,7 @@ int backup_state(rrsph_solver* s, Backup& b) {
     b.fields.emplace_back(S.itype, n * sizeof(int32_t));
     size_t total = 0;
     for (auto& f : b.fields) total += f.second;
-    RRSPH_CUDA_TRY(cudaMalloc(&b.buf, total));
+    RRSPH_CUDA_TRY(alloc_with_room(s, [&] { return cudaMalloc(&b.buf, total); }));
     char* dst = static_cast<char*>(b.buf);
     for (auto& f : b.fields) {
         RRSPH_CUDA_TRY(cudaMemcpyAsync(dst, f.first, f.second, cudaMemcpyDeviceToDevice, s->stream));

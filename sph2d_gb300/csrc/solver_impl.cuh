@@ -98,6 +98,14 @@ namespace rrsph_impl {
 void adjoint_release(rrsph_solver* s);
 // The status (and error message) the device flags f mean for s (solver.cu).
 int flags_status(const rrsph_solver* s, uint32_t f);
+// Whether memory a handle can do without may be taken: at most a quarter of what is
+// free, so that other solvers, other libraries and this handle's later calls find
+// theirs (3D summation density: up to 8.6M particles on an empty card).
+bool optional_memory_fits(size_t bytes);
+// cudaMalloc for s, which gives its stored pairs back where there is too little.
+cudaError_t malloc_with_room(rrsph_solver* s, void** p, size_t bytes);
+// Whether the recorded adjoint run of s reads the stored pairs (adjoint.cu).
+bool adjoint_uses_pairs(const rrsph_solver* s);
 }  // namespace rrsph_impl
 
 
