@@ -760,38 +760,38 @@ using rrsph_impl::AdjointRun;
     } while (0)
 
 template <typename T>
-int adj_alloc(AdjointRun* run, T** ptr, size_t count) {
+int adj_alloc(rrsph_solver* s, T** ptr, size_t count) {
     void* p = nullptr;
-    ADJ_TRY(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
-    run->allocs.push_back(p);
+    ADJ_TRY(rrsph_impl::malloc_with_room(s, &p, std::max<size_t>(count, 1) * sizeof(T)));
+    s->adj->allocs.push_back(p);
     *ptr = static_cast<T*>(p);
     return RRSPH_OK;
 }
 
-// The stored pairs' records where the forward step stores pairs and there is room
-// for them, else the masks of a segment's steps.
+// After what every run needs: the stored pairs' records where the forward step
+// stores pairs and the room is there (in one piece, the λa first), else the masks of a
+// segment's steps.
 int adj_alloc_pairs(rrsph_solver* s, AdjointRun* run) {
-    const size_t n = s->P.n;
-    void *la = nullptr, *rec = nullptr;
-    if (s->pairs64 && cudaMalloc(&la, n * sizeof(double2)) == cudaSuccess) {
-        run->allocs.push_back(la);
-        if (cudaMalloc(&rec, (size_t)s->P.pc.cap * n * 6 * sizeof(double)) == cudaSuccess) {
-            run->allocs.push_back(rec);
-            run->la = static_cast<double2*>(la);
-            run->rec = static_cast<double*>(rec);
+    const size_t n = s->P.n, bytes = n * sizeof(double2) + (size_t)s->P.pc.cap * n * 6 * sizeof(double);
+    void* p = nullptr;
+    if (s->pairs64 && rrsph_impl::optional_memory_fits(bytes)) {
+        if (cudaMalloc(&p, bytes) == cudaSuccess) {
+            run->allocs.push_back(p);
+            run->la = static_cast<double2*>(p);
+            run->rec = reinterpret_cast<double*>(run->la + n);
             return RRSPH_OK;
         }
+        cudaGetLastError();
     }
-    cudaGetLastError();
-    return adj_alloc(run, &run->seg_mask, run->K * 10 * n);
+    return adj_alloc(s, &run->seg_mask, run->K * 10 * n);
 }
 
-int alloc_snap(AdjointRun* run, rrsph::Snap& sn, size_t slots, size_t n) {
+int alloc_snap(rrsph_solver* s, rrsph::Snap& sn, size_t slots, size_t n) {
     int rc;
     double** f[6] = {&sn.rx, &sn.ry, &sn.vx, &sn.vy, &sn.ax, &sn.ay};
     for (auto* p : f)
-        if ((rc = adj_alloc(run, p, slots * n)) != 0) return rc;
-    return adj_alloc(run, &sn.itype, slots * n);
+        if ((rc = adj_alloc(s, p, slots * n)) != 0) return rc;
+    return adj_alloc(s, &sn.itype, slots * n);
 }
 
 // Copies between the solver's state and a snapshot slot.
@@ -969,20 +969,19 @@ extern "C" int rrsph_adjoint_forward(rrsph_solver* s, const rrsph_adjoint_config
     run->fourier_omega = s->P.fourier_omega;
     std::memcpy(run->fourier_coef, s->P.fourier_coef, sizeof(run->fourier_coef));
     const size_t n = s->P.n;
-    if ((rc = alloc_snap(run, run->ck, run->nck, n)) != 0 || (rc = alloc_snap(run, run->seg, run->K, n)) != 0 ||
-        (rc = adj_alloc(run, &run->ck_scal, run->nck)) != 0 || (rc = adj_alloc(run, &run->seg_rho, run->K * n)) != 0 ||
-        (rc = adj_alloc(run, &run->seg_key, run->K * n)) != 0 || (rc = adj_alloc(run, &run->seg_id, run->K * n)) != 0 ||
-        (rc = adj_alloc_pairs(s, run)) != 0)
+    if ((rc = alloc_snap(s, run->ck, run->nck, n)) != 0 || (rc = alloc_snap(s, run->seg, run->K, n)) != 0 ||
+        (rc = adj_alloc(s, &run->ck_scal, run->nck)) != 0 || (rc = adj_alloc(s, &run->seg_rho, run->K * n)) != 0 ||
+        (rc = adj_alloc(s, &run->seg_key, run->K * n)) != 0 || (rc = adj_alloc(s, &run->seg_id, run->K * n)) != 0)
         return rc;
     for (auto& set : run->lam)
         for (auto& p : set)
-            if ((rc = adj_alloc(run, &p, n)) != 0) return rc;
-    if ((rc = adj_alloc(run, &run->la_x, n)) != 0 || (rc = adj_alloc(run, &run->la_y, n)) != 0 ||
-        (rc = adj_alloc(run, &run->lrho, n)) != 0 || (rc = adj_alloc(run, &run->pr2, n)) != 0 ||
-        (rc = adj_alloc(run, &run->gvx, n)) != 0 || (rc = adj_alloc(run, &run->g_steps, run->N)) != 0 ||
-        (rc = adj_alloc(run, &run->end_rho, n)) != 0 || (rc = adj_alloc(run, &run->end_p, n)) != 0 ||
-        (rc = adj_alloc(run, &run->gauge_best, run->nsamples)) != 0 ||
-        (rc = adj_alloc(run, &run->gauge_id, run->nsamples)) != 0)
+            if ((rc = adj_alloc(s, &p, n)) != 0) return rc;
+    if ((rc = adj_alloc(s, &run->la_x, n)) != 0 || (rc = adj_alloc(s, &run->la_y, n)) != 0 ||
+        (rc = adj_alloc(s, &run->lrho, n)) != 0 || (rc = adj_alloc(s, &run->pr2, n)) != 0 ||
+        (rc = adj_alloc(s, &run->gvx, n)) != 0 || (rc = adj_alloc(s, &run->g_steps, run->N)) != 0 ||
+        (rc = adj_alloc(s, &run->end_rho, n)) != 0 || (rc = adj_alloc(s, &run->end_p, n)) != 0 ||
+        (rc = adj_alloc(s, &run->gauge_best, run->nsamples)) != 0 ||
+        (rc = adj_alloc(s, &run->gauge_id, run->nsamples)) != 0 || (rc = adj_alloc_pairs(s, run)) != 0)
         return rc;
     cudaStream_t st = s->stream;
     ADJ_TRY(cudaMemsetAsync(run->gauge_best, 0, std::max<uint64_t>(run->nsamples, 1) * sizeof(unsigned long long), st));
