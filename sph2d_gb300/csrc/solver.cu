@@ -1563,19 +1563,19 @@ extern "C" int rrsph_set_wave_makers(rrsph_solver* s, uint32_t count, const rrsp
                                    m.wave_magnitude, k, m.depth};
     }
     drop_graphs(s);  // the step graphs hold the state pointers by value
-    if (!s->S.wave_tank) {
-        if ((rc = dev_alloc(s, &s->S.wave_tank, n)) != 0) return rc;
-    }
+    // the handle's state changes once everything is there
+    int32_t* tank = s->S.wave_tank;
     rrsph::PistonLaw* table = nullptr;
     double* vx = nullptr;
+    if (!tank && (rc = dev_alloc(s, &tank, n)) != 0) return rc;
     if ((rc = dev_alloc(s, &table, std::max<size_t>(count, 1))) != 0) return rc;
     if ((rc = dev_alloc(s, &vx, std::max<size_t>(count, 1))) != 0) return rc;
-    RRSPH_CUDA_TRY(cudaMemcpy(s->S.wave_tank, owner.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
+    RRSPH_CUDA_TRY(cudaMemcpy(tank, owner.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
     if (count) RRSPH_CUDA_TRY(cudaMemcpy(table, laws.data(), count * sizeof(rrsph::PistonLaw), cudaMemcpyHostToDevice));
+    s->S.wave_tank = count ? tank : nullptr;  // an empty table restores the params' wave maker
     s->S.wave_law = table;
     s->S.wave_vx = vx;
     s->S.wave_count = count;
-    if (!count) s->S.wave_tank = nullptr;  // an empty table restores the params' wave maker
     return RRSPH_OK;
 }
 
