@@ -423,9 +423,11 @@ int rrsph_set_wave_makers(rrsph_solver* s, uint32_t count, const rrsph_wave_make
  * gathers that split a particle's list over four warps (few particles, FP32-mixed
  * with neighbour reuse) keep their own. */
 int rrsph_set_gather_threads(rrsph_solver* s, uint32_t density_threads, uint32_t force_threads);
-/* Autotuner: times `steps` steps on the uploaded state for every pair of
- * candidate gather block sizes (64, 128, 256), keeps the fastest and puts the
- * state back. threads_out[2] (may be NULL) receives {density, forces}. */
+/* Autotuner: times `steps` steps on the uploaded state with the sizes in use (the
+ * kernels' own, unless set) and for every pair of candidate gather block sizes (64,
+ * 128, 256), sets the fastest candidate where it is faster than the sizes in use, and
+ * puts the state back. threads_out[2] (may be NULL) receives the fastest candidate's
+ * {density, forces}. */
 int rrsph_autotune(rrsph_solver* s, uint32_t steps, uint32_t* threads_out);
 /* Autotuner of the candidate lists' skin (the FP32-mixed step with neighbour
  * reuse): for skins of 0.2, 0.3, 0.4, 0.5, 0.6 and 0.8 hsml in turn, rebuilds

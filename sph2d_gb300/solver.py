@@ -288,7 +288,8 @@ class Solver:
         check(lib().rrsph_set_gather_threads(self._h, density, forces))
 
     def autotune(self, steps: int = 5):
-        """Picks the gather block sizes by timing; returns (density, forces) threads."""
+        """Times candidate gather block sizes and sets the fastest where it beats the
+        sizes in use; returns that candidate's (density, forces) threads."""
         out = (C.c_uint32 * 2)()
         check(lib().rrsph_autotune(self._h, steps, out))
         return int(out[0]), int(out[1])
