@@ -404,6 +404,11 @@ __global__ void k_adj_pair_reorder(DevParams P, Sorted G, SnapView sn, const dou
 struct AdjTerms {
     double rx, ry, vx, vy, p, rho, msc;
 };
+// m sc and m (dsc/ddist)/dist of the far branch, for the pairs just beyond q = 1.
+__device__ __noinline__ Kern adj_beyond(double s2, double inv_h, double q, double y) {
+    const double t = 2.0 - q;
+    return {(s2 * y) * (t * t), -(s2 * t) * ((y * y) * fma(t, y, 2.0 * inv_h))};
+}
 // Inverse distance, distance, m sc and m (dsc/ddist)/dist; false: coincident.
 template <bool NEAR>
 __device__ __forceinline__ bool adj_kernel(const PairConst& C, double s2, double& y, double& dist, double& sc,
@@ -414,7 +419,11 @@ __device__ __forceinline__ bool adj_kernel(const PairConst& C, double s2, double
     dist = fma(fma(-r, r, s2), hy, r);
     y = fma(y1, fma(-r, hy, 0.5), y1);
     const double q = dist * C.inv_h;
-    if (NEAR) {
+    if (NEAR && beyond(q)) {  // (as cubic())
+        const Kern k = adj_beyond(C.s2, C.inv_h, q, y);
+        sc = k.w;
+        sc1 = k.s;
+    } else if (NEAR) {
         sc = fma(C.s1q, q, C.s1);
         sc1 = C.s1q * C.inv_h * y;
     } else {

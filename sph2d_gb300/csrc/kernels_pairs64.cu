@@ -49,7 +49,7 @@ __device__ __forceinline__ void warp_sum_add(unsigned long long* dst, unsigned l
 // offsets decides outside the guard band around the cutoff, the reference's
 // double test inside it and for particles outside their cell (clamped, or
 // beyond the key's bits), whose x the reorder set to NaN (+inf: non-existent).
-// near: the neighbours at up to one h, decided alike. Then the neighbours, and the owned ones,
+// near: the neighbours at up to one h, and some just beyond. Then the neighbours, and the owned ones,
 // in the cells before this one (saturated: a number past the slots is not stored).
 // Issue-bound: a dozen instructions per candidate. A group of lanes per
 // particle instead, a cell a lane, ran at 14 (3D: 9) lanes of 32: 124 us on the
@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_mas
             over = e - s > (wraps ? 0u : M::bits);
             if (!over) {
                 const MixedF& F = P.mf;
-                // the band around one h: the float test is good to a few units of 2^-24 of 8 h^2
-                const float h2_lo = F.h * F.h * (1.0f - 2e-5f), h2_hi = F.h * F.h * (1.0f + 2e-5f);
+                // one h, and the error of the float test above it
+                const float h2 = F.h * F.h * (1.0f + 2e-5f);
                 const float3 sh = stencil_shift<DIM>(c);
                 const float shx = sh.x * F.cell - pj.x, shy = sh.y * F.cell - pj.y;
                 const float shz = DIM == 3 ? sh.z * F.cell - pj.z : 0.0f;
@@ -98,38 +98,37 @@ __global__ void __launch_bounds__(32 * Pm<DIM>::nc, DIM == 3 ? 2 : 7) k_pair_mas
 #pragma unroll 1
                 for (uint32_t s0 = s; s0 < e; s0 += 32) {
                     const uint32_t len = min(e - s0, 32u);
-                    uint32_t in = 0, below = 0;        // below the guard band, or its end
-                    uint32_t close = 0, closer = 0;    // the same of one h
+                    uint32_t in = 0, below = 0, close = 0;  // below the guard band, or its end; at up to one h
 #pragma unroll 1
                     for (uint32_t j = 0; j < len; j += B) {
                         float4 q[B];
 #pragma unroll
                         for (uint32_t u = 0; u < B; u++) q[u] = G.P4[min(s0 + j + u, e - 1u)];
-                        uint32_t a = 0, b = 0, o = 0, p = 0;
+                        uint32_t a = 0, b = 0, o = 0;
 #pragma unroll
                         for (uint32_t u = 0; u < B; u++) {
                             const float dx = q[u].x + shx, dy = q[u].y + shy, dz = DIM == 3 ? q[u].z + shz : 0.0f;
                             const float d2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
                             if (d2 < F.cut2_lo) a |= 1u << u;
                             if (!(d2 >= F.cut2_hi)) b |= 1u << u;
-                            if (!(d2 >= h2_hi)) o |= 1u << u;
-                            if (d2 < h2_lo) p |= 1u << u;
+                            if (d2 < h2) o |= 1u << u;
                         }
                         in |= a << j;
                         below |= b << j;
                         close |= o << j;
-                        closer |= p << j;
                     }
                     const uint32_t valid = 0xFFFFFFFFu >> (32u - len);
                     in &= valid;
                     close &= valid;
-                    for (uint32_t band = ((below & ~in) | (close & ~closer)) & valid; band; band &= band - 1) {
+                    for (uint32_t band = below & valid & ~in; band; band &= band - 1) {
                         const uint32_t bit = __ffs(band) - 1, i = s0 + bit;
                         const D3 a = row<DIM>(G.pr, i), b = row<DIM>(G.pr, k);
                         const double r2 = exact_dist2<DIM>(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y),
                                                            DIM == 3 ? __dsub_rn(a.z, b.z) : 0.0);
-                        if (r2 < P.cut2 && G.itype[i] != P.type_non_existent) in |= 1u << bit;
-                        if (!(r2 <= P.h * P.h)) close &= ~(1u << bit);
+                        if (r2 < P.cut2 && G.itype[i] != P.type_non_existent) {
+                            in |= 1u << bit;
+                            if (r2 <= P.h * P.h) close |= 1u << bit;
+                        }
                     }
                     mask |= (T)in << ((s0 - s) & (M::bits - 1));
                     near |= (T)close << ((s0 - s) & (M::bits - 1));
@@ -311,8 +310,9 @@ struct Approach {  // a warp's second stack
     uint2 e[kStack];
     double dx[kStack], dy[kStack], dz[DIM == 3 ? kStack : 1], vr[kStack];
 };
+// (2D: at most 64 registers, for 32 blocks of one warp on an SM)
 template <int DIM>
-__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_forces(DevParams P, Sorted G) {
+__global__ void __launch_bounds__(kMaxGatherThreads, DIM == 2 ? 4 : 1) k_pair_forces(DevParams P, Sorted G) {
     extern __shared__ double2 pair_shared[];
     Approach<DIM>& A = reinterpret_cast<Approach<DIM>*>(pair_shared)[threadIdx.x >> 5];
     uint2* const stacks = reinterpret_cast<uint2*>(reinterpret_cast<Approach<DIM>*>(pair_shared) + (blockDim.x >> 5));

@@ -154,12 +154,21 @@ __device__ __forceinline__ double half_of(double x) {
 }
 
 // The cubic spline at squared distance d2 (SmoothingKernel.h:20-56): m W, and
-// m s with dW/dr = (r_i - r_j) s. NEAR: the branch q <= 1, where the two meet
-// with equal second derivatives, so which one takes a pair at q = 1 to float
-// accuracy does not show.
+// m s with dW/dr = (r_i - r_j) s. NEAR: the branch q <= 1, which the masks' float
+// test gives to all up to there and to some just beyond. These go through
+// cubic_beyond (the branches' gradients differ by 2 (q - 1)^2, 1e-13 at the float
+// test's error): a call, since the FP64 pipe would issue a few predicated operations
+// for every pair.
 struct Kern {
     double w, s;
 };
+__device__ __noinline__ Kern cubic_beyond(double w6, double s2, double q, double y1, double r) {
+    const double y = fma(y1, fma(-r, half_of(y1), 0.5), y1);
+    const double t = 2.0 - q, t2 = t * t;
+    return {(w6 * t) * t2, (s2 * y) * t2};
+}
+// q >= 1
+__device__ __forceinline__ bool beyond(double q) { return __double2hiint(q) >= 0x3FF00000; }
 template <bool NEAR, bool W>
 __device__ __forceinline__ Kern cubic(const PairConst& C, double d2) {
     const double y1 = inv_root_40(d2);
@@ -168,6 +177,7 @@ __device__ __forceinline__ Kern cubic(const PairConst& C, double d2) {
     const double q = __double2hiint(y1) == 0x7FF00000 ? 0.0 : dist * C.inv_h;
     Kern k{0.0, 0.0};
     if (NEAR) {
+        if (beyond(q)) return cubic_beyond(C.w6, C.s2, q, y1, r);
         if (W) k.w = fma(q * q, fma(C.w3, q, C.w2), C.w0q);
         k.s = fma(C.s1q, q, C.s1);
     } else {
