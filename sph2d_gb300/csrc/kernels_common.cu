@@ -27,6 +27,59 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
     key_pass<DIM, 2>(P, S, G, i, S.rx[i], S.ry[i], DIM == 3 ? S.rz[i] : 0.0, flags);
 }
 
+// The place of each id of a block among its cell's, where some cell holds more than
+// kCrowd: `mine` of the threads take part, with ids of cells [start, end) of the scattered
+// ids (a block's places are consecutive, so its ids of a cell too). Cell by cell the
+// block sorts its own ids, counts every id of the cell into the gap between them where
+// it falls, and adds the gaps up: end - start reads a block, and not a thread. All threads
+// of the block call.
+constexpr uint32_t kReorderThreads = 256;
+constexpr uint32_t kCrowd = 1024;  // (10,000 of 205k in a cell, grid and copies back: each thread reading 0.27 ms, so 0.13)
+__device__ __noinline__ uint32_t crowded_rank(const uint32_t* __restrict__ scattered, uint32_t id, uint32_t start,
+                                              uint32_t end, bool mine) {
+    __shared__ uint32_t ids[kReorderThreads], sorted[kReorderThreads], gaps[kReorderThreads], lead, from, to;
+    const uint32_t t = threadIdx.x;
+    uint32_t rank = 0;
+    while (true) {
+        if (t == 0) lead = kReorderThreads;
+        __syncthreads();
+        if (mine) atomicMin(&lead, t);
+        __syncthreads();
+        if (lead == kReorderThreads) return rank;
+        if (t == lead) {
+            from = start;
+            to = end;
+        }
+        __syncthreads();
+        const bool now = mine && start == from;
+        ids[t] = now ? id : 0xFFFFFFFFu;  // (never an id)
+        sorted[t] = 0xFFFFFFFFu;
+        gaps[t] = 0;
+        __syncthreads();
+        uint32_t at = 0;
+        if (now) {
+            for (uint32_t u = 0; u < kReorderThreads; u++) at += ids[u] < id ? 1u : 0u;
+            sorted[at] = id;
+        }
+        __syncthreads();
+        for (uint32_t j = from + t; j < to; j += kReorderThreads) {
+            const uint32_t x = scattered[j];
+            uint32_t gap = 0;  // of the block's ids those below x
+#pragma unroll
+            for (uint32_t step = kReorderThreads / 2; step; step >>= 1)
+                if (sorted[gap + step - 1] < x) gap += step;
+            if (sorted[gap] >= x) atomicAdd(&gaps[gap], 1u);  // (not above all of them)
+        }
+        __syncthreads();
+        if (now) {
+            for (uint32_t u = 0; u <= at; u++) rank += gaps[u];
+            rank -= 1;  // itself
+            mine = false;
+        }
+        __syncthreads();
+    }
+}
+
 // Gathers the state into cell order and (after the radix sort) records each cell's [start, end) in
 // the sorted arrays (the cells_start table of make_grid, GridFind.cpp:77-87).
 // R: 0 = FP64 gathers; 1 = the mixed loop with summation density; 2 = the
@@ -38,17 +91,29 @@ __global__ void k_keys(DevParams P, State S, Sorted G, const StepScalars* __rest
 template <int DIM, int R>
 __global__ void k_reorder(DevParams P, State S, Sorted G, GatherSrc F) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= P.n) return;
-    uint32_t key, id;
+    uint32_t key = 0, id = 0;
     if (G.scattered) {  // after the counting sort: the place among the cell's ids; the table is written
-        id = G.scattered[k];
-        key = G.keys_in[id];
-        const uint32_t s = G.cell_start[key], e = G.cell_end[key];
-        k = s;
-        for (uint32_t j = s; j < e; j++) k += G.scattered[j] < id ? 1u : 0u;
+        uint32_t s = 0, e = 0, rank = 0;
+        const bool valid = k < P.n;
+        if (valid) {
+            id = G.scattered[k];
+            key = G.keys_in[id];
+            s = G.cell_start[key];
+            e = G.cell_end[key];
+        }
+        const bool crowded = e - s > kCrowd;
+        if (!crowded)
+            for (uint32_t j = s; j < e; j++) rank += G.scattered[j] < id ? 1u : 0u;
+        if (__syncthreads_or(crowded)) {
+            const uint32_t r = crowded_rank(G.scattered, id, s, e, crowded);
+            if (crowded) rank = r;
+        }
+        if (!valid) return;
+        k = s + rank;
         G.key[k] = key;
         G.id[k] = id;
     } else {
+        if (k >= P.n) return;
         key = G.key[k];
         id = G.id[k];
         if (k == 0 || G.key[k - 1] != key) G.cell_start[key] = k;
@@ -489,14 +554,14 @@ void launch_keys(const DevParams& P, const State& S, Sorted& G, StepScalars* sca
 template <int DIM>
 void launch_reorder(const DevParams& P, const State& S, const Sorted& G, GatherSrc fsrc, int for_whom,
                     cudaStream_t st) {
-    const unsigned b = blocks_for(P.n, 256);
-    if (for_whom == kReorderPairs) k_reorder<DIM, 4><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else if (for_whom == kReorderFp64) k_reorder<DIM, 0><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else if (for_whom == kReorderReuse && P.density_treatment == 0) k_reorder<DIM, 5><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else if (for_whom == kReorderReuse) k_reorder<DIM, 6><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else if (!fsrc.loop) k_reorder<DIM, 3><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else if (P.density_treatment == 0) k_reorder<DIM, 1><<<b, 256, 0, st>>>(P, S, G, fsrc);
-    else k_reorder<DIM, 2><<<b, 256, 0, st>>>(P, S, G, fsrc);
+    const unsigned b = blocks_for(P.n, kReorderThreads);
+    if (for_whom == kReorderPairs) k_reorder<DIM, 4><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderFp64) k_reorder<DIM, 0><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderReuse && P.density_treatment == 0) k_reorder<DIM, 5><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else if (for_whom == kReorderReuse) k_reorder<DIM, 6><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else if (!fsrc.loop) k_reorder<DIM, 3><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else if (P.density_treatment == 0) k_reorder<DIM, 1><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
+    else k_reorder<DIM, 2><<<b, kReorderThreads, 0, st>>>(P, S, G, fsrc);
 }
 template <int DIM>
 void launch_whole_step(const DevParams& P, const State& S, const Sorted& G, StepScalars* scal_cur,

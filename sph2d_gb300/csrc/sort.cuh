@@ -28,7 +28,7 @@ void radix_sort_pairs_into(const uint32_t* keys_in, const uint32_t* vals_in, uin
 // kCountCells cells and 64 per particle: every particle takes a place in its cell by an
 // atomic count, one pass over the cells turns the counts into the cell table
 // (empty cells start at kEmpty) and the particles are
-// scattered to their cells; the reorder that follows orders each cell's few ids.
+// scattered to their cells; the reorder that follows orders each cell's ids.
 // Three launches for any key length against three per 8 bits, and the table with
 // them: 409k flume (2M cells) 55 -> 23 us, 6k dam break (8k cells) 28 -> 15 us.
 // Above the limits the pass over the cells would cost more than the radix sort.
