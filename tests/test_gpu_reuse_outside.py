@@ -134,3 +134,59 @@ def test_coincident_particles_count_each_other(gpu_available, name, reuse):
     assert rel_l2(rho[1], rho[0]) < 1e-6
     both = np.concatenate([first, first + 1])
     assert np.all(np.abs(rho[1][both] / rho[0][both] - 1.0) < 1e-6)
+
+
+def test_fp64_masks_at_the_last_key(gpu_available):
+    """The stored-pair FP64 step's masks at the same place, against the directed gathers."""
+    from sph2d_gb300 import Solver
+
+    for crowd in (20, 300):
+        c = _at_the_last_key(crowd, 40, 0.49, 1000)
+        with Solver(c.params(), "fp64") as s:
+            s.upload(c.r, c.v, c.rho, c.itype)
+            s.step(1)
+            rates, pairs = s.download_rates(), s.pair_count()[0]
+            s.upload(c.r, c.v, c.rho, c.itype)
+            drho = s.density()[0]
+            a = s.forces()[0]
+            assert pairs == s.neighbours(1000)[2]
+        assert rel_l2(rates["drho"], drho) < 1e-11 and rel_l2(rates["a"], a) < 1e-11
+
+
+def _large(dim):
+    """Fixed-point positions and one thread a particle: 2D above 36,000, 3D above 128,000."""
+    from sph2d_gb300 import cases
+
+    c = cases.dam_break_2d(seed=2, nx=300, ny=150, dx=0.02, tank=(6.6, 3.4)) if dim == 2 else \
+        cases.dam_break_3d(dx=0.0115, tank=(2.2, 0.5, 0.5))
+    c.v = np.random.default_rng(dim).standard_normal(c.v.shape) * 0.3
+    return c
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_large_sets_with_particles_outside_and_absent(gpu_available, dim):
+    """No consistency check: groups below the geometry minimum, within a cell of its
+    edge and 16, 32 and 64 cells away, and non-existent particles."""
+    c = _large(dim)
+    c.model["consistency_check"] = False
+    c.model["consistency_treatment"] = 0
+    p = c.params()
+    cell = 2.0 * p.hsml
+    c.itype[60:120:9] = 0
+    for first, cells in ((0, 0.4), (10, 16.0), (20, 32.0), (30, 64.0)):
+        for j in range(6):
+            c.r[first + j] = c.r[first]
+            c.r[first + j, 0] = p.x_mingeom - (cells + 0.3 * j) * cell
+            c.v[first + j] = 0.0
+    _same(p, c)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("cut", [0, 1, 127, 128, 129, 255])
+def test_large_sets_around_whole_blocks(gpu_available, dim, cut):
+    """The last `cut` + n % 256 particles left out."""
+    c = _large(dim)
+    n = c.ntotal - c.ntotal % 256 - cut
+    c.r, c.v, c.rho, c.itype = c.r[:n].copy(), c.v[:n].copy(), c.rho[:n].copy(), c.itype[:n].copy()
+    c.particle.update(ntotal=n, nvirt=n - c.particle["nfluid"])
+    _same(c.params(), c, steps=1)
