@@ -807,7 +807,10 @@ def run_reference(args, rank: int, world: int) -> dict | None:
     host cores, on the same workload and step window as the GPU arm. It loads
     neither the sph2d_gb300 package nor its library: the particles come from
     the workload generator loaded as a plain module, the parameters from the
-    oracle's own restatement of the reference's loading (oracle/params.py)."""
+    oracle's own restatement of the reference's loading (oracle/params.py).
+    Without the reference's sources the line says `unavailable`: its figures
+    are then those of this repository's C restatement (kind "port"), no
+    reference's."""
     if rank != 0:
         return None
     from oracle import build as ob
@@ -820,8 +823,11 @@ def run_reference(args, rank: int, world: int) -> dict | None:
     p = OP.case_params(case)
     r = reference_timing(case, p, args.warmup, args.steps)
     value = r["value"]
+    missing = {} if r["kind"] == "reference" else {
+        "unavailable": "the reference's RRSPH_OMP core is not built on this machine (its sources are not present); "
+                       "the figures are this repository's C restatement"}
     return {
-        "metric": METRIC, "value": value, "unit": UNIT, "impl": "reference", "n_gpus": world, "steps": args.steps,
+        **missing, "metric": METRIC, "value": value, "unit": UNIT, "impl": "reference", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": r["ms_per_step"], "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded flume particles of the workload's shape)",
         "config": workload_config(case, r["pairs_first"], args.warmup, args.steps),
