@@ -70,10 +70,10 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_density_mixed(DevParams P
                     if (!within_cutoff<DIM>(P, S, G, i, k, d2)) continue;
                     cnt++;
                     if (i - s < 32) bits |= 1u << (i - s);
-                    const float inv_dist = rsqrtf(d2);
+                    const float inv_dist = inv_distance(d2);
                     const float q = d2 * inv_dist * M.inv_h;
                     if (!cont) {
-                        part += kernel_wf(skf, f, fmaxf(q, 0.0f));  // (of coincident particles NaN: W(0))
+                        part += kernel_wf(skf, f, q);
                     } else {
                         const float sc = kernel_dwdr_scalef(skf, f, q, inv_dist, M.inv_h);
                         const float4 vdi = G.VD4[i];

@@ -126,9 +126,6 @@ __device__ __forceinline__ float cubic_s(const ReuseF& U, float q, float rs) {
     const float near = fmaf(3.0f, q, -4.0f);
     return q <= 1.0f ? near : far;
 }
-// 1 / distance, of coincident particles large enough to give q = 0.
-__device__ __forceinline__ float inv_distance(float d2) { return rsqrtf(fmaxf(d2, 1e-30f)); }
-
 // A compensated sum times a factor, as an unevaluated sum of two floats.
 __device__ __forceinline__ F2 scaled(const Kahan& a, F2 f) {
     const float hi = a.s * f.hi;
@@ -336,7 +333,7 @@ __device__ __forceinline__ float density_term(const DevParams& P, float3 d, floa
     float term = vcc * sc;
     if (P.density_treatment == 2) {
         const float rho_factor = __fdividef(vd4_drho<DIM>(vdi, vdj), M.rho0 + vdi.w);
-        term -= d2 > 0.0f ? 2.0f * M.dhc * (rho_factor * sc) : 0.0f;
+        term -= 2.0f * M.dhc * (rho_factor * sc);
     }
     return term;
 }

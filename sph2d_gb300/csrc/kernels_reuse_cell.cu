@@ -194,12 +194,9 @@ __device__ __forceinline__ uint32_t packed_counts(uint32_t c) {
 template <int SKF, bool CONT>
 __device__ __forceinline__ float density_term(const MixedF& M, int skf, float f, float dx, float dy, float d2,
                                               float4 vdi, float4 vdj, bool delta) {
-    const float inv_dist = rsqrtf(d2);
+    const float inv_dist = inv_distance(d2);
     const float q = d2 * inv_dist * M.inv_h;
-    if (!CONT) {
-        const float qw = fmaxf(q, 0.0f);  // (of coincident particles NaN: W(0))
-        return SKF == 1 ? cubic_wf_sel(f, qw) : kernel_wf(skf, f, qw);
-    }
+    if (!CONT) return SKF == 1 ? cubic_wf_sel(f, q) : kernel_wf(skf, f, q);
     const float sc = SKF == 1 ? cubic_dwdr_sel(f, q, inv_dist, M.inv_h)
                               : kernel_dwdr_scalef(skf, f, q, inv_dist, M.inv_h);
     float vcc = (vdi.x - vdj.x) * dx + (vdi.y - vdj.y) * dy;

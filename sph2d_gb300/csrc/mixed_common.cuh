@@ -21,6 +21,10 @@ struct Kahan {
     __device__ __forceinline__ double value() const { return f2d(s) - f2d(c); }
 };
 
+// 1 / distance, of coincident particles large enough to give q = 0 and finite
+// kernels (their separation, which multiplies the gradient, is zero).
+__device__ __forceinline__ float inv_distance(float d2) { return rsqrtf(fmaxf(d2, 1e-30f)); }
+
 // W(q) of smoothing kernel skf (SmoothingKernel.h:20-252), float.
 __device__ __forceinline__ float kernel_wf(int skf, float f, float q) {
     switch (skf) {
@@ -134,11 +138,11 @@ struct ForceAcc {
     __device__ __forceinline__ void pair_with(const float4 vi, const float2 pri, float dx, float dy, float dz,
                                               float d2, int32_t ti) {
         const MixedF& M = P.mf;
-        const float inv_dist = rsqrtf(d2);
+        const float inv_dist = inv_distance(d2);
         const float dist = d2 * inv_dist;
         const float q = dist * M.inv_h;
         float m = 0.0f;  // coefficient of diff (= r_i - r_j) in this pair's acceleration
-        if (ext && ti < 0 && dist < M.lj_rr0) m -= lj_coef(M, inv_dist);
+        if (ext && ti < 0 && dist < M.lj_rr0 && d2 > 0.0f) m -= lj_coef(M, inv_dist);
         const float rhoi = vi.w;
         const float sc = kernel_dwdr_scalef(intf_skf, M.kf[intf_skf], q, inv_dist, M.inv_h);
         if (intf) {

@@ -190,3 +190,71 @@ def test_large_sets_around_whole_blocks(gpu_available, dim, cut):
     c.r, c.v, c.rho, c.itype = c.r[:n].copy(), c.v[:n].copy(), c.rho[:n].copy(), c.itype[:n].copy()
     c.particle.update(ntotal=n, nvirt=n - c.particle["nfluid"])
     _same(c.params(), c, steps=1)
+
+
+def _coincident(name, what):
+    from test_gpu_moved_uploads import _scene
+
+    c = _scene(name)
+    m = c.model
+    m["density_treatment"] = 0 if what == "gauss_sum" else 1
+    m["max_neighbours"] = 900
+    if what.startswith("gauss"):
+        for k in ("density_skf", "intf_skf", "artificial_viscosity_skf", "average_velocity_skf",
+                  "artificial_pressure_skf"):
+            m[k] = 2
+        m["intf_hsml_coef"] = 1.0
+    if what == "xsph":
+        m.update(average_velocity=True, average_velocity_coef=0.05, average_velocity_skf=1)
+    if what == "delta":
+        m.update(density_treatment=2, density_delta_sph_coef=0.1)
+    rng = np.random.default_rng(4)
+    c.v = rng.standard_normal(c.v.shape) * 0.1 * (c.itype > 0)[:, None]
+    c.rho = c.rho * (1.0 + 1e-3 * rng.uniform(-1, 1, len(c.rho)))
+    first = np.arange(3, 1203, 12)
+    c.r[first] = c.r[first + 1]
+    return c, first
+
+
+@pytest.mark.parametrize("what", ["gauss_sum", "gauss_rate", "xsph"])
+@pytest.mark.parametrize("name,reuse", [("2d", True), ("2d_small", True), ("2d_small", False), ("3d_split", True),
+                                         ("3d_split", False)])
+def test_coincident_particles_in_the_other_sums(gpu_available, name, reuse, what):
+    """Gauss kernel (whose exponential of a NaN is one) and XSPH velocity: as in FP64."""
+    from sph2d_gb300 import Solver
+
+    c, first = _coincident(name, what)
+    p = c.params()
+    out = []
+    for precision in ("fp64", "mixed"):
+        with Solver(p, precision) as s:
+            if precision == "mixed":
+                s.set_neighbour_reuse(reuse)
+            s.upload(c.r, c.v, c.rho, c.itype)
+            s.step(1)
+            out.append(s.download() | s.download_rates())
+    for k, bar in (("v", 1e-5), ("a", 1e-5), ("rho", 1e-6)):
+        assert np.all(np.isfinite(out[1][k])) and rel_l2(out[1][k], out[0][k]) < bar, k
+    both = np.concatenate([first, first + 1])
+    assert rel_l2(out[1]["v"][both], out[0]["v"][both]) < 1e-5
+
+
+@pytest.mark.parametrize("name,reuse", [("2d", True), ("2d_small", True), ("2d_small", False), ("3d_split", True),
+                                         ("3d_split", False)])
+def test_the_delta_sph_term_of_coincident_particles(gpu_available, name, reuse):
+    """Its limit: the rate of particles 1e-6 h apart (the reference's is 0/0)."""
+    from sph2d_gb300 import Solver
+
+    c, first = _coincident(name, "delta")
+    p = c.params()
+    drho = []
+    for apart in (0.0, 1e-6 * p.hsml):
+        r = c.r.copy()
+        r[first, 0] += apart
+        with Solver(p, "mixed") as s:
+            s.set_neighbour_reuse(reuse)
+            s.upload(r, c.v, c.rho, c.itype)
+            s.step(1)
+            drho.append(s.download_rates()["drho"])
+    both = np.concatenate([first, first + 1])
+    assert rel_l2(drho[0][both], drho[1][both]) < 1e-4
