@@ -261,7 +261,7 @@ __device__ __forceinline__ void put_forces(const Sorted& G, uint32_t cap, uint32
 // FP64 operations a pair: 2D summation 12 in the near branch of the kernel, 16
 // in the far one; 3D continuity about 40.
 template <int DIM, bool CONT>
-__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_terms(DevParams P, Sorted G) {
+__device__ __forceinline__ void pair_terms(const DevParams& P, const Sorted& G) {
     extern __shared__ uint2 pair_stack[];
     const PairConst& C = P.pc;
     const uint32_t cap = C.cap;
@@ -300,6 +300,17 @@ __global__ void __launch_bounds__(kMaxGatherThreads) k_pair_terms(DevParams P, S
     });
 }
 
+template <int DIM, bool CONT>
+__global__ void __launch_bounds__(kMaxGatherThreads) k_pair_terms(DevParams P, Sorted G) {
+    pair_terms<DIM, CONT>(P, G);
+}
+// (at most 80 registers, for 25 single warps on an SM: 139k particles 845 us a step with
+// the 90 it takes else, so 807)
+template <>
+__global__ void __launch_bounds__(kMaxGatherThreads, 3) k_pair_terms<3, true>(DevParams P, Sorted G) {
+    pair_terms<3, true>(P, G);
+}
+
 // The accelerations, each pair once (summation density). A pair that recedes
 // (no viscosity) is done after 10 FP64 operations in 2D; the others (and the
 // wall pairs) go on to a second stack, and 32 of them at a time take the 12
@@ -310,9 +321,9 @@ struct Approach {  // a warp's second stack
     uint2 e[kStack];
     double dx[kStack], dy[kStack], dz[DIM == 3 ? kStack : 1], vr[kStack];
 };
-// (2D: at most 64 registers, for 32 blocks of one warp on an SM)
+// (at most 64 registers, for 32 blocks of one warp on an SM)
 template <int DIM>
-__global__ void __launch_bounds__(kMaxGatherThreads, DIM == 2 ? 4 : 1) k_pair_forces(DevParams P, Sorted G) {
+__global__ void __launch_bounds__(kMaxGatherThreads, 4) k_pair_forces(DevParams P, Sorted G) {
     extern __shared__ double2 pair_shared[];
     Approach<DIM>& A = reinterpret_cast<Approach<DIM>*>(pair_shared)[threadIdx.x >> 5];
     uint2* const stacks = reinterpret_cast<uint2*>(reinterpret_cast<Approach<DIM>*>(pair_shared) + (blockDim.x >> 5));

@@ -178,7 +178,8 @@ __device__ __forceinline__ float gap_to_cell(int d, float p, float cell) {
 // in one loop: a warp's lanes then wait for the lane with the most particles, not
 // in every cell for the lane whose cell holds most (half of the lanes were idle).
 // The entries pass through a ring in shared memory, as in the density pass: no
-// branch per candidate. BUILDFIG
+// branch per candidate. us a rebuild, walking cell by cell and so: 409k flume 96 / 88,
+// 43k dam break 31 / 22, 1.06M in 3D 1014 / 725.
 constexpr int kVlBuildThreads = 128;
 constexpr int kVlRow = 5;  // cells along an axis of the window, at most
 template <int DIM>
@@ -333,7 +334,9 @@ __device__ __forceinline__ float density_term(const DevParams& P, float3 d, floa
     float term = vcc * sc;
     if (P.density_treatment == 2) {
         const float rho_factor = __fdividef(vd4_drho<DIM>(vdi, vdj), M.rho0 + vdi.w);
-        term -= 2.0f * M.dhc * (rho_factor * sc);
+        // (never false: with the select the 3D gather takes 64 registers, without 75 and 139k
+        // particles 141 us a step instead of 133)
+        term -= d2 >= 0.0f ? 2.0f * M.dhc * (rho_factor * sc) : 0.0f;
     }
     return term;
 }
@@ -772,10 +775,12 @@ void launch_verlet_build(const DevParams& P, const State& S, const Sorted& G, cu
 }
 // Warps per 32 particles of the two gathers (DevParams::vl_split, fixed when a
 // solver is created): four where a thread per particle leaves the SMs a few warps
-// each, else one. us per step with 1 / 4 (8 is no faster): 2D, 6k particles 32.5 /
-// 25.6, 22k 36.9 / 27.8, 33k 38.9 / 34.8, 43k 39.5 / 40.8, 66k 40.9 / 45.7; 3D,
-// 72k 105 / 90, 194k 207 / 211. (A block keeps the registers of the warps that
-// are done while its first warp finishes the step.)
+// each, else one. us per step with 1 / 4 (8 is no faster; in 2D four is
+// kernels_reuse_cell.cu): 2D, 6k particles 27.9 / 23.1, 22k 28.4 / 25.5, 34k 30.1 /
+// 31.9, 43k 31.0 / 33.9, 66k 33.7 / 43.8; 3D, 67k 82.5 / 73.8, 139k 126.2 / 127.4,
+// 240k 204 / 216. (A block keeps the registers of the warps that are done while its
+// first warp finishes the step. The lines were drawn on earlier forms of both; the 2D
+// one would lie at about 30,000 today, but results differ by rounding across it.)
 int verlet_split(int dim, uint32_t n) { return n <= (dim == 3 ? 128000u : 36000u) ? 4 : 1; }
 
 template <int DIM>
