@@ -50,14 +50,13 @@ L2_FLUSH_BYTES = 256 << 20  # larger than the 129 MB L2
 FORCES_ALGORITHMIC_BYTES_PER_PARTICLE = 64 + 96 + 24
 # What the kernel as built reads and writes once per particle and per pair
 # (its own design's bytes, stated beside the algorithmic ones): per particle the
-# gather reads id 4, position+type float4 16, velocity+pressure+density float4
-# 16, (p, p/rho^2) float2 8, candidate and neighbour counts 4 + 4 and writes a.x,
+# gather reads id 4, position+type 16, velocity+pressure+density float4
+# 16, (p, p/rho^2) float2 8, the neighbour count 4 and writes a.x,
 # a.y doubles 16; the whole step reads r, v doubles 32, itype 4, key_of 4, build
-# cell 4, build offset 8, build slot 4 and writes r, v 32, v_predict float2 8,
-# cell offset float2 8, cell 4, key_of 4, sort key + id 8, the next step's
-# position and velocity float4s 32 and one cell-table word 4; per pair one
-# 4-byte word of this step's neighbour list.
-FORCES_DESIGN_BYTES_PER_PARTICLE = (52 + 16) + (32 + 4 + 4 + 4 + 8 + 4) + (32 + 8 + 8 + 4 + 4 + 8 + 32 + 4)
+# cell 4, build position 8, build slot 4 and writes r, v 32, v_predict float2 8,
+# position int2 8, key_of 4, sort key + id 8 and the next step's position and
+# velocity rows 32; per pair one 4-byte word of this step's neighbour list.
+FORCES_DESIGN_BYTES_PER_PARTICLE = (48 + 16) + (32 + 4 + 4 + 4 + 8 + 4) + (32 + 8 + 8 + 4 + 8 + 32)
 FORCES_DESIGN_BYTES_PER_PAIR = 4
 # Pair arithmetic of the FP32 pipe per directed pair: 16 flops for the density
 # (distance, kernel, sum) and 52 for the forces (form-2 pressure term,

@@ -107,7 +107,7 @@ struct Sorted {
     double* pq;        // 2D: rows of 2: density of the forces, p / rho^2
     double* pd;        // continuity density: rows of 2 (4): velocity v
     double* pe;        // delta-SPH: rows of 2: density rho, 1 / rho
-    uint32_t* pnear;   // [3^dim][n], words as nbmask: the neighbours at up to one h
+    uint32_t* pnear;   // [3^dim][n], words as nbmask: the neighbours at up to one h, and some just beyond
     uint8_t* pbefore;  // [3^dim][n]: neighbours in the stencil cells before this one (at most 255)
     uint8_t* pown;     // [3^dim][n], summation density: the same of those with a larger sorted index (owned pairs)
     uint32_t* pcount;  // [n]: neighbours the masks hold

@@ -1092,9 +1092,11 @@ extern "C" int rrsph_step(rrsph_solver* s, uint64_t nsteps, double* time_io) {
 
 namespace {
 // Particles above which p and rho come back while the force gather runs. us per
-// rrsph_step_host of one mixed 2D step, with / without: 2.5k 74.7 / 71.3, 10.9k
-// 95.3 / 86.1, 33k 146.2 / 123.7, 74k 191.9 / 187.8, 133k 225.6 / 231.1, 265k
-// 302.5 / 322.0; FP64: 33k 124.1 / 119.7, 133k 266.8 / 274.4.
+// rrsph_step_host of one step, with / without, when the line was drawn: mixed 2D 2.5k
+// 74.7 / 71.3, 10.9k 95.3 / 86.1, 33k 146.2 / 123.7, 74k 191.9 / 187.8, 133k 225.6 /
+// 231.1, 265k 302.5 / 322.0; FP64 33k 124.1 / 119.7, 133k 266.8 / 274.4. On a later
+// machine 2D 6k 71.9 / 71.0, 34k 90.6 / 91.0, 66k 103.2 / 107.7, 131k 133.2 / 143.5; 3D
+// mixed 67k 175.1 / 176.4, 139k 315 / 322, 240k 504 / 514, 385k 756 / 765.
 constexpr size_t kEarlyCopies = 100000;
 // rrsph_step_host (upload first) and rrsph_step_download (the state on the
 // device); the arguments are checked by the callers.
